@@ -136,7 +136,8 @@ cudaError_t raise_smem_limit(const void* kernel, int bytes) {
 }
 
 CUtensorMap make_row_map(const uint8_t* d_rows, uint64_t bytes_per_row, uint64_t num_rows,
-                         uint64_t pitch, uint32_t box_x, uint32_t box_y) {
+                         uint64_t pitch, uint32_t box_x, uint32_t box_y,
+                         CUtensorMapSwizzle swizzle) {
   if (reinterpret_cast<uintptr_t>(d_rows) % 16 != 0)
     fail(GNM_ERR_INVALID, "packed rows must start on a 16-byte boundary");
   if (pitch % 16 != 0) fail(GNM_ERR_INVALID, "row pitch must be a multiple of 16 bytes");
@@ -148,7 +149,7 @@ CUtensorMap make_row_map(const uint8_t* d_rows, uint64_t bytes_per_row, uint64_t
   cuuint32_t estr[2] = {1, 1};
   CUresult r = encode_fn()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(d_rows),
                            dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) fail(GNM_ERR_COMPUTE, "cuTensorMapEncodeTiled failed for the row map");
   return map;
@@ -507,8 +508,8 @@ static gnm_plan* plan_create_impl(const gnm_prep_view* prep, gnm_engine engine, 
                             cudaMemcpyHostToDevice),
                  "upload output map");
     }
-    p->d_err = dalloc<uint32_t>(p, 1, "cudaMalloc(error word)");
-    check_cuda(cudaMemset(p->d_err, 0, 4), "memset");
+    p->d_err = dalloc<uint32_t>(p, kPlanWords, "cudaMalloc(error word)");
+    check_cuda(cudaMemset(p->d_err, 0, kPlanWords * 4), "memset");
 
     trace.mark("  plan: baseline, maps");
     if (p->engine == GNM_ENGINE_PLAIN) {
@@ -538,7 +539,7 @@ static void plan_reset_impl(gnm_plan* p, cudaStream_t s) {
   } else {
     tensor_reset(p, s);
   }
-  check_cuda(cudaMemsetAsync(p->d_err, 0, 4, s), "reset error word");
+  check_cuda(cudaMemsetAsync(p->d_err, 0, kPlanWords * 4, s), "reset error word");
   p->launches = 0;
 }
 
@@ -1277,8 +1278,8 @@ static gnm_plan* plan_create_projection(int device, uint64_t n, uint64_t K, uint
                "upload baseline");
     p->d_zero_base = dalloc<double>(p, K, "cudaMalloc(zero baseline)");
     check_cuda(cudaMemset(p->d_zero_base, 0, K * sizeof(double)), "memset");
-    p->d_err = dalloc<uint32_t>(p, 1, "cudaMalloc(error word)");
-    check_cuda(cudaMemset(p->d_err, 0, 4), "memset");
+    p->d_err = dalloc<uint32_t>(p, kPlanWords, "cudaMalloc(error word)");
+    check_cuda(cudaMemset(p->d_err, 0, kPlanWords * 4), "memset");
     plain_geometry(p);
     upload_plain_records(p, rec, trace);
     check_cuda(cudaStreamSynchronize(0), "plan upload");

@@ -78,6 +78,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
   return mbar_wait_timed(bar, parity, kWaitLimitNs);
 }
 
+// The same by a whole converged warp, with a warp-uniform answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xFFFFFFFFu, mbar_wait_bounded(bar, parity));
+}
+
 // ---- clusters ----------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;

@@ -115,9 +115,14 @@ uint64_t pgen_samples(const gnm_pgen* pg);
 uint64_t pgen_variants(const gnm_pgen* pg);
 
 CUtensorMap make_row_map(const uint8_t* d_rows, uint64_t bytes_per_row, uint64_t num_rows,
-                         uint64_t pitch, uint32_t box_x, uint32_t box_y);
+                         uint64_t pitch, uint32_t box_x, uint32_t box_y,
+                         CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE);
 
 }  // namespace gnm
+
+// Words at gnm_plan::d_err that every reset clears: the error word, then the
+// narrow tensor engine's slot state.
+constexpr uint32_t kPlanWords = 4;
 
 struct gnm_plan {
   int device = 0;

@@ -28,6 +28,18 @@ __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// One lane of a converged warp, and a warp-uniform branch for the compiler: what
+// the lane issues is addressed from uniform registers.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 // D[tmem] (+)= A[smem desc] * B[smem desc]; BF16 inputs, FP32 accumulation.
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
                                            uint32_t idesc, uint32_t accumulate) {
@@ -48,6 +60,44 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint6
       "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// D (S32, TMEM) (+)= A x B with 8-bit integer operands, A in tensor memory (lane =
+// row, one 32-bit column per four consecutive K bytes: eight columns per MMA), B
+// in shared memory.
+__device__ __forceinline__ void tc_mma_i8_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
+                                             uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// 16 lanes x 32 32-bit columns from 16 registers per thread: thread l's registers
+// 2c and 2c + 1 go to lanes l / 4 and l / 4 + 8, column 4c + l % 4.
+__device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
+      "%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_wait() {
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// Two 16 x 16 byte matrices, transposed (lane l holds the address of row l % 16 of
+// matrix l / 16, 16-byte aligned): thread l's register 2m + h is rows
+// 4 (l % 4) .. + 3 (one per byte) of column l / 4 + 8 h of matrix m.
+__device__ __forceinline__ void ldmatrix_t_b8(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
 }
 
 // ---- SM pairs (cta_group::2): one MMA spans the two CTAs of a cluster ----
@@ -165,6 +215,11 @@ __host__ __device__ constexpr uint32_t idesc_s8u8_s32(uint32_t M, uint32_t N) {
 // bytes either way).
 __host__ __device__ constexpr uint32_t idesc_s8s8_s32(uint32_t M, uint32_t N) {
   return (2u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
+}
+
+// kind::i8 with unsigned A and signed B.
+__host__ __device__ constexpr uint32_t idesc_u8s8_s32(uint32_t M, uint32_t N) {
+  return (2u << 4) | (0u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
 // 3D tiled TMA load (x innermost; x * element size must be a multiple of 16).

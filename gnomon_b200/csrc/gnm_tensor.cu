@@ -71,11 +71,16 @@ struct TensorPlan {
   uint32_t ptiles = 0, stiles = 0;
   __nv_bfloat16* d_planes_dos = nullptr;  // [4][K_pad][V_pad] W' limbs
   __nv_bfloat16* d_planes_mis = nullptr;  // [4][K_pad][V_pad] -corr limbs, member
-  double* d_part_sum = nullptr;           // wide: [K_pad][P_pad]; narrow: [nsplits][K16][P_pad]
+  double* d_part_sum = nullptr;           // wide: [K_pad][P_pad]; narrow: [slots][K16][P_nar]
   uint32_t* d_part_cnt = nullptr;
   uint64_t part_elems = 0;                // elements of d_part_sum / d_part_cnt
-  uint32_t nsplits = 1;                   // narrow: variant splits (grid z)
-  uint64_t nslot = 0;                     // narrow: elements per split slot (K16 * P_pad)
+  uint32_t nsplits = 1;                   // narrow BF16: variant splits (grid z)
+  uint64_t P_nar = 0;                     // narrow: people rounded up to 512
+  uint64_t nslot = 0;                     // narrow: elements per slot (K16 * P_nar)
+  uint32_t nalloc = 0;                    // narrow: slots allocated
+  uint32_t ncta = 1;                      // narrow 8-bit: CTAs per score tile
+  uint32_t* d_state = nullptr;            // narrow: slot state (slots_written)
+  bool wide_clear = false;                // wide partials cleared since the last reset
   CUtensorMap map_dos, map_mis;
   int8_t* d_planes8 = nullptr;            // [9][K_pad][V_pad8] 8-bit limbs (dosage, -corr, member)
   double* d_quanta8 = nullptr;            // [9][K_pad] quantum of each 8-bit plane
@@ -1290,80 +1295,166 @@ __global__ void __launch_bounds__(kNrThreads, 1)
 }
 
 // ---- narrow engine on 8-bit limbs -------------------------------------------------
-// gnm_tc_narrow with tcgen05.mma kind::i8: M = 128 people, N = 16 scores x
-// the 8-bit planes of each operand (row n = 16 * plane + score, one 3D TMA box
-// of the wide engine's [9][K_pad][V] limb planes: dosage limbs 0-3, N = 64;
-// correction limbs 0-3 and the member plane, N = 80), K = 128 variants per
-// stage.  Per 32-variant slice two MMAs, the dosage operand against the
-// dosage limbs and the missing indicator against the rest, into 64 + 80 S32
-// accumulator columns.  Every operand byte is half the BF16 kernel's, which is what
-// bounds that kernel: its stage time is set by shared-memory traffic (TMA
-// writes, operand stores, MMA operand reads), not by the MMAs.  The TMA ring
-// (limb planes + packed rows) runs ST stages deep beside a two-deep ring of
-// expanded operands, as in gnm_t8_accumulate; sums stay exact in S32 for
-// blocks of up to 2^23 variants and reach the FP64 partials of the CTA's
-// variant split (natural person order) once per block.
-constexpr int kT8NrStages = 5;
+// Few score columns on tcgen05.mma kind::i8 with people as M: the genotype
+// operand A is expanded straight into TENSOR MEMORY, never into shared memory.
+//
+// What bounds it: with A in shared memory (the form this kernel replaced) a
+// stage stored and re-read 64 KB of expanded operands per 128 people x 128
+// variants, and shared-memory traffic, not the MMAs, set its time (tensor pipe
+// 21 % busy).  Here the packed bytes are all that crosses shared memory:
+//
+//   * ldmatrix.m16n16.trans.b8 reads 16 variants x 16 packed bytes and hands
+//     lane l the bytes of four consecutive variants, 4 (l % 4) ..., of byte
+//     column l / 4 (and l / 4 + 8): one register is 4 variants x 4 people;
+//   * per register, S = x >> 1 and D = x - ((x | S) & 0x55555555) give the
+//     dosage fields (codes 00, 01, 10, 11 -> 0, 0, 1, 2); person q's operand word is
+//     D & (0x03030303 << 2q) and its missing word x & ~S & (0x01010101 << 2q):
+//     the field stays where it is, so person q's row is 4^q times its value,
+//     and the epilogue's quantum takes 4^-q (a power of two: exact).  11
+//     integer instructions per 16 genotypes and both operands;
+//   * tcgen05.st.16x128b has the same fragment layout (lane l: TMEM row l / 4
+//     and l / 4 + 8, 32-bit column l % 4), so the registers go to tensor memory
+//     with no shuffle.  Byte column r of a warp's 8 is people 4r .. 4r + 3 on
+//     TMEM lanes r, r + 8, r + 16, r + 24 of the warp's lane quadrant.
+//
+// Dosage limbs and correction limbs share their quanta (max over both), so
+// both products add into the SAME 64 accumulator columns (limb j, score s:
+// column 16 j + s), and the member plane gets 16 more: 80 columns per 128
+// people.  That leaves room for NMT = 4 blocks of 128 people per CTA (320
+// columns) beside a three-slot ring of operands (64 columns per 32 variants),
+// and every 18 KB of limbs staged from L2 feeds 512 people instead of 128.
+// NMT = 2 (256 people, eight slots) takes the cohorts and calls too small to
+// fill the chip with 512-person tiles.
+//
+// Work is split evenly, not by tiles: a CTA takes `quota` consecutive
+// (people tile, stage) units of its score tile, so one CTA covers the tail of
+// one tile and the head of the next and every SM finishes together; each of
+// a tile's few segments writes its own FP64 slot.  CTAs of different score
+// tiles walk the rows in step and share them in L2.
+//
+// S32 sums are exact for 2^17 variants: |limb x 4^q x dosage| <= 127 x 128.
+constexpr uint32_t kT8NrScoreRows = 4 * kNrScores;   // limb rows of one operand
+constexpr uint32_t kT8NrCols = 5 * kNrScores;        // accumulator columns per 128 people
+constexpr uint32_t kT8NrFlush = 1024;                // stages per exact S32 block (2^17 variants)
+constexpr uint32_t kT8NrGroups = 4;                  // expansion warps per TMEM lane quadrant
+constexpr uint32_t kT8NrThreads = 128 + 128 * kT8NrGroups;   // TMA, two MMA warps, one idle
 
-constexpr uint32_t kT8NrNDos = 4 * kNrScores;   // dosage limbs 0-3
-constexpr uint32_t kT8NrNMis = 5 * kNrScores;   // correction limbs 0-3, member plane
-
+template <int NMT>
 struct T8NrSmem {
-  static constexpr uint32_t kBStages = 2;
-  static constexpr uint32_t kA = kNrM * kT8K;               // 16 KB per operand (people rows)
-  static constexpr uint32_t kPkRow = kNrM / 4;              // 32 packed bytes per variant row
-  static constexpr uint32_t kPk = kT8K * kPkRow;            // 4 KB
+  static constexpr uint32_t kStages = NMT == 4 ? 6 : 8;
+  static constexpr uint32_t kSlots = NMT == 4 ? 3 : 8;      // operand ring, 32 variants each
+  static constexpr uint32_t kSlotCols = 16 * NMT;           // 8 dosage + 8 missing per block
+  static constexpr uint32_t kParts = NMT / 2;               // a slot's parts: two blocks each
+  static constexpr uint32_t kRing0 = kT8NrCols * NMT;       // first operand column
+  static constexpr uint32_t kPeople = kNrM * NMT;
+  static constexpr uint32_t kPkRow = kPeople / 4;           // packed bytes per variant row
+  static constexpr uint32_t kPk = kT8K * kPkRow;
   static constexpr uint32_t kBDos = 0;                      // offsets inside a TMA stage
-  static constexpr uint32_t kBMis = kT8NrNDos * kT8K;       // 8 KB
-  static constexpr uint32_t kPkIn = kBMis + kT8NrNMis * kT8K;   // + 10 KB
-  static constexpr uint32_t kTma = kPkIn + kPk;             // one TMA stage: 22 KB
-  static constexpr uint32_t kAOff = kT8NrStages * kTma;     // operand ring
-  static constexpr uint32_t kBarOff = kAOff + kBStages * 2 * kA;
-  static constexpr uint32_t kHolder = kBarOff + 8 * (2 * kT8NrStages + 2 * kBStages + 2);
-  static constexpr uint32_t kTotal = kHolder + 16 + 1024;  // + alignment slack
+  static constexpr uint32_t kBMis = kT8NrScoreRows * kT8K;  // 8 KB
+  static constexpr uint32_t kPkIn = kBMis + kT8NrCols * kT8K;   // + 10 KB
+  static constexpr uint32_t kTma = kPkIn + kPk;             // 34 / 26 KB
+  static constexpr uint32_t kBarOff = kStages * kTma;
+  static constexpr uint32_t kBars = 2 * kStages + 2 * kSlots * kParts + 4;
+  static constexpr uint32_t kHolder = kBarOff + 8 * kBars;
+  static constexpr uint32_t kTotal = kHolder + 16 + 1024;   // + alignment slack
   static_assert(kTotal <= 227 * 1024, "shared memory");
-  static_assert(kTma % 1024 == 0 && kAOff % 1024 == 0 && kBMis % 1024 == 0 && kPkIn % 1024 == 0,
-                "operand alignment");
+  static_assert(kTma % 1024 == 0 && kBMis % 1024 == 0 && kPkIn % 1024 == 0, "operand alignment");
+  static_assert(kRing0 + kSlots * kSlotCols <= 512, "tensor memory columns");
 };
 
-__global__ void __launch_bounds__(kNrThreads, 1)
+// Slots of the narrow engine's partials that hold sums since the last reset, kept
+// on the device so that a reset is one small memset and a captured call behaves
+// as a plain one: a kernel writes the slots from `valid` on and adds to the
+// others, and its last CTA (every CTA has read `valid` by then) moves `valid` up.
+//   state[0] = valid, state[1] = CTAs of the running launch that are done
+__device__ __forceinline__ void slots_written(uint32_t* state, uint32_t slots, uint32_t ctas) {
+  __threadfence();
+  if (atomicAdd(state + 1, 1u) == ctas - 1) {
+    state[1] = 0u;
+    if (state[0] < slots) state[0] = slots;
+  }
+}
+
+// Zeroes slots valid .. slots - 1 ahead of a kernel that only adds.
+__global__ void gnm_tc_open_slots(double* sum, uint32_t* cnt, uint64_t slot_stride,
+                                  uint32_t slots, uint32_t* state) {
+  const uint32_t valid = *reinterpret_cast<volatile uint32_t*>(state);
+  const uint64_t end = uint64_t(slots) * slot_stride;
+  for (uint64_t x = valid * slot_stride + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < end;
+       x += uint64_t(gridDim.x) * blockDim.x) {
+    sum[x] = 0.0;
+    cnt[x] = 0u;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) slots_written(state, slots, gridDim.x);
+}
+
+struct T8NrArgs {
+  uint64_t num_rows;       // rows of this block
+  int32_t a_x0;            // absolute variant index of block row 0 (multiple of 128)
+  double* part_sum;        // [slots][K rounded to 16][P_pad]
+  uint32_t* part_cnt;
+  uint64_t P_pad;
+  uint64_t slot_stride;    // elements per slot
+  uint32_t* err;
+  uint32_t stages;         // stages of the block (128 variants each)
+  uint32_t ptiles;         // people tiles
+  uint32_t quota;          // (people tile, stage) units per CTA
+  uint32_t slots;          // slots of every tile; those without a segment are zeroed
+  uint32_t* state;         // {slots written since the reset, CTAs done}: see SlotState
+  const double* quanta;    // [kT8Planes][K_pad]
+  uint64_t K_pad;
+};
+
+template <int NMT>
+__global__ void __launch_bounds__(kT8NrThreads, 1)
     gnm_t8_narrow(const __grid_constant__ CUtensorMap dmap,
                   const __grid_constant__ CUtensorMap mmap,
-                  const __grid_constant__ CUtensorMap pmap, NrArgs a, const double* quanta,
-                  uint64_t K_pad) {
-  using L = T8NrSmem;
-  constexpr uint32_t ST = kT8NrStages;
-  constexpr uint32_t BS = L::kBStages;
+                  const __grid_constant__ CUtensorMap pmap, T8NrArgs a) {
+  using L = T8NrSmem<NMT>;
+  constexpr uint32_t ST = L::kStages, R = L::kSlots, RP = R * L::kParts;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sb = smem_u32(smem);
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t ptile = blockIdx.x, stile = blockIdx.y, split = blockIdx.z;
-  const uint32_t nall = uint32_t((a.num_rows + kT8K - 1) / kT8K);
-  const uint32_t it0 = split * a.stages_per_split;
-  const uint32_t nit = it0 < nall ? min(a.stages_per_split, nall - it0) : 0u;
-  auto full = [&](uint32_t s) { return sb + L::kBarOff + 8 * s; };
-  auto tempty = [&](uint32_t s) { return sb + L::kBarOff + 8 * (ST + s); };
-  auto bready = [&](uint32_t b) { return sb + L::kBarOff + 8 * (2 * ST + b); };
-  auto bempty = [&](uint32_t b) { return sb + L::kBarOff + 8 * (2 * ST + BS + b); };
-  const uint32_t accfull = sb + L::kBarOff + 8 * (2 * ST + 2 * BS);
-  const uint32_t accempty = sb + L::kBarOff + 8 * (2 * ST + 2 * BS + 1);
+  const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t stile = blockIdx.y;
+  const uint64_t units = uint64_t(a.ptiles) * a.stages;
+  const uint64_t u0 = uint64_t(blockIdx.x) * a.quota;
+  const uint64_t u1 = u0 + a.quota < units ? u0 + a.quota : units;
+  if (u0 >= u1) return;   // uniform per CTA (the host launches none such)
+  auto full = [&](uint32_t s) { return sb + L::kBarOff + 8 * s; };           // TMA landed
+  auto tempty = [&](uint32_t s) { return sb + L::kBarOff + 8 * (ST + s); };  // stage free
+  // part p of operand slot b: filled by its four warps / read by its MMAs
+  auto ready = [&](uint32_t b, uint32_t p) {
+    return sb + L::kBarOff + 8 * (2 * ST + b * L::kParts + p);
+  };
+  auto sfree = [&](uint32_t b, uint32_t p) {
+    return sb + L::kBarOff + 8 * (2 * ST + RP + b * L::kParts + p);
+  };
+  const uint32_t accfull = sb + L::kBarOff + 8 * (2 * ST + 2 * RP);
+  const uint32_t accempty = accfull + 8, drain0 = accfull + 16;   // one drain per MMA warp
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kHolder + 8);
   const uint32_t abort_addr = sb + L::kHolder + 8;
-  if (nit == 0) return;   // a split past the block's last stage (uniform per CTA)
+  auto give_up = [&](uint32_t code) {
+    *abort_flag = 1u;
+    atomicOr(a.err, code);
+  };
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < ST; ++s) {
       mbar_init(full(s), 1);
-      mbar_init(tempty(s), 1);
+      mbar_init(tempty(s), 2);   // both MMA warps
     }
-    for (uint32_t b = 0; b < BS; ++b) {
-      mbar_init(bready(b), kNrExpand);
-      mbar_init(bempty(b), 1);
-    }
-    mbar_init(accfull, 1);
-    mbar_init(accempty, kNrExpand);
+    for (uint32_t b = 0; b < R; ++b)
+      for (uint32_t p = 0; p < L::kParts; ++p) {
+        mbar_init(ready(b, p), 4);
+        mbar_init(sfree(b, p), 2 / L::kParts);
+      }
+    mbar_init(accfull, 2);
+    mbar_init(accempty, 4 * kT8NrGroups);
+    mbar_init(drain0, 1);
+    mbar_init(drain0 + 8, 1);
     *abort_flag = 0u;
     fence_mbar_init();
     prefetch_tmap(&dmap);
@@ -1371,7 +1462,7 @@ __global__ void __launch_bounds__(kNrThreads, 1)
     prefetch_tmap(&pmap);
   }
   if (warp == 1) {
-    tmem_alloc(sb + L::kHolder, 256);   // 64 + 80 columns
+    tmem_alloc(sb + L::kHolder, 512);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -1382,164 +1473,266 @@ __global__ void __launch_bounds__(kNrThreads, 1)
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      for (uint32_t it = 0; it < nit; ++it) {
-        const uint32_t s = it % ST, ph = (it / ST) & 1u;
+      uint32_t n = 0;            // stages issued
+      uint32_t tile = uint32_t(u0 / a.stages), st = uint32_t(u0 % a.stages);
+      bool ok = true;
+      for (uint64_t u = u0; u < u1; ++u, ++n) {
+        const uint32_t s = n % ST, ph = (n / ST) & 1u;
         if (!mbar_wait_bounded(tempty(s), ph ^ 1u)) {
-          *abort_flag = 1u;
-          atomicOr(a.err, kErrMmaTimeout);
+          give_up(kErrMmaTimeout);
+          ok = false;
           break;
         }
-        if (lds_volatile_u32(abort_addr)) break;
-        const uint32_t st = sb + s * L::kTma;
+        if (lds_volatile_u32(abort_addr)) {
+          ok = false;
+          break;
+        }
+        const uint32_t at = sb + s * L::kTma;
         mbar_arrive_expect_tx(full(s), L::kTma);
-        const int32_t x = a.a_x0 + int32_t((it0 + it) * kT8K);
-        tma_load_3d(st + L::kBDos, &dmap, x, int32_t(stile * kNrScores), 0, full(s));
-        tma_load_3d(st + L::kBMis, &mmap, x, int32_t(stile * kNrScores), 4, full(s));
-        tma_load_2d(st + L::kPkIn, &pmap, int32_t(ptile * L::kPkRow),
-                    int32_t((it0 + it) * kT8K), full(s));
+        const int32_t x = a.a_x0 + int32_t(st * kT8K);
+        tma_load_2d(at + L::kPkIn, &pmap, int32_t(tile * L::kPkRow), int32_t(st * kT8K), full(s));
+        tma_load_3d(at + L::kBMis, &mmap, x, int32_t(stile * kNrScores), 4, full(s));
+        tma_load_3d(at + L::kBDos, &dmap, x, int32_t(stile * kNrScores), 0, full(s));
+        if (++st == a.stages) {
+          st = 0;
+          ++tile;
+        }
       }
+      if (!ok)   // nothing may still be in flight when the CTA exits (bounded)
+        for (uint32_t i = n > ST ? n - ST : 0; i < n; ++i)
+          mbar_wait_bounded(full(i % ST), (i / ST) & 1u);
     }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc_d = idesc_s8s8_s32(kNrM, kT8NrNDos);
-      constexpr uint32_t idesc_m = idesc_s8s8_s32(kNrM, kT8NrNMis);
-      uint32_t blk = 0;
-      for (uint32_t it = 0; it < nit; ++it) {
-        const uint32_t s = it % ST;
-        const uint32_t bsl = it % BS, bph = (it / BS) & 1u;
-        const bool first = (it % kT8Flush) == 0;
-        if (first && it > 0) {
-          if (!mbar_wait_bounded(accempty, (blk - 1) & 1u)) {
-            *abort_flag = 1u;
-            atomicOr(a.err, kErrMmaTimeout);
-            break;
+  } else if (warp == 1 || warp == 2) {
+    // ---------------- MMA issuers ----------------
+    // Warp 1 + i issues the MMAs of people blocks i NMT / 2 ...  Issue is what a
+    // single warp runs out of: an MMA of these shapes takes 37 clocks, the
+    // tensor core queues only a few, and each wait costs the warp about 90, so
+    // one warp left the pipe idle for 40 % of a stage (2,000 clocks instead of
+    // 1,200); two cover each other's waits.  Each whole warp runs the loop, with
+    // votes for conditions, and one elected lane issues: addresses and
+    // descriptors then stay in uniform registers, which tcgen05.mma reads (a
+    // loop that only lane 0 runs moves each over per instruction: 60 clocks per
+    // MMA).
+    constexpr uint32_t idesc_d = idesc_u8s8_s32(kNrM, kT8NrScoreRows);
+    constexpr uint32_t idesc_m = idesc_u8s8_s32(kNrM, kT8NrCols);
+    constexpr uint32_t kMine = NMT / 2;                  // blocks of this warp
+    const uint32_t b0 = (warp - 1) * kMine;
+    const uint32_t part = NMT == 4 ? warp - 1 : 0u;
+    uint32_t st = uint32_t(u0 % a.stages), blk = 0, inblk = 0, n = 0, slot = 0, sph = 0;
+    const uint32_t left = uint32_t(u1 - u0);
+    const uint32_t utmem = __shfl_sync(0xFFFFFFFFu, tmem, 0);
+    bool ok = true;
+    for (; n < left && ok; ++n) {
+      const uint32_t s = n % ST;
+      if (inblk == 0 && blk > 0 && !mbar_wait_warp(accempty, (blk - 1) & 1u)) {
+        give_up(kErrMmaTimeout);
+        ok = false;
+        break;
+      }
+      const uint32_t at = sb + s * L::kTma;
+      const uint64_t bm0 = desc_kmajor_sw128(at + L::kBMis);
+      const uint64_t bd0 = desc_kmajor_sw128(at + L::kBDos);
+      const bool last = st + 1 == a.stages || inblk + 1 == kT8NrFlush || n + 1 == left;
+#pragma unroll
+      for (uint32_t kk = 0; kk < kT8K / 32; ++kk) {   // 32 variants per slot and MMA
+        // the warps that filled the slot waited for the stage's limbs too
+        if (!mbar_wait_warp(ready(slot, part), sph)) {
+          give_up(kErrMmaTimeout);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t bm = bm0 + 2 * kk, bd = bd0 + 2 * kk;   // 32 bytes further
+          const uint32_t op = utmem + L::kRing0 + slot * L::kSlotCols + 16 * b0;
+          const uint32_t d = utmem + kT8NrCols * b0;
+          // the missing product covers all 80 columns, so it starts a block
+          const uint32_t acc = (inblk == 0 && kk == 0) ? 0u : 1u;
+#pragma unroll
+          for (uint32_t t = 0; t < kMine; ++t)
+            tc_mma_i8_ta(d + t * kT8NrCols, op + 16 * t + 8, bm, idesc_m, acc);
+#pragma unroll
+          for (uint32_t t = 0; t < kMine; ++t)
+            tc_mma_i8_ta(d + t * kT8NrCols, op + 16 * t, bd, idesc_d, 1u);
+          tc_commit(sfree(slot, part));
+          if (kk == kT8K / 32 - 1) {
+            tc_commit(tempty(s));
+            if (last) tc_commit(accfull);
           }
         }
-        if (!mbar_wait_bounded(bready(bsl), bph)) {
-          *abort_flag = 1u;
-          atomicOr(a.err, kErrMmaTimeout);
-          break;
+        __syncwarp();
+        if (++slot == R) {
+          slot = 0;
+          sph ^= 1u;
         }
-        if (lds_volatile_u32(abort_addr)) break;
-        tc_fence_after();
-        const uint32_t st = sb + s * L::kTma;
-        const uint32_t ad = sb + L::kAOff + bsl * 2 * L::kA;
-        const uint32_t am = ad + L::kA;
-#pragma unroll
-        for (uint32_t kk = 0; kk < kT8K / 32; ++kk) {   // K = 32 bytes per MMA
-          const uint32_t acc = (first && kk == 0) ? 0u : 1u;
-          tc_mma_i8(tmem, desc_kmajor_sw128(ad + kk * 32),
-                    desc_kmajor_sw128(st + L::kBDos + kk * 32), idesc_d, acc);
-          tc_mma_i8(tmem + kT8NrNDos, desc_kmajor_sw128(am + kk * 32),
-                    desc_kmajor_sw128(st + L::kBMis + kk * 32), idesc_m, acc);
-        }
-        tc_commit(tempty(s));
-        tc_commit(bempty(bsl));
-        if ((it % kT8Flush) == kT8Flush - 1 || it == nit - 1) {
-          tc_commit(accfull);
-          ++blk;
-        }
+      }
+      ++inblk;
+      if (++st == a.stages) st = 0;
+      if (last) {   // end of a block
+        ++blk;
+        inblk = 0;
       }
     }
-  } else {
-    // ---------------- genotype expansion + epilogue (warps 2-9) ----------------
-    // warp 2 + e: 16-variant chunk e of the stage; lane = byte column (people
-    // 4 lane .. 4 lane + 3); both operands from the same packed bytes
-    const uint32_t c = warp - 2;
-    const uint32_t col = lane;
-    const uint32_t quad = warp & 3;         // TMEM lane quadrant of this warp
-    const uint32_t half = (warp - 2) >> 2;  // epilogue: scores 8 half .. 8 half + 7
-    double* ps = a.part_sum + uint64_t(split) * a.slot_stride;
-    uint32_t* pc = a.part_cnt + uint64_t(split) * a.slot_stride;
-    uint32_t blk = 0;
-    for (uint32_t it = 0; it < nit; ++it) {
-      const uint32_t s = it % ST, ph = (it / ST) & 1u;
-      const uint32_t bsl = it % BS, bph = (it / BS) & 1u;
+    // after a failure (this warp's or another's) the issued MMAs finish before the
+    // CTA's memory goes (bounded)
+    if (!ok) {
+      const uint32_t drain = drain0 + 8 * (warp - 1);
+      if (elect_one()) tc_commit(drain);
+      __syncwarp();
+      mbar_wait_bounded(drain, 0);
+    }
+  } else if (warp >= 4) {
+    // ---------------- genotype expansion + epilogue (warps 4-19) ----------------
+    const uint32_t quad = warp & 3;          // TMEM lane quadrant of this warp
+    const uint32_t grp = (warp - 4) >> 2;    // 0..3
+    // 512 people: a warp takes every second slot and half of its quadrant's
+    // 32 packed bytes; 256 people: every fourth slot, all 16 bytes
+    constexpr uint32_t kEvery = NMT == 4 ? 2 : 4;
+    const uint32_t mine = NMT == 4 ? (grp & 1u) : grp;
+    const uint32_t pairm = NMT == 4 ? (grp >> 1) : 0u;       // blocks 2 pairm, 2 pairm + 1
+    const uint32_t chunk = (NMT / 2) * quad + pairm;         // 16-byte chunk of the row
+    // this lane's ldmatrix row in the first of its slots (rows 32 apart keep
+    // the swizzle's row bits), and the operand columns of the warp's blocks
+    const uint32_t row = 32 * mine + lane;
+    const uint32_t pk0 = sb + L::kPkIn + row * L::kPkRow +
+                         ((NMT == 4 ? (chunk ^ (row & 7u)) : (chunk ^ ((row >> 1) & 3u))) << 4);
+    const uint32_t op0 = tmem + ((32 * quad) << 16) + L::kRing0 + 32 * pairm;
+    uint32_t tile = uint32_t(u0 / a.stages), st = uint32_t(u0 % a.stages);
+    uint32_t blk = 0, inblk = 0, n = 0, slot = mine, sph = 0;
+    bool first = true;   // the segment's first block
+    const uint64_t valid = *reinterpret_cast<volatile uint32_t*>(a.state);
+    for (uint64_t u = u0; u < u1; ++u, ++n) {
+      const uint32_t s = n % ST, ph = (n / ST) & 1u;
       if (!mbar_wait_bounded(full(s), ph)) {
-        *abort_flag = 1u;
-        atomicOr(a.err, kErrTmaTimeout);
+        give_up(kErrTmaTimeout);
         break;
       }
-      if (!mbar_wait_bounded(bempty(bsl), bph ^ 1u)) {
-        *abort_flag = 1u;
-        atomicOr(a.err, kErrMmaTimeout);
-        break;
-      }
-      if (lds_volatile_u32(abort_addr)) break;
-      const uint32_t pk = sb + s * L::kTma + L::kPkIn;
-      const uint32_t ad = sb + L::kAOff + bsl * 2 * L::kA;
-      const uint32_t am = ad + L::kA;
-      {
-        uint32_t x[4] = {0u, 0u, 0u, 0u};
+      constexpr uint32_t kTurns = 4 / kEvery;   // this warp's slots of the stage
+      uint32_t x[kTurns][4];   // [16 variants each][byte columns 0-7, 8-15]
 #pragma unroll
-        for (uint32_t i = 0; i < 16; ++i)
-          x[i >> 2] |= lds_u8(pk + (16 * c + i) * L::kPkRow + col) << (8 * (i & 3));
-        uint32_t xd[4], xm[4];
+      for (uint32_t j = 0; j < kTurns; ++j)
+        ldmatrix_t_b8(pk0 + s * L::kTma + j * (32 * kEvery * L::kPkRow), x[j]);
+      const uint32_t aborted = lds_volatile_u32(abort_addr);
+      bool ok = true;
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-          xd[i] = code_fields<false>(x[i]);
-          xm[i] = code_fields<true>(x[i]);
+      for (uint32_t j = 0; j < kTurns; ++j) {
+        // columns of block h: dosage of variants 0-15, 16-31, missing likewise;
+        // lo: people 0 and 1 of every byte, hi: people 2 and 3
+        uint32_t lo[16], hi[16];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) {
+#pragma unroll
+          for (uint32_t c = 0; c < 2; ++c) {
+            const uint32_t xc = x[j][2 * c + h], sc = xc >> 1;
+            const uint32_t dc = xc - ((xc | sc) & 0x55555555u);
+            const uint32_t at = 8 * h + 2 * c;
+            lo[at] = dc & 0x03030303u;
+            lo[at + 1] = dc & 0x0C0C0C0Cu;
+            hi[at] = dc & 0x30303030u;
+            hi[at + 1] = dc & 0xC0C0C0C0u;
+            lo[at + 4] = xc & ~sc & 0x01010101u;
+            lo[at + 5] = xc & ~sc & 0x04040404u;
+            hi[at + 4] = xc & ~sc & 0x10101010u;
+            hi[at + 5] = xc & ~sc & 0x40404040u;
+          }
         }
-#pragma unroll
-        for (uint32_t q = 0; q < 4; ++q) {
-          uint4 vd, vm;
-          vd.x = (xd[0] >> (2 * q)) & 0x03030303u;
-          vd.y = (xd[1] >> (2 * q)) & 0x03030303u;
-          vd.z = (xd[2] >> (2 * q)) & 0x03030303u;
-          vd.w = (xd[3] >> (2 * q)) & 0x03030303u;
-          vm.x = (xm[0] >> (2 * q)) & 0x03030303u;
-          vm.y = (xm[1] >> (2 * q)) & 0x03030303u;
-          vm.z = (xm[2] >> (2 * q)) & 0x03030303u;
-          vm.w = (xm[3] >> (2 * q)) & 0x03030303u;
-          // operand row of person 4col + q (conflict-free 16-byte stores)
-          const uint32_t n = 32 * q + col;
-          const uint32_t off = (n >> 3) * 1024 + (n & 7) * 128 + ((c ^ (n & 7)) << 4);
-          sts_u128(ad + off, vd);
-          sts_u128(am + off, vm);
-        }
-      }
-      fence_proxy_async_smem();
-      mbar_arrive(bready(bsl));
-
-      if ((it % kT8Flush) == kT8Flush - 1 || it == nit - 1) {
-        if (!mbar_wait_bounded(accfull, blk & 1u)) {
-          *abort_flag = 1u;
-          atomicOr(a.err, kErrMmaTimeout);
+        if (!mbar_wait_bounded(sfree(slot, pairm), sph ^ 1u)) {
+          give_up(kErrMmaTimeout);
+          ok = false;
           break;
         }
         tc_fence_after();
-        // TMEM lane 32 quad + lane = operand row n -> person 4 (n % 32) + n / 32.
-        // Column group g (16 columns): dosage limbs 0-3, -C limbs 0-3, member
-        // (plane g of the limb planes); this thread reads its 8 scores of
-        // every group.
-        const uint64_t person = uint64_t(ptile) * kNrM + 4 * lane + quad;
-        const uint32_t lane_base = tmem + ((32 * quad) << 16) + 8 * half;
-        const uint64_t k0 = uint64_t(stile) * kNrScores + 8 * half;
-        double acc[8];
-        uint32_t cnt[8];
+        const uint32_t op = op0 + slot * L::kSlotCols;
+        tmem_st_16x128b_x8(op, lo);
+        tmem_st_16x128b_x8(op + (16u << 16), hi);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ready(slot, pairm));
+        slot += kEvery;
+        if (slot >= R) {
+          slot -= R;
+          sph ^= 1u;
+        }
+      }
+      if (!ok || aborted) break;
+      ++inblk;
+      const uint32_t tile_now = tile;
+      const bool tile_end = ++st == a.stages;
+      if (tile_end) {
+        st = 0;
+        ++tile;
+      }
+      if (tile_end || inblk == kT8NrFlush || u + 1 == u1) {
+        // ---- epilogue: drain one 128-person block of the tile ----
+        inblk = 0;
+        if (!mbar_wait_bounded(accfull, blk & 1u)) {
+          give_up(kErrMmaTimeout);
+          break;
+        }
+        ++blk;
+        tc_fence_after();
+        const uint32_t t = grp % NMT;
+        const uint32_t q = lane >> 3;        // row scale 4^q
+        // TMEM lane 8q + r of quadrant `quad`, block t: person q of the
+        // quadrant's packed byte 8t + r
+        const uint64_t person = uint64_t(tile_now) * L::kPeople +
+                                4 * (8 * NMT * quad + 8 * t + (lane & 7u)) + q;
+        const uint32_t base = tmem + ((32 * quad) << 16) + t * kT8NrCols;
+        const double scale = 1.0 / double(1u << (2 * q));
+        const uint64_t first_cta = uint64_t(tile_now) * a.stages / a.quota;
+        const uint64_t sl = blockIdx.x - first_cta;
+        const bool write = sl >= valid && first;
+        const bool in = person < a.P_pad;
+        constexpr uint32_t kHalves = NMT == 4 ? 2 : 1;   // 256 people: two warps share a block
+#pragma unroll 1
+        for (uint32_t i = 0; i < kHalves; ++i) {
+          const uint32_t half = NMT == 4 ? i : (grp >> 1);
+          const uint64_t k0 = uint64_t(stile) * kNrScores + 8 * half;
+          double acc[8];
+          uint32_t cnt[8];
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) acc[k] = 0.0;
+          for (uint32_t k = 0; k < 8; ++k) acc[k] = 0.0;
 #pragma unroll
-        for (uint32_t g = 0; g < 9; ++g) {
-          uint32_t d[8];
-          tmem_ld8(lane_base + 16 * g, d);
-          tmem_ld_wait();
+          for (uint32_t g = 0; g < 5; ++g) {
+            uint32_t d[8];
+            tmem_ld8(base + 16 * g + 8 * half, d);
+            tmem_ld_wait();
 #pragma unroll
-          for (uint32_t k = 0; k < 8; ++k) {
-            if (g < 8) acc[k] = fma(double(int32_t(d[k])), quanta[g * K_pad + k0 + k], acc[k]);
-            else cnt[k] = d[k];
+            for (uint32_t k = 0; k < 8; ++k) {
+              if (g < 4)
+                acc[k] = fma(double(int32_t(d[k])), a.quanta[g * a.K_pad + k0 + k] * scale, acc[k]);
+              else
+                cnt[k] = d[k] >> (2 * q);
+            }
+          }
+          if (in) {
+            double* ps = a.part_sum + sl * a.slot_stride + k0 * a.P_pad + person;
+            uint32_t* pc = a.part_cnt + sl * a.slot_stride + k0 * a.P_pad + person;
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) {
+              if (write) {
+                ps[k * a.P_pad] = acc[k];
+                pc[k * a.P_pad] = cnt[k];
+              } else {
+                ps[k * a.P_pad] += acc[k];
+                pc[k * a.P_pad] += cnt[k];
+              }
+            }
+            if (tile_end) {   // the tile's last segment: zero its unused new slots
+              for (uint64_t z = sl + 1 > valid ? sl + 1 : valid; z < a.slots; ++z)
+#pragma unroll
+                for (uint32_t k = 0; k < 8; ++k) {
+                  ps[(z - sl) * a.slot_stride + k * a.P_pad] = 0.0;
+                  pc[(z - sl) * a.slot_stride + k * a.P_pad] = 0u;
+                }
+            }
           }
         }
         tc_fence_before();
-        mbar_arrive(accempty);
-        ++blk;
-#pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-          const uint64_t at = (k0 + k) * a.P_pad + person;
-          ps[at] += acc[k];
-          pc[at] += cnt[k];
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(accempty);
+        first = tile_end;
       }
     }
   }
@@ -1547,8 +1740,9 @@ __global__ void __launch_bounds__(kNrThreads, 1)
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 256);
+    tmem_dealloc(tmem, 512);
   }
+  if (threadIdx.x == 0) slots_written(a.state, a.slots, gridDim.x * gridDim.y);
 }
 
 // Limb planes from the CSR: one thread per variant.
@@ -1620,40 +1814,104 @@ __global__ void gnm_tc_build_planes(const float* w, const float* corr, const uin
   }
 }
 
-// out[o*K + k] = init[k] + part_sum[k][slot(fam(o))]; slot(f) is the operand
-// row of person f: tile (f / 256), row 128*h + 32*(r%4) + (r%128)/4 with
-// r = f % 256 and h = r / 128.  `pass` (may be null): the SM-pair kernel's
-// partials of passes 1-3, [3][pass_stride], added after part_sum in pass
-// order.  The narrow engine's epilogue writes in person order, one slot per
-// variant split: those slots are added in split order.
-__global__ void gnm_tc_finalize(const double* part_sum, const uint32_t* part_cnt, uint64_t P_pad,
-                                const double* init, const uint32_t* out_to_fam, uint64_t P,
-                                uint64_t K, uint32_t nslots, uint64_t slot_stride,
-                                const double* pass, uint64_t pass_stride, double* sums,
-                                uint32_t* counts) {
-  const uint64_t x = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (x >= P * K) return;
-  const uint64_t o = x / K, k = x % K;
-  const uint64_t f = out_to_fam ? out_to_fam[o] : o;
-  if (nslots == 0) {   // wide engine: one slot, operand-row order
-    const uint64_t r = f % kTcN, h = r / 128, rr = r % 128;
-    const uint64_t slot = (f / kTcN) * kTcN + 128 * h + 32 * (rr % 4) + rr / 4;
-    double s = part_sum[k * P_pad + slot];
-    if (pass)
-      for (uint32_t j = 0; j < 3; ++j) s += pass[j * pass_stride + k * P_pad + slot];
-    sums[x] = init[k] + s;
-    counts[x] = part_cnt[k * P_pad + slot];
-    return;
+// out[o*K + k] = init[k] + the sum over the partials of person fam(o).  The
+// partials are [score][person] and the output [person][score], so a CTA turns a
+// block of 32 people in shared memory: its loads are consecutive people of one
+// score, its stores consecutive scores of one person.  (One thread per output
+// read a different cache line per thread: 2.02 ms against 0.46 ms on 100,000
+// people x 512 scores, four FP64 arrays and the counts.)
+//
+// Wide engine: one value in operand-row order, slot(f) = tile (f / 256), row
+// 128*h + 32*(r%4) + (r%128)/4 with r = f % 256 and h = r / 128, plus the
+// SM-pair kernel's partials of passes 1-3 (`pass`, may be null:
+// [3][pass_stride]) in pass order.  Nothing accumulated since the reset
+// (`empty`): the initial value.
+constexpr uint32_t kFinTile = 32;
+__global__ void __launch_bounds__(256)
+    gnm_tc_finalize(const double* part_sum, const uint32_t* part_cnt, uint64_t P_pad,
+                    const double* init, const uint32_t* out_to_fam, uint64_t P, uint64_t K,
+                    const double* pass, uint64_t pass_stride, uint32_t empty, double* sums,
+                    uint32_t* counts) {
+  __shared__ double s_sum[kFinTile][kFinTile + 1];
+  __shared__ uint32_t s_cnt[kFinTile][kFinTile + 1];
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const uint64_t o0 = uint64_t(blockIdx.x) * kFinTile, k0 = uint64_t(blockIdx.y) * kFinTile;
+  constexpr uint32_t kPer = kFinTile / 8;   // scores per warp
+  const uint64_t o = o0 + lane;
+  const bool in = o < P && !empty;
+  const uint64_t f = !in ? 0 : (out_to_fam ? out_to_fam[o] : o);
+  const uint64_t fr = f % kTcN, h = fr / 128, rr = fr % 128;
+  const uint64_t at = (f / kTcN) * kTcN + 128 * h + 32 * (rr % 4) + rr / 4;
+#pragma unroll
+  for (uint32_t i = 0; i < kPer; ++i) {
+    const uint64_t k = k0 + w + 8 * i;
+    double acc = 0.0;
+    uint32_t cnt = 0;
+    if (in && k < K) {
+      acc = part_sum[k * P_pad + at];
+      cnt = part_cnt[k * P_pad + at];
+      if (pass)
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) acc += pass[j * pass_stride + k * P_pad + at];
+    }
+    s_sum[w + 8 * i][lane] = acc;
+    s_cnt[w + 8 * i][lane] = cnt;
   }
-  // narrow engine: natural order, variant-split slots added in split order
-  double s = 0.0;
-  uint32_t c = 0;
-  for (uint32_t z = 0; z < nslots; ++z) {
-    s += part_sum[z * slot_stride + k * P_pad + f];
-    c += part_cnt[z * slot_stride + k * P_pad + f];
+  __syncthreads();
+  const uint64_t k = k0 + lane;
+  if (k >= K) return;
+  const double base = init[k];
+#pragma unroll
+  for (uint32_t i = 0; i < kPer; ++i) {
+    const uint32_t r = w + 8 * i;
+    if (o0 + r < P) {
+      sums[(o0 + r) * K + k] = base + s_sum[lane][r];
+      counts[(o0 + r) * K + k] = s_cnt[lane][r];
+    }
   }
-  sums[x] = init[k] + s;
-  counts[x] = c;
+}
+
+// Narrow engine: person order, the slots written since the reset (`*state`).  A
+// CTA takes 32 people x 8 scores; two warps share a score, even and odd slots
+// four at a time, so the sum over a small cohort's many slots (48 of them: one
+// per CTA that met the tile) is a few memory latencies, and its order is fixed.
+constexpr uint32_t kSlotScores = 8, kSlotWarps = 2 * kSlotScores;
+__global__ void __launch_bounds__(32 * kSlotWarps)
+    gnm_tc_finalize_slots(const double* part_sum, const uint32_t* part_cnt, uint64_t P_pad,
+                          const double* init, const uint32_t* out_to_fam, uint64_t P, uint64_t K,
+                          const uint32_t* state, uint64_t slot_stride, double* sums,
+                          uint32_t* counts) {
+  __shared__ double s_sum[kSlotWarps][33];
+  __shared__ uint32_t s_cnt[kSlotWarps][33];
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const uint64_t o0 = uint64_t(blockIdx.x) * 32, k0 = uint64_t(blockIdx.y) * kSlotScores;
+  const uint64_t o = o0 + lane, k = k0 + w % kSlotScores;
+  const uint32_t nslots = *state, part = w / kSlotScores;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  uint32_t cnt = 0;
+  if (o < P && k < K) {
+    const uint64_t f = out_to_fam ? out_to_fam[o] : o;
+    const double* ps = part_sum + k * P_pad + f;
+    const uint32_t* pc = part_cnt + k * P_pad + f;
+    for (uint32_t z = part; z < nslots; z += 8) {
+#pragma unroll
+      for (uint32_t i = 0; i < 4; ++i)
+        if (z + 2 * i < nslots) {
+          acc[i] += ps[(z + 2 * i) * slot_stride];
+          cnt += pc[(z + 2 * i) * slot_stride];
+        }
+    }
+  }
+  s_sum[w][lane] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+  s_cnt[w][lane] = cnt;
+  __syncthreads();
+  // thread -> (person, score), scores fastest
+  if (threadIdx.x >= 32 * kSlotScores) return;
+  const uint32_t ks = threadIdx.x % kSlotScores, p = threadIdx.x / kSlotScores;
+  if (o0 + p >= P || k0 + ks >= K) return;
+  const uint64_t x = (o0 + p) * K + k0 + ks;
+  sums[x] = init[k0 + ks] + (s_sum[ks][p] + s_sum[ks + kSlotScores][p]);
+  counts[x] = s_cnt[ks][p] + s_cnt[ks + kSlotScores][p];
 }
 
 // ---- backward: dW[v,k] = sum_p d(p,v) dS[p,k], dC[v,k] = -sum_{p missing} dS[p,k]
@@ -2530,8 +2788,14 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device),
                "cudaDeviceGetAttribute");
     t->nsplits = narrow_splits(base, t->V_pad / kTcK, std::max(1, sms));
-    t->nslot = k16 * t->P_pad;
-    t->part_elems = std::max(t->part_elems, uint64_t(t->nsplits) * t->nslot);
+    t->P_nar = std::max<uint64_t>(1, (p->fam + 4 * kNrM - 1) / (4 * kNrM)) * (4 * kNrM);
+    t->nslot = k16 * t->P_nar;
+    // a tile of S stages meets at most S / quota + 2 CTAs' shares, and quota >=
+    // ptiles * S / ncta
+    t->ncta = std::max<uint32_t>(1, uint32_t(std::max(1, sms)) / uint32_t(k16 / kNrScores));
+    t->nalloc = std::max(t->nsplits, t->ncta / uint32_t(t->P_nar / (4 * kNrM)) + 2);
+    t->part_elems = std::max(t->part_elems, uint64_t(t->nalloc) * t->nslot);
+    t->d_state = p->d_err + 1;   // cleared with the error word by every reset
   }
   alloc(reinterpret_cast<void**>(&t->d_part_sum), t->part_elems * 8, "cudaMalloc(partials)");
   alloc(reinterpret_cast<void**>(&t->d_part_cnt), t->part_elems * 4, "cudaMalloc(partials)");
@@ -2643,11 +2907,52 @@ void tensor_set_narrow(gnm_plan* p, bool narrow) {
   p->tensor->narrow = narrow;
 }
 
+// The wide partials start from zero; the narrow engine's slots are written, not
+// added to, by the first call after the reset (slots_written).
+static void clear_wide(TensorPlan* t, cudaStream_t s) {
+  const uint64_t n = t->K_pad * t->P_pad;
+  check_cuda(cudaMemsetAsync(t->d_part_sum, 0, n * 8, s), "reset partials");
+  check_cuda(cudaMemsetAsync(t->d_part_cnt, 0, n * 4, s), "reset partials");
+  t->wide_clear = true;
+}
+
 void tensor_reset(gnm_plan* p, cudaStream_t s) {
   TensorPlan* t = p->tensor;
-  check_cuda(cudaMemsetAsync(t->d_part_sum, 0, t->part_elems * 8, s), "reset partials");
-  check_cuda(cudaMemsetAsync(t->d_part_cnt, 0, t->part_elems * 4, s), "reset partials");
+  t->wide_clear = false;
+  if (!t->narrow) clear_wide(t, s);
   t->pass_valid = false;   // the next SM-pair accumulate writes its pass arrays
+}
+
+template <int NMT>
+static void launch_t8_narrow(const TensorPlan* t, const uint8_t* d_rows, uint64_t pitch,
+                             uint64_t bpv, uint64_t nv, uint32_t stiles, T8NrArgs a,
+                             cudaStream_t s) {
+  using L = T8NrSmem<NMT>;
+  const CUtensorMap pmap =
+      make_row_map(d_rows, bpv, nv, pitch, L::kPkRow, kT8K,
+                   NMT == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
+  check_cuda(raise_smem_limit(reinterpret_cast<const void*>(gnm_t8_narrow<NMT>), int(L::kTotal)),
+             "narrow 8-bit shared memory");
+  a.ptiles = uint32_t(std::max<uint64_t>(1, (bpv + L::kPkRow - 1) / L::kPkRow));
+  const uint64_t units = uint64_t(a.ptiles) * a.stages;
+  a.quota = uint32_t((units + t->ncta - 1) / t->ncta);
+  a.slots = (a.stages + a.quota - 2) / a.quota + 1;
+  if (a.slots > t->nalloc) fail(GNM_ERR_COMPUTE, "narrow engine: more slots than allocated");
+  const dim3 grid(uint32_t((units + a.quota - 1) / a.quota), stiles);
+  gnm_t8_narrow<NMT><<<grid, kT8NrThreads, L::kTotal, s>>>(t->nmap8_dos, t->nmap8_mis, pmap, a);
+  check_cuda(cudaGetLastError(), "narrow 8-bit tensor launch");
+}
+
+// People tiles of 256 instead of 512 when the slowest CTA's share of 512-person
+// tiles holds over 1.25 times the work of its share of 256-person tiles (a last
+// tile that is mostly padding, a cohort of a few hundred people).  Otherwise
+// 512: half the limb traffic per person.  100,000 variants x 16 scores,
+// 20,000 people: 191 us on 512-person tiles, 266 us on 256-person ones; 10,000
+// variants: 44 and 50 us.
+static bool narrow_small_tiles(const TensorPlan* t, uint64_t people, uint64_t stages) {
+  const uint64_t u4 = (people + 511) / 512 * stages, u2 = (people + 255) / 256 * stages;
+  const uint64_t q4 = (u4 + t->ncta - 1) / t->ncta, q2 = (u2 + t->ncta - 1) / t->ncta;
+  return 8 * q4 > 5 * q2;
 }
 
 void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint64_t v0,
@@ -2656,25 +2961,23 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
   if (v0 % kTcK != 0)
     fail(GNM_ERR_INVALID, "tensor engine blocks must start at a multiple of 64 variants");
   if (t->narrow && t->i8 && v0 % kT8K == 0) {
-    const CUtensorMap pmap8 = make_row_map(d_rows, p->bpv, nv, pitch, kNrM / 4, kT8K);
-    check_cuda(raise_smem_limit(reinterpret_cast<const void*>(gnm_t8_narrow),
-                                int(T8NrSmem::kTotal)),
-               "narrow 8-bit shared memory");
-    NrArgs a;
+    T8NrArgs a{};
     a.num_rows = nv;
     a.a_x0 = int32_t(v0);
-    const uint32_t nall = uint32_t((nv + kT8K - 1) / kT8K);
-    a.stages_per_split = (nall + t->nsplits - 1) / t->nsplits;
     a.part_sum = t->d_part_sum;
     a.part_cnt = t->d_part_cnt;
-    a.P_pad = t->P_pad;
+    a.P_pad = t->P_nar;
     a.slot_stride = t->nslot;
     a.err = p->d_err;
-    const dim3 grid(uint32_t((p->fam + kNrM - 1) / kNrM),
-                    uint32_t((p->K + kNrScores - 1) / kNrScores), t->nsplits);
-    gnm_t8_narrow<<<grid, kNrThreads, T8NrSmem::kTotal, s>>>(t->nmap8_dos, t->nmap8_mis, pmap8,
-                                                             a, t->d_quanta8, t->K_pad);
-    check_cuda(cudaGetLastError(), "narrow 8-bit tensor launch");
+    a.stages = uint32_t((nv + kT8K - 1) / kT8K);
+    a.state = t->d_state;
+    a.quanta = t->d_quanta8;
+    a.K_pad = t->K_pad;
+    const uint32_t stiles = uint32_t((p->K + kNrScores - 1) / kNrScores);
+    if (narrow_small_tiles(t, p->fam, a.stages))
+      launch_t8_narrow<2>(t, d_rows, pitch, p->bpv, nv, stiles, a, s);
+    else
+      launch_t8_narrow<4>(t, d_rows, pitch, p->bpv, nv, stiles, a, s);
     p->launches += 1;
     return;
   }
@@ -2689,16 +2992,20 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
     a.stages_per_split = (nall + t->nsplits - 1) / t->nsplits;
     a.part_sum = t->d_part_sum;
     a.part_cnt = t->d_part_cnt;
-    a.P_pad = t->P_pad;
+    a.P_pad = t->P_nar;
     a.slot_stride = t->nslot;
     a.err = p->d_err;
+    gnm_tc_open_slots<<<296, 256, 0, s>>>(t->d_part_sum, t->d_part_cnt, t->nslot, t->nsplits,
+                                          t->d_state);
+    check_cuda(cudaGetLastError(), "narrow slots launch");
     const dim3 grid(uint32_t((p->fam + kNrM - 1) / kNrM),
                     uint32_t((p->K + kNrScores - 1) / kNrScores), t->nsplits);
     gnm_tc_narrow<<<grid, kNrThreads, NrSmem::kTotal, s>>>(t->nmap_dos, t->nmap_mis, pmap, a);
     check_cuda(cudaGetLastError(), "narrow tensor launch");
-    p->launches += 1;
+    p->launches += 2;
     return;
   }
+  if (!t->wide_clear) clear_wide(t, s);   // the reset met a narrow plan
   if (t->i8 && v0 % kT8K == 0) {
     // dosage limbs 0-1 and 2-3, correction limbs 0-1 and 2-3, then the counts
     const CUtensorMap pmap8 = make_row_map(d_rows, p->bpv, nv, pitch, kTcN / 4, kT8K);
@@ -2792,10 +3099,18 @@ void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_b
   TensorPlan* t = p->tensor;
   const uint64_t n = p->P * p->K;
   if (n == 0) return;
-  gnm_tc_finalize<<<uint32_t((n + 255) / 256), 256, 0, s>>>(
-      t->d_part_sum, t->d_part_cnt, t->P_pad, add_baseline ? p->d_baseline : p->d_zero_base,
-      p->d_out_to_fam, p->P, p->K, t->narrow ? t->nsplits : 0u, t->nslot,
-      t->pass_valid ? t->d_part_pass : nullptr, t->K_pad * t->P_pad, d_sums, d_counts);
+  const double* init = add_baseline ? p->d_baseline : p->d_zero_base;
+  const uint32_t gx = uint32_t((p->P + 31) / 32);
+  if (t->narrow)
+    gnm_tc_finalize_slots<<<dim3(gx, uint32_t((p->K + kSlotScores - 1) / kSlotScores)),
+                            32 * kSlotWarps, 0, s>>>(t->d_part_sum, t->d_part_cnt, t->P_nar, init,
+                                                     p->d_out_to_fam, p->P, p->K, t->d_state,
+                                                     t->nslot, d_sums, d_counts);
+  else
+    gnm_tc_finalize<<<dim3(gx, uint32_t((p->K + kFinTile - 1) / kFinTile)), 256, 0, s>>>(
+        t->d_part_sum, t->d_part_cnt, t->P_pad, init, p->d_out_to_fam, p->P, p->K,
+        t->pass_valid ? t->d_part_pass : nullptr, t->K_pad * t->P_pad, t->wide_clear ? 0u : 1u,
+        d_sums, d_counts);
   check_cuda(cudaGetLastError(), "tensor finalize launch");
   p->launches += 1;
 }
