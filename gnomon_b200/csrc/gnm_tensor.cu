@@ -1636,6 +1636,10 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
             hi[at + 5] = xc & ~sc & 0x40404040u;
           }
         }
+        // operands first, then the wait for their slot (the compiler would sink the
+        // arithmetic below it)
+#pragma unroll
+        for (uint32_t i = 0; i < 16; ++i) asm volatile("" : "+r"(lo[i]), "+r"(hi[i]));
         if (!mbar_wait_bounded(sfree(slot, pairm), sph ^ 1u)) {
           give_up(kErrMmaTimeout);
           ok = false;
@@ -2221,79 +2225,152 @@ __global__ void __launch_bounds__(kBwThreads, 1)
 }
 
 // ---- backward on 8-bit limbs -------------------------------------------------------
-// gnm_tc_backward with tcgen05.mma kind::i8: A = the allele-2 dosage of 128
-// variants (one byte per person, K-major rows expanded in place from the
-// packed rows), B = dS split into four signed 8-bit limbs per score (row
+// G = d^T dS and C = -m^T dS as one tcgen05.mma kind::i8 pass: A = the dosage and
+// the missing indicator of 128 variants (TMEM lanes), expanded straight into
+// TENSOR MEMORY, B = dS split into four signed 8-bit limbs per score (row
 // n = 16 * limb + score; q0 = max_p |dS[p,k]| / 127, q(j+1) = q(j) / 254, every
 // |limb| <= 127, residual below 2^-31.9 of the score's largest |dS|), S32
-// accumulators exact for up to 2^23 people, converted to FP64 with the
-// quanta once per call.  K = 128 people per stage (a 128-byte operand row),
-// so every operand byte is half the BF16 kernel's.  The sparse missing-call
-// term is the BF16 kernel's: the thread that expands a row adds the FP32 dS
-// row of each code-01 call, flushed to FP64 every 4096 people.
-constexpr uint32_t kBw8K = 128;                      // people per stage
-constexpr uint32_t kBw8Stages = 6;
-constexpr uint32_t kBw8Flush = (1u << 23) / kBw8K;   // stages per exact S32 block
-constexpr uint32_t kBw8MissFlush = 4096 / kBw8K;     // stages per FP32 missing-term sum
+// accumulators converted to FP64 with the quanta.
+//
+// What bounds it: the form this replaced stored the expanded dosage in shared
+// memory, where the MMA read it back, and added the FP32 dS row of every
+// missing call on CUDA cores, one dependent chain per row; tensor pipe 11 %
+// busy.  Here a thread owns one variant row (its TMEM lane):
+//
+//   * 16 packed bytes (64 people) per shared load, rows swizzled by the TMA so
+//     that eight lanes' loads fall in different banks;
+//   * a word's 16 dosages D = x - ((x | x >> 1) & 0x55555555) and missing bits
+//     M = x & ~(x >> 1) & 0x55555555 become four operand words each by a LEFT
+//     shift and a mask: people q, q + 4, q + 8, q + 12 in the top bits of the
+//     four bytes, 64 times their value (the quantum takes 2^-6).  Left shifts
+//     and the subtraction are multiply-adds by constants, so they run on the FMA
+//     pipe beside the masks on the integer pipe;
+//   * gnm_bw_build8 lays dS out in that order of people, so nothing is
+//     transposed; tcgen05.st.32x32b writes 64 people of both operands.
+//
+// Both operands meet the same limbs (two MMAs of N = 64 per 32 people: 37
+// clocks each, the tensor core's floor for M = 128 at these N); the dense
+// missing product costs less than the sparse FP32 sums did and is exact to the
+// limbs.  256 variants per CTA share each limb tile (2 x 128 accumulator
+// columns + 256 of operand ring).  CTAs take equal shares of (variant tile,
+// 512-person stage) units; a tile inside one share is written by its CTA, the
+// segments of a tile that spans shares go through FP64 slots that gnm_bw_join
+// adds in order.  S32 sums are exact for 2^17 people (127 x 2 x 64 each).
+constexpr uint32_t kBw8K = 512;                      // people per stage
+constexpr uint32_t kBw8Tile = 2 * kBwM;              // variants per CTA tile
+constexpr uint32_t kBw8Stages = 3;
+constexpr uint32_t kBw8Flush = (1u << 17) / kBw8K;   // stages per exact S32 block
+constexpr uint32_t kBw8Slots = 4;                    // operand slots per 128 variants, 64 people each
+constexpr uint32_t kBw8SlotCols = 32;                // 16 dosage + 16 missing columns
+constexpr uint32_t kBw8AccCols = 2 * kBwN;           // G and C columns per 128 variants
+constexpr uint32_t kBw8Threads = 128 + 512;          // TMA, two MMA warps, one idle; 16 expansion
 
 struct Bw8Smem {
-  static constexpr uint32_t kA = kBwM * kBw8K;               // 16 KB dosage operand
-  static constexpr uint32_t kB = kBwN * kBw8K;               // 8 KB dS limbs
-  static constexpr uint32_t kPkRow = kBw8K / 4;              // 32 packed bytes per variant
-  static constexpr uint32_t kPk = kBwM * kPkRow;             // 4 KB packed rows
-  static constexpr uint32_t kDs = kBw8K * kBwScores * 4;     // 8 KB FP32 dS
-  static constexpr uint32_t kAOff = 0;
-  static constexpr uint32_t kBOff = kAOff + kA;
-  static constexpr uint32_t kPkOff = kBOff + kB;
-  static constexpr uint32_t kDsOff = kPkOff + kPk;
-  static constexpr uint32_t kStage = kDsOff + kDs;            // 36 KB
+  static constexpr uint32_t kBox = kBwN * 128;               // 8 KB: limbs of 128 people
+  static constexpr uint32_t kB = kBw8K / 128 * kBox;         // 32 KB
+  static constexpr uint32_t kPkRow = kBw8K / 4;              // 128 packed bytes per variant
+  static constexpr uint32_t kPk = kBw8Tile * kPkRow;         // 32 KB packed rows
+  static constexpr uint32_t kPkOff = kB;
+  static constexpr uint32_t kStage = kB + kPk;
   static constexpr uint32_t kBarOff = kBw8Stages * kStage;
-  static constexpr uint32_t kHolder = kBarOff + 8 * (3 * kBw8Stages + 2);
+  static constexpr uint32_t kBars = 2 * kBw8Stages + 4 * kBw8Slots + 4;
+  static constexpr uint32_t kHolder = kBarOff + 8 * kBars;
   static constexpr uint32_t kTotal = kHolder + 16 + 1024;     // + alignment slack
-  static constexpr uint32_t kSwap = 2 * kBwM * kBwScores * 8;
   static_assert(kTotal <= 227 * 1024, "shared memory");
+  static_assert(kStage % 1024 == 0 && kPkOff % 1024 == 0, "operand alignment");
+  static constexpr uint32_t kRing0 = 2 * kBw8AccCols;
+  static_assert(kRing0 + 2 * kBw8Slots * kBw8SlotCols <= 512, "tensor memory columns");
+  static_assert(kBw8K / 64 == 2 * kBw8Slots, "a stage is two turns of the operand ring");
 };
-static_assert(Bw8Smem::kStage % 1024 == 0 && Bw8Smem::kBOff % 1024 == 0, "operand alignment");
-static_assert(Bw8Smem::kSwap <= Bw8Smem::kBarOff, "swap area");
 
-__global__ void __launch_bounds__(kBwThreads, 1)
+struct Bw8Args {
+  uint64_t V, K, K16;
+  uint32_t stages;         // 512-person stages
+  uint32_t vtiles;         // 256-variant tiles
+  uint32_t quota;          // (variant tile, stage) units per CTA
+  const double* quanta;    // [4][K16]
+  double* part;            // [score tiles][CTAs][2][G, C][256][16]: a CTA's first / last segment
+  float* gw;
+  float* gc;               // may be null (CORR false)
+  uint32_t* err;
+  const uint8_t* rows;     // packed rows and FP32 dS [people][K]: non-finite scores
+  uint64_t pitch;
+  const float* ds;
+  uint64_t people;
+};
+
+// The missing term of one variant over people [p0, p1) of a score whose largest
+// |dS| is an infinity or NaN, which limbs cannot hold: the sum of the dS values
+// themselves, so that only variants at which such a person is missing get one.
+__device__ __noinline__ double bw_missing_sum(const Bw8Args& a, uint64_t v, uint64_t k, uint64_t p0,
+                                              uint64_t p1) {
+  double s = 0.0;
+  for (uint64_t p = p0; p < p1 && p < a.people; ++p)
+    if (((a.rows[v * a.pitch + p / 4] >> (2 * (p % 4))) & 3u) == 1u) s += double(a.ds[p * a.K + k]);
+  return s;
+}
+
+// Elements of one segment slot of Bw8Args::part.
+constexpr uint64_t kBw8SlotElems = 2 * uint64_t(kBw8Tile) * kBwScores;
+
+// {-1, 4, 16, 64}: the subtraction and the left shifts of the expansion as integer
+// multiply-adds; in constant memory, unknown at compile time, so that the
+// compiler issues IMAD on the FMA pipe (see gnm_plain.cu).
+__constant__ uint32_t c_bw[4] = {0xFFFFFFFFu, 4u, 16u, 64u};
+
+template <bool CORR>
+__global__ void __launch_bounds__(kBw8Threads, 1)
     gnm_t8_backward(const __grid_constant__ CUtensorMap rmap,
-                    const __grid_constant__ CUtensorMap bmap,
-                    const __grid_constant__ CUtensorMap dmap, BwArgs a, const double* quanta,
-                    uint64_t K16) {
+                    const __grid_constant__ CUtensorMap bmap, Bw8Args a) {
   using L = Bw8Smem;
+  constexpr uint32_t ST = kBw8Stages, R = kBw8Slots;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sb = smem_u32(smem);
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t vtile = blockIdx.x, stile = blockIdx.y;
-  const uint32_t nit = a.nstages;
-  constexpr uint32_t ST = kBw8Stages;
+  const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t stile = blockIdx.y;
+  const uint64_t units = uint64_t(a.vtiles) * a.stages;
+  const uint64_t u0 = uint64_t(blockIdx.x) * a.quota;
+  const uint64_t u1 = u0 + a.quota < units ? u0 + a.quota : units;
+  if (u0 >= u1) return;   // uniform per CTA (the host launches none such)
   auto full = [&](uint32_t s) { return sb + L::kBarOff + 8 * s; };
-  auto aready = [&](uint32_t s) { return sb + L::kBarOff + 8 * (ST + s); };
-  auto empty = [&](uint32_t s) { return sb + L::kBarOff + 8 * (2 * ST + s); };
-  const uint32_t accfull = sb + L::kBarOff + 8 * (3 * ST);
-  const uint32_t accempty = sb + L::kBarOff + 8 * (3 * ST + 1);
+  auto tempty = [&](uint32_t s) { return sb + L::kBarOff + 8 * (ST + s); };
+  // operand slot b of 128-variant block t: filled by its four warps / read by its MMAs
+  auto ready = [&](uint32_t t, uint32_t b) { return sb + L::kBarOff + 8 * (2 * ST + t * R + b); };
+  auto sfree = [&](uint32_t t, uint32_t b) {
+    return sb + L::kBarOff + 8 * (2 * ST + (2 + t) * R + b);
+  };
+  const uint32_t accfull = sb + L::kBarOff + 8 * (2 * ST + 4 * R);
+  const uint32_t accempty = accfull + 8, drain0 = accfull + 16;   // one drain per MMA warp
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kHolder + 8);
   const uint32_t abort_addr = sb + L::kHolder + 8;
+  auto give_up = [&](uint32_t code) {
+    *abort_flag = 1u;
+    atomicOr(a.err, code);
+  };
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < ST; ++s) {
       mbar_init(full(s), 1);
-      mbar_init(aready(s), kBwExpand);
-      mbar_init(empty(s), 1);
+      mbar_init(tempty(s), 2);   // both MMA warps
     }
-    mbar_init(accfull, 1);
-    mbar_init(accempty, kBwExpand);
+    for (uint32_t t = 0; t < 2; ++t)
+      for (uint32_t b = 0; b < R; ++b) {
+        mbar_init(ready(t, b), 4);
+        mbar_init(sfree(t, b), 1);
+      }
+    mbar_init(accfull, 2);
+    mbar_init(accempty, 16);
+    mbar_init(drain0, 1);
+    mbar_init(drain0 + 8, 1);
     *abort_flag = 0u;
     fence_mbar_init();
     prefetch_tmap(&rmap);
     prefetch_tmap(&bmap);
-    prefetch_tmap(&dmap);
   }
   if (warp == 1) {
-    tmem_alloc(sb + L::kHolder, kBwN);
+    tmem_alloc(sb + L::kHolder, 512);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -2304,181 +2381,225 @@ __global__ void __launch_bounds__(kBwThreads, 1)
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      for (uint32_t it = 0; it < nit; ++it) {
-        const uint32_t s = it % ST, ph = (it / ST) & 1u;
-        if (!mbar_wait_bounded(empty(s), ph ^ 1u)) {
-          *abort_flag = 1u;
-          atomicOr(a.err, kErrMmaTimeout);
+      uint32_t n = 0;
+      uint32_t tile = uint32_t(u0 / a.stages), st = uint32_t(u0 % a.stages);
+      bool ok = true;
+      for (uint64_t u = u0; u < u1; ++u, ++n) {
+        const uint32_t s = n % ST, ph = (n / ST) & 1u;
+        if (!mbar_wait_bounded(tempty(s), ph ^ 1u)) {
+          give_up(kErrMmaTimeout);
+          ok = false;
           break;
         }
-        if (lds_volatile_u32(abort_addr)) break;
-        const uint32_t st = sb + s * L::kStage;
-        mbar_arrive_expect_tx(full(s), L::kB + L::kPk + L::kDs);
-        tma_load_2d(st + L::kPkOff, &rmap, int32_t(it * L::kPkRow), int32_t(vtile * kBwM),
-                    full(s));
-        tma_load_2d(st + L::kBOff, &bmap, int32_t(it * kBw8K), int32_t(stile * kBwN), full(s));
-        tma_load_2d(st + L::kDsOff, &dmap, int32_t(stile * kBwScores), int32_t(it * kBw8K),
-                    full(s));
-      }
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_s8s8_s32(kBwM, kBwN);
-      uint32_t blk = 0;
-      for (uint32_t it = 0; it < nit; ++it) {
-        const uint32_t s = it % ST, ph = (it / ST) & 1u;
-        const bool first = (it % kBw8Flush) == 0;
-        if (first && it > 0) {
-          if (!mbar_wait_bounded(accempty, (blk - 1) & 1u)) {
-            *abort_flag = 1u;
-            atomicOr(a.err, kErrMmaTimeout);
-            break;
-          }
-        }
-        if (!mbar_wait_bounded(aready(s), ph)) {
-          *abort_flag = 1u;
-          atomicOr(a.err, kErrMmaTimeout);
+        if (lds_volatile_u32(abort_addr)) {
+          ok = false;
           break;
         }
-        if (lds_volatile_u32(abort_addr)) break;
-        tc_fence_after();
-        const uint32_t a0 = sb + s * L::kStage + L::kAOff;
-        const uint32_t b0 = sb + s * L::kStage + L::kBOff;
+        const uint32_t at = sb + s * L::kStage;
+        mbar_arrive_expect_tx(full(s), L::kStage);
+        tma_load_2d(at + L::kPkOff, &rmap, int32_t(st * L::kPkRow), int32_t(tile * kBw8Tile),
+                    full(s));
 #pragma unroll
-        for (uint32_t kk = 0; kk < kBw8K / 32; ++kk)
-          tc_mma_i8(tmem, desc_kmajor_sw128(a0 + kk * 32), desc_kmajor_sw128(b0 + kk * 32), idesc,
-                    (first && kk == 0) ? 0u : 1u);
-        tc_commit(empty(s));
-        if ((it % kBw8Flush) == kBw8Flush - 1 || it == nit - 1) {
-          tc_commit(accfull);
-          ++blk;
+        for (uint32_t j = 0; j < kBw8K / 128; ++j)
+          tma_load_2d(at + j * L::kBox, &bmap, int32_t(st * kBw8K + 128 * j),
+                      int32_t(stile * kBwN), full(s));
+        if (++st == a.stages) {
+          st = 0;
+          ++tile;
         }
       }
+      if (!ok)   // nothing may still be in flight when the CTA exits (bounded)
+        for (uint32_t i = n > ST ? n - ST : 0; i < n; ++i)
+          mbar_wait_bounded(full(i % ST), (i / ST) & 1u);
     }
-  } else {
-    // ---------------- genotype expansion + epilogue (warps 2-9) ----------------
-    const uint32_t quad = warp & 3;
-    const uint32_t half = (warp - 2) >> 2;  // people 64 half .. of each stage; scores 8 half ..
-    const uint32_t r = 32 * quad + lane;    // variant row of this thread and its TMEM lane
-    double gwd[8], gcd[kBwScores];
-    float gcf[kBwScores];   // missing term of the last <= kBw8MissFlush stages
-#pragma unroll
-    for (uint32_t k = 0; k < kBwScores; ++k) {
-      gcd[k] = 0.0;
-      gcf[k] = 0.0f;
-    }
-#pragma unroll
-    for (uint32_t k = 0; k < 8; ++k) gwd[k] = 0.0;
+  } else if (warp == 1 || warp == 2) {
+    // ---------------- MMA issuers (see gnm_t8_narrow): warp 1 + t, block t ----------------
+    constexpr uint32_t idesc = idesc_u8s8_s32(kBwM, kBwN);
+    const uint32_t t = warp - 1;
+    uint32_t st = uint32_t(u0 % a.stages), blk = 0, inblk = 0, n = 0;
+    const uint32_t left = uint32_t(u1 - u0);
+    const uint32_t utmem = __shfl_sync(0xFFFFFFFFu, tmem, 0);
+    const uint32_t d = utmem + kBw8AccCols * t;
     bool ok = true;
-    uint32_t blk = 0;
-    for (uint32_t it = 0; it < nit; ++it) {
-      const uint32_t s = it % ST, ph = (it / ST) & 1u;
-      if (!mbar_wait_bounded(full(s), ph)) {
-        *abort_flag = 1u;
-        atomicOr(a.err, kErrTmaTimeout);
+    for (; n < left && ok; ++n) {
+      const uint32_t s = n % ST;
+      if (inblk == 0 && blk > 0 && !mbar_wait_warp(accempty, (blk - 1) & 1u)) {
+        give_up(kErrMmaTimeout);
         ok = false;
         break;
       }
-      if (lds_volatile_u32(abort_addr)) {
-        ok = false;
-        break;
-      }
-      const uint32_t st = sb + s * L::kStage;
-      // words 4 half .. 4 half + 3 of the row: people 64 half + 16 w ..
-      const uint4 x4 = lds_u128(st + L::kPkOff + r * L::kPkRow + 16 * half);
-      const uint32_t xw[4] = {x4.x, x4.y, x4.z, x4.w};
-      const uint32_t arow = st + L::kAOff + (r >> 3) * 1024 + (r & 7) * 128;
+      const bool last = st + 1 == a.stages || inblk + 1 == kBw8Flush || n + 1 == left;
 #pragma unroll
-      for (uint32_t w = 0; w < 4; ++w) {
-        // byte t of s_q = dosage of person 4t + q of the word; a 4 x 4 byte
-        // transpose puts person 4t + i at byte i of word t
-        const uint32_t d = code_fields<false>(xw[w]);
-        const uint32_t s0 = d & 0x03030303u, s1 = (d >> 2) & 0x03030303u;
-        const uint32_t s2 = (d >> 4) & 0x03030303u, s3 = (d >> 6) & 0x03030303u;
-        const uint32_t lo01 = __byte_perm(s0, s1, 0x5140u), hi01 = __byte_perm(s0, s1, 0x7362u);
-        const uint32_t lo23 = __byte_perm(s2, s3, 0x5140u), hi23 = __byte_perm(s2, s3, 0x7362u);
-        uint4 v;
-        v.x = __byte_perm(lo01, lo23, 0x5410u);
-        v.y = __byte_perm(lo01, lo23, 0x7632u);
-        v.z = __byte_perm(hi01, hi23, 0x5410u);
-        v.w = __byte_perm(hi01, hi23, 0x7632u);
-        const uint32_t c = 4 * half + w;   // 16-byte chunk: people 16c .. 16c + 15
-        sts_u128(arow + ((c ^ (r & 7)) << 4), v);
-      }
-      // missing calls (code 01): add the person's FP32 dS row; bit 2i of m is
-      // person i of the word
-#pragma unroll
-      for (uint32_t w = 0; w < 4; ++w) {
-        uint32_t m = xw[w] & ~(xw[w] >> 1) & 0x55555555u;
-        while (m) {
-          const uint32_t b = 31u - __clz(m);
-          m ^= 1u << b;
-          const uint32_t drow = st + L::kDsOff + (64 * half + 16 * w + b / 2) * (kBwScores * 4);
-#pragma unroll
-          for (uint32_t q = 0; q < kBwScores / 4; ++q) {
-            const uint4 f = lds_u128(drow + 16 * q);
-            gcf[4 * q + 0] += __uint_as_float(f.x);
-            gcf[4 * q + 1] += __uint_as_float(f.y);
-            gcf[4 * q + 2] += __uint_as_float(f.z);
-            gcf[4 * q + 3] += __uint_as_float(f.w);
-          }
-        }
-      }
-      if ((it % kBw8MissFlush) == kBw8MissFlush - 1 || it == nit - 1) {
-#pragma unroll
-        for (uint32_t k = 0; k < kBwScores; ++k) {
-          gcd[k] += double(gcf[k]);
-          gcf[k] = 0.0f;
-        }
-      }
-      fence_proxy_async_smem();
-      mbar_arrive(aready(s));
-
-      if ((it % kBw8Flush) == kBw8Flush - 1 || it == nit - 1) {
-        if (!mbar_wait_bounded(accfull, blk & 1u)) {
-          *abort_flag = 1u;
-          atomicOr(a.err, kErrMmaTimeout);
+      for (uint32_t i = 0; i < kBw8K / 64; ++i) {   // 64 people per slot
+        if (!mbar_wait_warp(ready(t, i % R), (i / R) & 1u)) {
+          give_up(kErrMmaTimeout);
           ok = false;
           break;
         }
         tc_fence_after();
-        // columns 16 j + 8 half + k: limb j of score 8 half + k
-        const uint32_t lane_base = tmem + ((32 * quad) << 16) + 8 * half;
-        const uint64_t k0 = uint64_t(stile) * kBwScores + 8 * half;
+        if (elect_one()) {
+          const uint64_t b0 = desc_kmajor_sw128(sb + s * L::kStage + (i / 2) * L::kBox) + 4 * (i % 2);
+          const uint32_t op = utmem + L::kRing0 + (t * R + i % R) * kBw8SlotCols;
+          const uint32_t acc = (inblk == 0 && i == 0) ? 0u : 1u;
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-          uint32_t d[8];
-          tmem_ld8(lane_base + 16 * j, d);
-          tmem_ld_wait();
-#pragma unroll
-          for (uint32_t k = 0; k < 8; ++k)
-            gwd[k] = fma(double(int32_t(d[k])), quanta[j * K16 + k0 + k], gwd[k]);
+          for (uint32_t kk = 0; kk < 2; ++kk) {
+            tc_mma_i8_ta(d, op + 8 * kk, b0 + 2 * kk, idesc, kk ? 1u : acc);
+            if (CORR) tc_mma_i8_ta(d + kBwN, op + 16 + 8 * kk, b0 + 2 * kk, idesc, kk ? 1u : acc);
+          }
+          tc_commit(sfree(t, i % R));
+          if (i == kBw8K / 64 - 1) {
+            tc_commit(tempty(s));
+            if (last) tc_commit(accfull);
+          }
         }
-        tc_fence_before();
-        mbar_arrive(accempty);
+        __syncwarp();
+      }
+      ++inblk;
+      if (++st == a.stages) st = 0;
+      if (last) {
         ++blk;
+        inblk = 0;
       }
     }
-    // The two halves of a row hold the missing term of different people: add
-    // them in a fixed order through shared memory (stage buffers are idle: the
-    // last accumulator commit followed every MMA, and every TMA was consumed).
-    named_barrier(1, kBwExpand);
-    double* swap = reinterpret_cast<double*>(smem);
+    if (!ok) {   // issued MMAs finish before the CTA's memory goes (bounded)
+      const uint32_t drain = drain0 + 8 * t;
+      if (elect_one()) tc_commit(drain);
+      __syncwarp();
+      mbar_wait_bounded(drain, 0);
+    }
+  } else if (warp >= 4) {
+    // ---------------- genotype expansion + epilogue (warps 4-19) ----------------
+    const uint32_t quad = warp & 3;
+    const uint32_t grp = (warp - 4) >> 2;
+    const uint32_t t = grp & 1u, mine = grp >> 1;   // block; this warp takes every second slot
+    const uint32_t r = kBwM * t + 32 * quad + lane;  // variant row of the tile
+    const uint32_t pk0 = sb + L::kPkOff + r * L::kPkRow;
+    const uint32_t op0 =
+        tmem + ((32 * quad) << 16) + L::kRing0 + (t * R + mine) * kBw8SlotCols;
+    const uint32_t ready0 = ready(t, mine), sfree0 = sfree(t, mine);
+    uint32_t tile = uint32_t(u0 / a.stages), st = uint32_t(u0 % a.stages);
+    uint32_t blk = 0, inblk = 0, n = 0;
+    double acc[kBwScores];   // epilogue: G (mine 0) or C (mine 1) of this row
 #pragma unroll
-    for (uint32_t k = 0; k < kBwScores; ++k) swap[(half * kBwM + r) * kBwScores + k] = gcd[k];
-    named_barrier(1, kBwExpand);
-    const uint64_t v = uint64_t(vtile) * kBwM + r;
-    if (ok && !lds_volatile_u32(abort_addr) && v < a.V) {
+    for (uint32_t k = 0; k < kBwScores; ++k) acc[k] = 0.0;
+    for (uint64_t u = u0; u < u1; ++u, ++n) {
+      const uint32_t s = n % ST, ph = (n / ST) & 1u;
+      if (!mbar_wait_bounded(full(s), ph)) {
+        give_up(kErrTmaTimeout);
+        break;
+      }
+      const uint32_t aborted = lds_volatile_u32(abort_addr);
+      bool ok = true;
+      uint4 x4 = lds_u128(pk0 + s * L::kStage + ((mine ^ (r & 7u)) << 4));
 #pragma unroll
-      for (uint32_t k = 0; k < 8; ++k) {
-        const uint32_t kl = 8 * half + k;
-        const uint64_t kk = uint64_t(stile) * kBwScores + kl;
-        if (kk < a.K) {
-          a.gw[v * a.K + kk] = float(gwd[k]);
-          if (a.gc)
-            a.gc[v * a.K + kk] =
-                float(-(swap[r * kBwScores + kl] + swap[(kBwM + r) * kBwScores + kl]));
+      for (uint32_t j = 0; j < kBw8K / 128; ++j) {
+        const uint32_t xw[4] = {x4.x, x4.y, x4.z, x4.w};
+        if (j + 1 < kBw8K / 128)   // the next slot's 64 people
+          x4 = lds_u128(pk0 + s * L::kStage + (((2 * (j + 1) + mine) ^ (r & 7u)) << 4));
+        uint32_t v[32];
+#pragma unroll
+        for (uint32_t w = 0; w < 4; ++w) {
+          const uint32_t x = xw[w], sh = x >> 1;
+          const uint32_t d = ((x | sh) & 0x55555555u) * c_bw[0] + x;   // x - (...)
+          v[4 * w + 0] = (d * c_bw[3]) & 0xC0C0C0C0u;
+          v[4 * w + 1] = (d * c_bw[2]) & 0xC0C0C0C0u;
+          v[4 * w + 2] = (d * c_bw[1]) & 0xC0C0C0C0u;
+          v[4 * w + 3] = d & 0xC0C0C0C0u;
+          if (CORR) {
+            const uint32_t m = x & ~sh & 0x55555555u;
+            v[16 + 4 * w + 0] = (m * c_bw[3]) & 0x40404040u;
+            v[16 + 4 * w + 1] = (m * c_bw[2]) & 0x40404040u;
+            v[16 + 4 * w + 2] = (m * c_bw[1]) & 0x40404040u;
+            v[16 + 4 * w + 3] = m & 0x40404040u;
+          }
+        }
+        // operands first, then the wait for their slot: the wait covers the MMAs of
+        // two slots before, and the compiler would sink the arithmetic below it
+#pragma unroll
+        for (uint32_t i = 0; i < (CORR ? 32u : 16u); ++i) asm volatile("" : "+r"(v[i]));
+        // a stage is two turns of the ring, so slots and phases are constants
+        const uint32_t op = op0 + (2 * (j % 2)) * kBw8SlotCols;
+        if (!mbar_wait_bounded(sfree0 + 16 * (j % 2), (j / 2) ^ 1u)) {
+          give_up(kErrMmaTimeout);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        if (CORR)
+          tmem_st_32x32b_x32(op, v);
+        else
+          tmem_st_32x32b_x16(op, v);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ready0 + 16 * (j % 2));
+      }
+      if (!ok || aborted) break;
+      ++inblk;
+      const uint32_t tile_now = tile;
+      const bool tile_end = ++st == a.stages;
+      if (tile_end) {
+        st = 0;
+        ++tile;
+      }
+      if (tile_end || inblk == kBw8Flush || u + 1 == u1) {
+        inblk = 0;
+        if (!mbar_wait_bounded(accfull, blk & 1u)) {
+          give_up(kErrMmaTimeout);
+          break;
+        }
+        ++blk;
+        tc_fence_after();
+        if (CORR || mine == 0) {
+          const uint32_t base = tmem + ((32 * quad) << 16) + t * kBw8AccCols + mine * kBwN;
+          // -64 for C: the product is of the missing indicator, C its negative
+          const double scale = mine ? -1.0 / 64.0 : 1.0 / 64.0;
+#pragma unroll
+          for (uint32_t j = 0; j < 4; ++j)
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+              uint32_t d[8];
+              tmem_ld8(base + 16 * j + 8 * h, d);
+              tmem_ld_wait();
+#pragma unroll
+              for (uint32_t k = 0; k < 8; ++k)
+                acc[8 * h + k] =
+                    fma(double(int32_t(d[k])),
+                        a.quanta[j * a.K16 + uint64_t(stile) * kBwScores + 8 * h + k] * scale,
+                        acc[8 * h + k]);
+            }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(accempty);
+        if (tile_end || u + 1 == u1) {   // the segment is complete
+          const uint64_t t0 = uint64_t(tile_now) * a.stages;
+          const uint64_t v = uint64_t(tile_now) * kBw8Tile + r;
+          const uint64_t k0 = uint64_t(stile) * kBwScores;
+          if (CORR && mine == 1 && v < a.V) {
+            const uint64_t s0 = (t0 >= u0 ? t0 : u0) - t0;   // the segment's stages
+#pragma unroll
+            for (uint32_t k = 0; k < kBwScores; ++k)
+              if (k0 + k < a.K && !isfinite(a.quanta[k0 + k]))
+                acc[k] = -bw_missing_sum(a, v, k0 + k, s0 * kBw8K, (u + 1 - t0) * kBw8K);
+          }
+          if (CORR || mine == 0) {
+            if (t0 >= u0 && tile_end) {   // the whole tile is this CTA's
+              float* out = mine ? a.gc : a.gw;
+              if (v < a.V)
+#pragma unroll
+                for (uint32_t k = 0; k < kBwScores; ++k)
+                  if (k0 + k < a.K) out[v * a.K + k0 + k] = float(acc[k]);
+            } else {   // slot 0: the tile began in an earlier share, 1: it goes on in the next
+              const uint64_t cta = uint64_t(stile) * gridDim.x + blockIdx.x;
+              double* ps = a.part + (2 * cta + (t0 >= u0 ? 1 : 0)) * kBw8SlotElems +
+                           (uint64_t(mine) * kBw8Tile + r) * kBwScores;
+#pragma unroll
+              for (uint32_t k = 0; k < kBwScores; ++k) ps[k] = acc[k];
+            }
+          }
+#pragma unroll
+          for (uint32_t k = 0; k < kBwScores; ++k) acc[k] = 0.0;
         }
       }
     }
@@ -2487,32 +2608,64 @@ __global__ void __launch_bounds__(kBwThreads, 1)
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, kBwN);
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// Adds the segments of every variant tile that spans CTA shares, in share order.
+// blockIdx.x = boundary between shares b and b + 1: the tile cut by it is joined
+// by the first boundary that cuts it.
+__global__ void __launch_bounds__(256) gnm_bw_join(Bw8Args a, uint32_t ctas) {
+  const uint64_t cut = uint64_t(blockIdx.x + 1) * a.quota;   // first unit of share b + 1
+  const uint64_t tile = cut / a.stages, t0 = tile * a.stages, t1 = t0 + a.stages;
+  if (cut == t0 || cut - t0 > a.quota) return;   // no tile is cut / an earlier boundary cut it
+  const uint64_t first = blockIdx.x, last = (t1 - 1) / a.quota;
+  const uint32_t stile = blockIdx.y;
+  const uint32_t ops = a.gc ? 2 : 1;
+  for (uint32_t x = blockIdx.z * blockDim.x + threadIdx.x; x < ops * kBw8Tile * kBwScores;
+       x += gridDim.z * blockDim.x) {
+    const uint32_t op = x / (kBw8Tile * kBwScores), e = x % (kBw8Tile * kBwScores);
+    const uint64_t v = tile * kBw8Tile + e / kBwScores;
+    const uint64_t k = uint64_t(stile) * kBwScores + e % kBwScores;
+    if (v >= a.V || k >= a.K) continue;
+    double s = 0.0;
+    for (uint64_t c = first; c <= last; ++c) {
+      // the first share holds the tile as its last segment, the others as their first
+      const uint64_t slot = 2 * (uint64_t(stile) * ctas + c) + (c == first ? 1 : 0);
+      s += a.part[slot * kBw8SlotElems + uint64_t(op) * kBw8Tile * kBwScores + e];
+    }
+    (op ? a.gc : a.gw)[v * a.K + k] = float(s);
   }
 }
 
 // dS [rows][K] -> 8-bit limb rows (tile t = k / 16: rows 64t + 16j + k % 16,
-// limb j) of P_pad people each, their quanta [4][K16], and the FP32 copy
-// [P_pad][K16] for the missing term; zeros past the last person and score.
-__global__ void gnm_bw_build8(const float* g, uint64_t rows, uint64_t K, uint64_t K16,
-                              uint64_t P_pad, const uint32_t* amax_bits, int8_t* planes,
-                              double* quanta, float* ds) {
-  const uint64_t x = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (x >= K16 * P_pad) return;
-  const uint64_t p = x % P_pad, k = x / P_pad;
-  const bool in = p < rows && k < K;
-  const float val = in ? g[p * K + k] : 0.0f;
-  ds[p * K16 + k] = val;
+// limb j) of P_pad people each, and their quanta [4][K16]; zeros past the last
+// person and score.  Person p of each 16 is stored at 4 (p % 4) + p / 4 % 4, the
+// order in which gnm_t8_backward expands a packed word.  A CTA takes 32 people x
+// 16 scores: it reads whole dS rows and writes 32 consecutive bytes of a limb row.
+__global__ void __launch_bounds__(512)
+    gnm_bw_build8(const float* g, uint64_t rows, uint64_t K, uint64_t K16, uint64_t P_pad,
+                  const uint32_t* amax_bits, int8_t* planes, double* quanta) {
+  __shared__ float s_val[32][kBwScores + 1];
+  const uint64_t p0 = uint64_t(blockIdx.x) * 32, k0 = uint64_t(blockIdx.y) * kBwScores;
+  {
+    const uint32_t p = threadIdx.x / kBwScores, k = threadIdx.x % kBwScores;
+    s_val[p][k] = (p0 + p < rows && k0 + k < K) ? g[(p0 + p) * K + k0 + k] : 0.0f;
+  }
+  __syncthreads();
+  const uint32_t at = threadIdx.x % 32, ks = threadIdx.x / 32;   // stored position, score
+  const uint32_t p = (at & 16u) + 4 * (at % 4) + at / 4 % 4;     // its person (an involution)
+  const uint64_t k = k0 + ks;
   const float am = k < K ? __uint_as_float(amax_bits[k]) : 0.0f;
-  double q = am > 0.0f ? double(am) / 127.0 : 1.0;
-  const uint64_t row0 = (k / kBwScores) * kBwN + (k % kBwScores);
-  double rem = double(val);
+  double q = am == 0.0f ? 1.0 : double(am) / 127.0;   // a NaN stays one
+  const uint64_t row0 = uint64_t(blockIdx.y) * kBwN + ks;
+  double rem = double(s_val[p][ks]);
 #pragma unroll
   for (uint32_t j = 0; j < 4; ++j, q /= 254.0) {
     const double li = fmin(fmax(rint(rem / q), -127.0), 127.0);
     rem -= li * q;
-    planes[(row0 + kBwScores * j) * P_pad + p] = int8_t(li);
-    if (p == 0) quanta[j * K16 + k] = q;
+    planes[(row0 + kBwScores * j) * P_pad + p0 + at] = int8_t(li);
+    if (blockIdx.x == 0 && at == 0) quanta[j * K16 + k] = q;
   }
 }
 
@@ -2526,16 +2679,34 @@ __global__ void gnm_scatter_grad(const float* gs, const uint32_t* out_to_fam, ui
 }
 
 // Per-score max |dS| as float bit patterns (non-negative floats order like
-// their bits); thread = (64-person chunk, score), consecutive threads read
-// consecutive scores of a row.
-__global__ void gnm_bw_amax(const float* g, uint64_t rows, uint64_t K, uint32_t* amax_bits) {
-  const uint64_t x = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const uint64_t k = x % K, p0 = (x / K) * 64;
-  if (p0 >= rows) return;
-  const uint64_t p1 = p0 + 64 < rows ? p0 + 64 : rows;
-  uint32_t m = 0;
-  for (uint64_t p = p0; p < p1; ++p) m = max(m, __float_as_uint(fabsf(g[p * K + k])));
-  atomicMax(amax_bits + k, m);
+// their bits): a thread reads every 256 K-th element, so its score is fixed and
+// a warp's loads are consecutive; scores meet in shared memory when they fit.
+constexpr uint32_t kAmaxPer = 8;   // elements per thread
+__global__ void __launch_bounds__(256)
+    gnm_bw_amax(const float* g, uint64_t rows, uint64_t K, uint32_t* amax_bits) {
+  extern __shared__ uint32_t s_max[];
+  const bool shared = K <= kAmaxSharedScores;
+  if (shared) {
+    for (uint64_t k = threadIdx.x; k < K; k += 256) s_max[k] = 0u;
+    __syncthreads();
+  }
+  const uint64_t n = rows * K, x0 = uint64_t(blockIdx.x) * (256 * kAmaxPer) + threadIdx.x;
+  uint32_t v[kAmaxPer];
+#pragma unroll
+  for (uint32_t i = 0; i < kAmaxPer; ++i) {
+    const uint64_t x = x0 + 256 * i;
+    v[i] = x < n ? __float_as_uint(fabsf(g[x])) : 0u;
+  }
+#pragma unroll
+  for (uint32_t i = 0; i < kAmaxPer; ++i) {
+    const uint64_t x = x0 + 256 * i;
+    if (x < n && v[i]) atomicMax((shared ? s_max : amax_bits) + x % K, v[i]);
+  }
+  if (shared) {
+    __syncthreads();
+    for (uint64_t k = threadIdx.x; k < K; k += 256)
+      if (s_max[k]) atomicMax(amax_bits + k, s_max[k]);
+  }
 }
 
 // dS [rows][K] -> limb rows (tile t = k / 16: rows 64t + 16j + k % 16, limb j)
@@ -3115,18 +3286,45 @@ void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_b
   p->launches += 1;
 }
 
-// dS limbs in 8 bits (gnm_t8_backward): buffers [limb rows][P_pad] int8,
-// [P_pad][K16] FP32 dS, [4][K16] FP64 quanta, [K16] maxima, re-derived on
-// every call.
+static void launch_bw_amax(const gnm_plan* p, const float* gsf, uint32_t* amax, cudaStream_t s) {
+  const uint64_t n = p->fam * p->K;
+  if (!n) return;
+  const uint32_t smem = p->K <= kAmaxSharedScores ? uint32_t(p->K * 4) : 0u;
+  const uint64_t blocks = (n + 256 * kAmaxPer - 1) / (256 * kAmaxPer);
+  gnm_bw_amax<<<uint32_t(blocks), 256, smem, s>>>(gsf, p->fam, p->K, amax);
+  check_cuda(cudaGetLastError(), "gradient maximum launch");
+}
+
+// dS limbs in 8 bits (gnm_t8_backward): buffers [limb rows][P_pad] int8, [4][K16]
+// FP64 quanta, [K16] maxima, segment slots, re-derived on every call.
 static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, const float* gsf,
                          float* d_grad_w, float* d_grad_corr, cudaStream_t s) {
   const uint64_t K16 = (p->K + kBwScores - 1) / kBwScores * kBwScores;
   const uint64_t P_pad = std::max<uint64_t>(kBw8K, (p->fam + kBw8K - 1) / kBw8K * kBw8K);
   const uint64_t limb_rows = K16 / kBwScores * kBwN;
+  int sms = 0;
+  check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device),
+             "cudaDeviceGetAttribute");
+  Bw8Args a;
+  a.V = p->V;
+  a.K = p->K;
+  a.K16 = K16;
+  a.stages = uint32_t(P_pad / kBw8K);
+  a.vtiles = uint32_t((p->V + kBw8Tile - 1) / kBw8Tile);
+  const uint64_t units = uint64_t(a.vtiles) * a.stages, stiles = K16 / kBwScores;
+  const uint64_t share = std::max<uint64_t>(1, uint64_t(std::max(1, sms)) / stiles);
+  a.quota = uint32_t((units + share - 1) / share);
+  // whole tiles per share when that lengthens the longest share by no more than
+  // the join costs (about 5 us, four stages of 1.2 us)
+  const uint32_t whole = (a.quota + a.stages - 1) / a.stages * a.stages;
+  if (whole - a.quota <= 4) a.quota = whole;
+  const uint32_t ctas = uint32_t((units + a.quota - 1) / a.quota);
+
   const uint64_t planes_bytes = (limb_rows * P_pad + 255) / 256 * 256;
-  const uint64_t ds_bytes = (P_pad * K16 * 4 + 255) / 256 * 256;
   const uint64_t q_bytes = 4 * K16 * 8;
-  const uint64_t need = planes_bytes + ds_bytes + q_bytes + K16 * 4;
+  const uint64_t amax_bytes = (K16 * 4 + 255) / 256 * 256;
+  const uint64_t part_bytes = 2 * ctas * stiles * kBw8SlotElems * 8;
+  const uint64_t need = planes_bytes + q_bytes + amax_bytes + part_bytes;
   if (p->bw_bytes < need) {
     check_cuda(cudaStreamSynchronize(s), "backward buffer resize");
     pool_free(p->d_bw);
@@ -3138,41 +3336,45 @@ static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, con
     p->device_bytes += need;
   }
   auto* planes = reinterpret_cast<int8_t*>(p->d_bw);
-  auto* ds = reinterpret_cast<float*>(p->d_bw + planes_bytes);
-  auto* quanta = reinterpret_cast<double*>(p->d_bw + planes_bytes + ds_bytes);
-  auto* amax = reinterpret_cast<uint32_t*>(p->d_bw + planes_bytes + ds_bytes + q_bytes);
-  check_cuda(cudaMemsetAsync(amax, 0, K16 * 4, s), "memset");
-  const uint64_t na = (p->fam + 63) / 64 * p->K;
-  if (na) {
-    gnm_bw_amax<<<uint32_t((na + 255) / 256), 256, 0, s>>>(gsf, p->fam, p->K, amax);
-    check_cuda(cudaGetLastError(), "gradient maximum launch");
-    p->launches += 1;
-  }
-  const uint64_t nb = K16 * P_pad;
-  gnm_bw_build8<<<uint32_t((nb + 255) / 256), 256, 0, s>>>(gsf, p->fam, p->K, K16, P_pad, amax,
-                                                           planes, quanta, ds);
-  check_cuda(cudaGetLastError(), "gradient limb launch");
-  p->launches += 1;
-
-  const CUtensorMap rmap = make_row_map(d_rows, p->bpv, p->V, pitch, Bw8Smem::kPkRow, kBwM);
-  const CUtensorMap bmap =
-      make_2d_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, planes, P_pad, limb_rows, kBw8K, kBwN,
-                  CU_TENSOR_MAP_SWIZZLE_128B, "gradient limbs");
-  const CUtensorMap dmap = make_2d_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ds, K16, P_pad,
-                                       kBwScores, kBw8K, CU_TENSOR_MAP_SWIZZLE_NONE, "gradient");
-  check_cuda(raise_smem_limit(reinterpret_cast<const void*>(gnm_t8_backward), int(Bw8Smem::kTotal)),
-             "backward shared memory");
-  BwArgs a;
-  a.V = p->V;
-  a.K = p->K;
-  a.nstages = uint32_t(P_pad / kBw8K);
+  auto* quanta = reinterpret_cast<double*>(p->d_bw + planes_bytes);
+  auto* amax = reinterpret_cast<uint32_t*>(p->d_bw + planes_bytes + q_bytes);
+  a.quanta = quanta;
+  a.part = reinterpret_cast<double*>(p->d_bw + planes_bytes + q_bytes + amax_bytes);
   a.gw = d_grad_w;
   a.gc = d_grad_corr;
   a.err = p->d_err;
-  const dim3 grid(uint32_t((p->V + kBwM - 1) / kBwM), uint32_t(K16 / kBwScores));
-  gnm_t8_backward<<<grid, kBwThreads, Bw8Smem::kTotal, s>>>(rmap, bmap, dmap, a, quanta, K16);
-  check_cuda(cudaGetLastError(), "backward launch");
-  p->launches += 1;
+  a.rows = d_rows;
+  a.pitch = pitch;
+  a.ds = gsf;
+  a.people = p->fam;
+  check_cuda(cudaMemsetAsync(amax, 0, K16 * 4, s), "memset");
+  launch_bw_amax(p, gsf, amax, s);
+  gnm_bw_build8<<<dim3(uint32_t(P_pad / 32), uint32_t(stiles)), 512, 0, s>>>(
+      gsf, p->fam, p->K, K16, P_pad, amax, planes, quanta);
+  check_cuda(cudaGetLastError(), "gradient limb launch");
+
+  const CUtensorMap rmap = make_row_map(d_rows, p->bpv, p->V, pitch, Bw8Smem::kPkRow, kBw8Tile,
+                                        CU_TENSOR_MAP_SWIZZLE_128B);
+  const CUtensorMap bmap =
+      make_2d_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, planes, P_pad, limb_rows, 128, kBwN,
+                  CU_TENSOR_MAP_SWIZZLE_128B, "gradient limbs");
+  const dim3 grid(ctas, uint32_t(stiles));
+  auto launch = [&](auto kernel) {
+    check_cuda(raise_smem_limit(reinterpret_cast<const void*>(kernel), int(Bw8Smem::kTotal)),
+               "backward shared memory");
+    kernel<<<grid, kBw8Threads, Bw8Smem::kTotal, s>>>(rmap, bmap, a);
+    check_cuda(cudaGetLastError(), "backward launch");
+  };
+  if (d_grad_corr)
+    launch(gnm_t8_backward<true>);
+  else
+    launch(gnm_t8_backward<false>);
+  p->launches += 3;
+  if (a.quota % a.stages != 0 && ctas > 1) {   // some tile spans shares
+    gnm_bw_join<<<dim3(ctas - 1, uint32_t(stiles), 8), 256, 0, s>>>(a, ctas);
+    check_cuda(cudaGetLastError(), "backward join launch");
+    p->launches += 1;
+  }
 }
 
 void backward_dw(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, const float* d_grad_s,
@@ -3225,12 +3427,8 @@ void backward_dw(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, const float
   auto* ds = reinterpret_cast<float*>(p->d_bw + planes_bytes);
   auto* amax = reinterpret_cast<uint32_t*>(p->d_bw + planes_bytes + ds_bytes);
   check_cuda(cudaMemsetAsync(amax, 0, K16 * 4, s), "memset");
-  const uint64_t na = (p->fam + 63) / 64 * p->K;
-  if (na) {
-    gnm_bw_amax<<<uint32_t((na + 255) / 256), 256, 0, s>>>(gsf, p->fam, p->K, amax);
-    check_cuda(cudaGetLastError(), "gradient maximum launch");
-    p->launches += 1;
-  }
+  launch_bw_amax(p, gsf, amax, s);
+  p->launches += 1;
   const uint64_t nb = K16 * P_pad;
   gnm_bw_build<<<uint32_t((nb + 255) / 256), 256, 0, s>>>(gsf, p->fam, p->K, K16, P_pad, amax,
                                                           planes, ds);
