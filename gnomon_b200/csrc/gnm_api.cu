@@ -333,6 +333,33 @@ static void plain_shape(gnm_plan* p, uint32_t kernel, double mult) {
   p->split_mult = mult;
 }
 
+// The shape of a plan that is not tuned.  512-byte tiles (four scoring warps) for
+// every size: a cohort's last, partly filled tile wastes least, and several CTAs
+// per SM cover each other's waits.  Passes of three scores run best without the
+// producer warp, whose registers they need (30,011 people x 150,007 variants,
+// uneven scores: 0.91 against 1.05 ms); one and two scores with it (1.44 against
+// 1.49 ms on 50,000 x 400,000 x 1).  Splits per tile: whole waves of CTAs, just
+// under, since one CTA more costs a wave (78 splits of the 15 tiles above: 0.91
+// ms, 83: 0.97), as many as leave about 60 stages in a CTA and at most six, so
+// that uneven CTAs even out (50,000 x 1,000,000 x 1: 3.83 ms at one wave, 3.55
+// at six).  Where one wave has fewer than 12 stages per CTA, one CTA per SM: a
+// CTA's start and its partials would cost more than its stages (2,000 x 50,000:
+// 23 us at 139 splits, 48 us at 592).
+static void plain_shape_default(gnm_plan* p) {
+  const uint32_t kernel = p->K >= 3 ? kPlain512 : kPlain512Ws;
+  const uint64_t tiles = std::max<uint64_t>(1, (p->bpv + 511) / 512);
+  const uint64_t stages = std::max<uint64_t>(1, (p->V + kPlainRows - 1) / kPlainRows);
+  const uint64_t slots = uint64_t(plain_ctas_per_sm(kernel)) * uint64_t(p->num_sms);
+  const uint64_t waves =
+      std::min<uint64_t>(6, std::max<uint64_t>(1, (stages * tiles + 30 * slots) / (60 * slots)));
+  const uint64_t splits =
+      waves > 1 ? waves * slots / tiles
+                : std::max(std::min(stages, uint64_t(p->num_sms) / tiles),
+                           std::min(slots / tiles, (stages + 11) / 12));
+  plain_shape_fixed(p, kernel,
+                    uint32_t(std::min<uint64_t>(0xFFFFu, std::max<uint64_t>(1, splits))));
+}
+
 static void plain_geometry(gnm_plan* p) {
   // partial slots are padded to whole tiles of the widest kernel, so every
   // kernel's people index stays inside a slot
@@ -340,7 +367,7 @@ static void plain_geometry(gnm_plan* p) {
                    kPlainWideTileBytes * 4;
   check_cuda(cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device),
              "cudaDeviceGetAttribute");
-  plain_shape(p, kPlainDefaultKernel, 1.0);
+  plain_shape_default(p);
   // keep partials of all scores within 8 GiB (many score columns still get a
   // full-occupancy grid); allocate room for the autotuner's largest candidate
   // (eight times the CTA slots, any kernel)
@@ -357,12 +384,8 @@ static void plain_geometry(gnm_plan* p) {
   }
   while (alloc > 1 && alloc * per_split_bytes > cap) --alloc;
   p->splits_alloc = uint32_t(alloc);
-  // shrink the default grid until its slots fit the allocation
-  double mult = 1.0;
-  while (p->slots > p->splits_alloc && mult > 1e-3) {
-    mult *= 0.5;
-    plain_shape(p, kPlainDefaultKernel, mult);
-  }
+  // keep the default grid's slots inside the allocation
+  if (p->slots > p->splits_alloc) plain_shape_fixed(p, p->kernel, p->splits_alloc);
 }
 
 static void upload_plain_records(gnm_plan* p, const std::vector<float4>& rec, PhaseTrace& trace);
@@ -403,6 +426,9 @@ static void build_plain_records(gnm_plan* p, const gnm_prep_view* prep, PhaseTra
   upload_plain_records(p, rec, trace);
 }
 
+// Scores one launch takes on its grid's y dimension.
+constexpr uint64_t kMaxGridY = 65535;
+
 // Upload a plain plan's cell records, allocate its partials and build the
 // stage tables while they fit the cache.
 static void upload_plain_records(gnm_plan* p, const std::vector<float4>& rec, PhaseTrace& trace) {
@@ -424,25 +450,31 @@ static void upload_plain_records(gnm_plan* p, const std::vector<float4>& rec, Ph
   if (p->K * stages * kPlainTableBytes <= kTableCacheBytes) {
     p->tab_stages = stages;
     p->d_tables = dalloc<uint8_t>(p, p->K * stages * kPlainTableBytes, "cudaMalloc(stage tables)");
-    for (uint64_t k = 0; k < p->K; ++k) {
+    for (uint64_t k = 0; k < p->K; k += kMaxGridY) {
       TableArgs t{};
       t.records = p->d_records + k * p->rec_stride;
       t.row0 = 0;
       t.num_rows = p->V;
       t.tables = p->d_tables + k * stages * kPlainTableBytes;
+      t.scores = uint32_t(std::min(kMaxGridY, p->K - k));
+      t.record_stride = p->rec_stride;
+      t.table_stride = stages * kPlainTableBytes;
       check_cuda(launch_plain_tables(t, 0), "stage table launch");
     }
   }
 }
 
-// Stage tables for score k over block rows [v0, v0 + nv): the cached tables
-// when the block starts on a stage boundary, else a fresh build into scratch.
-static const uint8_t* plain_tables_for(gnm_plan* p, uint64_t k, uint64_t v0, uint64_t nv,
-                                       cudaStream_t s) {
-  if (p->d_tables && v0 % kPlainRows == 0)
+// Stage tables for scores [k, k + n) over block rows [v0, v0 + nv), `stride`
+// bytes apart: the cached tables when the block starts on a stage boundary, else
+// a fresh build into scratch.
+static const uint8_t* plain_tables_for(gnm_plan* p, uint64_t k, uint32_t n, uint64_t v0,
+                                       uint64_t nv, uint64_t* stride, cudaStream_t s) {
+  if (p->d_tables && v0 % kPlainRows == 0) {
+    *stride = p->tab_stages * kPlainTableBytes;
     return p->d_tables + (k * p->tab_stages + v0 / kPlainRows) * kPlainTableBytes;
+  }
   const uint64_t stages = (nv + kPlainRows - 1) / kPlainRows;
-  if (stages > p->tab_scratch_stages) {
+  if (n * stages > p->tab_scratch_stages) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     check_cuda(cudaStreamIsCapturing(s, &cs), "cudaStreamIsCapturing");
     if (cs != cudaStreamCaptureStatusNone)
@@ -456,14 +488,19 @@ static const uint8_t* plain_tables_for(gnm_plan* p, uint64_t k, uint64_t v0, uin
       p->d_tab_scratch = nullptr;
       p->tab_scratch_stages = 0;
     }
-    p->d_tab_scratch = dalloc<uint8_t>(p, stages * kPlainTableBytes, "cudaMalloc(table scratch)");
-    p->tab_scratch_stages = stages;
+    p->d_tab_scratch =
+        dalloc<uint8_t>(p, n * stages * kPlainTableBytes, "cudaMalloc(table scratch)");
+    p->tab_scratch_stages = n * stages;
   }
+  *stride = stages * kPlainTableBytes;
   TableArgs t{};
   t.records = p->d_records + k * p->rec_stride;
   t.row0 = v0;
   t.num_rows = nv;
   t.tables = p->d_tab_scratch;
+  t.scores = n;
+  t.record_stride = p->rec_stride;
+  t.table_stride = *stride;
   check_cuda(launch_plain_tables(t, s), "stage table launch");
   ++p->launches;
   return p->d_tab_scratch;
@@ -555,7 +592,6 @@ static void accumulate_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, 
   const CUtensorMap map = make_row_map(d_rows, p->bpv, nv, pitch, kPlainBoxBytes, kPlainRows);
   const uint64_t stages = (nv + kPlainRows - 1) / kPlainRows;
   const uint32_t sps = uint32_t((stages + p->splits - 1) / p->splits);
-  const uint32_t lsps = uint32_t((stages + p->last_splits - 1) / p->last_splits);
   // Slots this launch covers (every tile gets the same count).  The first
   // launch after a reset writes them; a later one adds, after clearing any
   // slots past those written so far.
@@ -573,22 +609,37 @@ static void accumulate_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, 
                "clear partials");
   }
   p->valid_slots = std::max(p->valid_slots, covered);
-  for (uint64_t k = 0; k < p->K; ++k) {
+  // Passes of kPlainPassScores scores, the rest in a last one.  Two scores share a
+  // pass in two launches, each over half of the splits (callers count one
+  // accumulate and one finalize launch per score up to two scores); where half
+  // of the splits do not fill the SMs they go one by one.
+  const uint64_t half_ctas = uint64_t(p->tiles) * covered / 2;
+  const bool halves = p->K == 2 && half_ctas >= uint64_t(p->num_sms) * plain_ctas_per_sm(p->kernel);
+  const uint32_t pass = p->K == 2 && !halves ? 1u : kPlainPassScores;
+  for (uint64_t k = 0; k < p->K;) {
+    const uint32_t n = uint32_t(std::min<uint64_t>(pass, p->K - k));
     PlainArgs a;
-    a.tables = plain_tables_for(p, k, v0, nv, s);
+    a.tables = plain_tables_for(p, k, n, v0, nv, &a.table_stride, s);
     a.num_rows = nv;
     a.bytes_per_row = p->bpv;
     a.tiles = p->tiles;
     a.splits = uint32_t((stages + sps - 1) / sps);   // non-empty splits of a full tile
     a.stages_per_split = sps;
-    a.last_stages_per_split = lsps;
-    a.part_sum = p->d_part_sum + k * uint64_t(p->splits_alloc) * p->part_stride;
-    a.part_cnt = p->d_part_cnt + k * uint64_t(p->splits_alloc) * p->part_stride;
+    a.score_stride = uint64_t(p->splits_alloc) * p->part_stride;
+    a.part_sum = p->d_part_sum + k * a.score_stride;
+    a.part_cnt = p->d_part_cnt + k * a.score_stride;
     a.part_stride = p->part_stride;
     a.err = p->d_err;
     a.store = store ? 1u : 0u;
-    check_cuda(launch_plain_accumulate(map, a, p->kernel, s), "plain accumulate launch");
-    ++p->launches;
+    const uint32_t all = a.splits;
+    const uint32_t parts = halves ? 2 : 1;
+    for (uint32_t h = 0; h < parts; ++h) {
+      a.split0 = h * (all / 2);
+      a.splits = h + 1 < parts ? all / 2 : all - a.split0;
+      check_cuda(launch_plain_accumulate(map, a, p->kernel, n, s), "plain accumulate launch");
+      ++p->launches;
+    }
+    k += n;
   }
 }
 
@@ -599,10 +650,13 @@ static void finalize_impl(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool 
     tensor_finalize(p, d_sums, d_counts, add_baseline, s);
     return;
   }
-  for (uint64_t k = 0; k < p->K; ++k) {
+  // every score in one launch; up to two scores, one launch each (see accumulate)
+  const uint64_t step = p->K <= 2 ? 1 : kMaxGridY;
+  for (uint64_t k = 0; k < p->K; k += step) {
     FinalizeArgs a;
-    a.part_sum = p->d_part_sum + k * uint64_t(p->splits_alloc) * p->part_stride;
-    a.part_cnt = p->d_part_cnt + k * uint64_t(p->splits_alloc) * p->part_stride;
+    a.score_stride = uint64_t(p->splits_alloc) * p->part_stride;
+    a.part_sum = p->d_part_sum + k * a.score_stride;
+    a.part_cnt = p->d_part_cnt + k * a.score_stride;
     a.part_stride = p->part_stride;
     a.num_splits = p->valid_slots;
     a.baseline = add_baseline ? p->d_baseline : p->d_zero_base;
@@ -610,6 +664,7 @@ static void finalize_impl(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool 
     a.num_people = p->P;
     a.K = p->K;
     a.k = k;
+    a.scores = uint32_t(std::min(step, p->K - k));
     a.sums = d_sums;
     a.counts = d_counts;
     check_cuda(launch_finalize(a, s), "finalize launch");

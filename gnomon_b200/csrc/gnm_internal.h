@@ -25,9 +25,12 @@ constexpr uint32_t kPlainWideTileBytes = 2048;   // also the partial-slot paddin
 constexpr uint32_t kPlainBoxBytes = 256;     // TMA box inner extent (max 256 elements)
 constexpr uint32_t kPlainRows = 30;          // variant rows per pipeline stage (10 groups of 3)
 constexpr uint32_t kPlainGroups = kPlainRows / 3;
-// One stage table: 10 group tables of 64 FP32 entries (256 B each) + the
-// stage's membership word, padded to a multiple of 16 bytes (bulk copies).
-constexpr uint32_t kPlainTableBytes = kPlainGroups * 256 + 16;   // 2576
+// One stage table: 10 group tables of 64 int32 entries (256 B each), the stage's
+// membership word and grid step (16 B), and a 0 / 1 membership word per row
+// (32 words; a multiple of 16 bytes in all, for bulk copies).
+constexpr uint32_t kPlainTailOff = kPlainGroups * 256;
+constexpr uint32_t kPlainRowsOff = kPlainTailOff + 16;
+constexpr uint32_t kPlainTableBytes = kPlainRowsOff + 128;   // 2704
 constexpr uint32_t kRecordPad = 64;          // zero records past the last variant
 constexpr uint64_t kTableCacheBytes = uint64_t(4) << 30;  // per-plan stage-table cache budget
 
@@ -41,19 +44,26 @@ struct TableArgs {
   uint64_t row0;           // index of table row 0 in the source arrays
   uint64_t num_rows;       // rows covered; tables for ceil(num_rows / kPlainRows) stages
   uint8_t* tables;         // out: [stages][kPlainTableBytes]
+  uint32_t scores = 1;     // scores built by the launch (grid.y, at most 65,535)
+  uint64_t record_stride = 0, table_stride = 0;   // records, table bytes between them
 };
+
+// Score columns one pass over the rows can serve.
+constexpr uint32_t kPlainPassScores = 3;
 
 struct PlainArgs {
   const uint8_t* tables;   // [stages of this block][kPlainTableBytes], stage 0 = block row 0
+  uint64_t table_stride;   // bytes between the tables of the pass's scores
   uint64_t num_rows;       // rows in this block
   uint64_t bytes_per_row;  // meaningful bytes of a row (ceil(people / 4))
   uint32_t tiles;          // people tiles (the last may be partly populated)
-  uint32_t splits;         // variant splits of each full tile (CTAs per full tile)
-  uint32_t stages_per_split;        // stages per split of a full tile
-  uint32_t last_stages_per_split;   // stages per split of the last tile
-  double* part_sum;        // [splits][part_stride] partials of this score
+  uint32_t splits;         // variant splits of each tile in this launch (CTAs per tile)
+  uint32_t split0 = 0;     // the first of them
+  uint32_t stages_per_split;
+  double* part_sum;        // [splits][part_stride] partials of the pass's first score
   uint32_t* part_cnt;
   uint64_t part_stride;
+  uint64_t score_stride;   // partials between the pass's scores
   uint32_t* err;
   uint32_t store = 0;      // 1: write the partials (first launch since a reset); 0: add to them
 };
@@ -66,7 +76,9 @@ struct FinalizeArgs {
   const double* baseline;   // [K]
   const uint32_t* out_to_fam;
   uint64_t num_people;
-  uint64_t K, k;
+  uint64_t K, k;            // columns, first column of the launch
+  uint32_t scores = 1;      // columns of the launch (grid.y, at most 65,535)
+  uint64_t score_stride = 0;   // partials between columns
   double* sums;             // [P][K]
   uint32_t* counts;
 };
@@ -88,16 +100,14 @@ enum : uint32_t {
 };
 constexpr uint32_t kPlainKernels[] = {kPlain1024, kPlain512, kPlain512Ws, kPlain1024Ws,
                                       kPlain2048Ws};
-constexpr uint32_t kPlainDefaultKernel = kPlain2048Ws;   // fastest on the bandwidth workload
 inline uint32_t plain_tile_bytes(uint32_t kernel) { return kernel & ~1u; }
 inline uint32_t plain_ctas_per_sm(uint32_t kernel) {
   return plain_tile_bytes(kernel) >= 2048 ? 1u : 2048u / plain_tile_bytes(kernel);
 }
 
-// Launches (tiles - 1) * splits + ceil(stages / last_stages_per_split) CTAs of
-// the given plain kernel.
+// Launches tiles * splits CTAs of the given plain kernel for `scores` (1 to kPlainPassScores) score columns.
 cudaError_t launch_plain_accumulate(const CUtensorMap& map, const PlainArgs& a, uint32_t kernel,
-                                    cudaStream_t s);
+                                    uint32_t scores, cudaStream_t s);
 uint32_t plain_grid(const PlainArgs& a);
 cudaError_t launch_finalize(const FinalizeArgs& a, cudaStream_t s);
 cudaError_t launch_repitch(const uint8_t* src, uint64_t bpv, uint64_t nrows, uint8_t* dst,

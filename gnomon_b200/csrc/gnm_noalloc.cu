@@ -127,17 +127,18 @@ static void score_noalloc(const uint8_t* d_rows, uint64_t pitch, uint64_t V, uin
     const uint64_t cst = (nv + kPlainRows - 1) / kPlainRows;
     PlainArgs a;
     a.tables = tables;
+    a.table_stride = 0;
     a.num_rows = nv;
     a.bytes_per_row = bpv;
     a.tiles = tiles;
     a.splits = uint32_t((cst + sps - 1) / sps);   // the same split count for every tile
     a.stages_per_split = sps;
-    a.last_stages_per_split = sps;
     a.part_sum = part_sum;
     a.part_cnt = part_cnt;
     a.part_stride = stride;
+    a.score_stride = 0;
     a.err = err;
-    check_cuda(launch_plain_accumulate(map, a, kPlain1024, s), "plain accumulate launch");
+    check_cuda(launch_plain_accumulate(map, a, kPlain1024, 1, s), "plain accumulate launch");
   }
   FinalizeArgs f;
   f.part_sum = part_sum;

@@ -2,7 +2,7 @@
 //
 // Replaces the reference GPU engine's unpack_plink -> zero -> scatter ->
 // 3x SGEMM -> combine chain (score/cuda_backend.rs:62-218, 2067-2333) for small
-// score counts with one fused accumulate kernel per score column:
+// score counts with one fused accumulate kernel for one to three score columns:
 //
 //   * the weights of every 3 consecutive variant rows are folded once per plan
 //     (gnm_plain_tables) into a 64-entry table: entry (ca, cb, cc) is the exact
@@ -10,13 +10,12 @@
 //     dosage_weight, 2*dosage_weight} (prepare.rs:197-208 folding; code 00
 //     contributes 0), put on the stage's int32 fixed-point grid, so decode,
 //     effect-allele flip and the missing-call rule become ONE lookup per
-//     person per 3 variants; ten group tables, the membership word and the
-//     grid step make one 2576-byte stage table;
+//     person per 3 variants; ten group tables, the membership words and the
+//     grid step make one 2704-byte stage table;
 //   * packed .bed rows are TMA-staged (cp.async.bulk.tensor into this CTA
-//     only) in [30 rows x TILE bytes] stages with their stage table (a 1D bulk
-//     copy on the same mbarrier), three buffers deep; TILE is 512, 1024 or
-//     2048 bytes of every row (2048, 4096 or 8192 people), the autotuner's
-//     choice;
+//     only) in [30 rows x TILE bytes] stages with their stage tables (1D bulk
+//     copies on the same mbarrier), two or three buffers deep; TILE is 512,
+//     1024 or 2048 bytes of every row (2048, 4096 or 8192 people);
 //   * each thread owns one 32-bit word column = 16 people; per 3 rows it
 //     transposes the 2-bit codes into per-person 6-bit indices (one byte each,
 //     pre-scaled by 4) with shift/mask ops and turns each byte into a
@@ -24,11 +23,12 @@
 //     groups' lookups go into a person's sum with one three-input add;
 //   * warps run the stages independently: a warp waits only for the stage's
 //     TMA; it releases the buffer either through a shared counter whose last
-//     arriver issues the TMA of the stage three ahead, or (producer-warp
+//     arriver issues the TMA of the buffer's next stage, or (producer-warp
 //     kernels) by arriving on a release mbarrier that a producer warp waits on
 //     before it issues that TMA — no CTA-wide barrier per stage;
 //   * missing calls (code 01) are counted with SWAR bit tricks on the raw row
-//     words (x & ~(x>>1) & member_mask, three rows summed with one add);
+//     words (x & ~(x>>1) & 0x55555555), per score only where the scores'
+//     members differ;
 //   * a stage's ten lookups per person add up exactly in int32 and reach FP64
 //     once per stage (sum x grid step); variant splits write FP64 partials
 //     that gnm_finalize reduces in a fixed order (deterministic) and gathers
@@ -40,32 +40,44 @@
 
 #include "gnm_device.cuh"
 #include "gnm_internal.h"
+#include "gnm_tcgen05.cuh"
 
 namespace gnm {
 
 // Shared-memory layout of one plain CTA (dynamic smem, offsets in bytes) for
 // a people tile of TILE bytes of every row (TILE / 4 threads, 4 * TILE people).
-template <uint32_t TILE>
+template <uint32_t TILE, uint32_t NS>
 struct PlainSmem {
-  static constexpr uint32_t kStages = 3;
+  // 512-byte tiles take two buffers: with three, two and three scores leave
+  // room for three CTAs per SM instead of four (two scores, 30,011 people x
+  // 150,007 variants x 4: 1.14 against 1.16 ms; one score: no difference)
+  static constexpr uint32_t kStages = TILE == 512 ? 2 : 3;
   static constexpr uint32_t kThreads = TILE / 4;
   static constexpr uint32_t kWarps = kThreads / 32;
   static constexpr uint32_t kBoxes = TILE / kPlainBoxBytes;                  // TMA boxes per stage
   static constexpr uint32_t kStageBytes = kPlainRows * TILE;                 // 30720 at 1 KB
   static constexpr uint32_t kBoxBytes = kPlainRows * kPlainBoxBytes;         // 7680
-  static constexpr uint32_t kTabStride = 3072;   // one stage table, padded to 1 KB in total
+  static constexpr uint32_t kTabOne = 3072;      // one score's stage table, padded
+  static constexpr uint32_t kTabStride = NS * kTabOne;
   static constexpr uint32_t kTabOff = 0;
-  static constexpr uint32_t kTileOff = kTabOff + kStages * kTabStride;      // 9216
+  static constexpr uint32_t kTileOff = kTabOff + kStages * kTabStride;
   static constexpr uint32_t kBarOff = kTileOff + kStages * kStageBytes;     // 3 mbarriers
   static constexpr uint32_t kRelOff = kBarOff + 8 * kStages;                // 3 release counters
   static constexpr uint32_t kLastOff = kRelOff + 4 * kStages;               // 3 last-issued stages
   static constexpr uint32_t kEmptyOff = kLastOff + 4 * kStages;             // 3 "released" mbarriers
-  static constexpr uint32_t kTotal = kEmptyOff + 8 * kStages;
+  static constexpr uint32_t kHolder = kEmptyOff + 8 * kStages;              // tensor memory address
+  static constexpr uint32_t kTotal = kHolder + 8;
+  // FP64 sums of a warp's people: 2 x 16 columns per score of its lane quadrant
+  static constexpr uint32_t kWarpCols = 32 * NS;
+  static constexpr uint32_t kCols = kWarpCols * (kWarps / 4);
+  static constexpr uint32_t kTmemCols = kCols <= 32 ? 32 : kCols <= 64 ? 64 : kCols <= 128 ? 128
+                                                      : kCols <= 256 ? 256 : 512;
+  static_assert(kCols <= 512 && kTotal <= 227 * 1024, "tensor memory, shared memory");
   static_assert(kEmptyOff % 8 == 0, "mbarrier alignment");
   static_assert(TILE % kPlainBoxBytes == 0 && TILE % 128 == 0, "whole boxes and warps");
   static_assert(kPlainRows % 3 == 0 && kPlainRows <= 32, "groups of 3 rows, one ballot");
   static_assert(kPlainGroups % 2 == 0, "groups are scored in pairs");
-  static_assert(kTabStride >= kPlainTableBytes && kTabStride % 256 == 0, "table stride");
+  static_assert(kTabOne >= kPlainTableBytes && kTabOne % 256 == 0, "table stride");
   static_assert(kTileOff % 1024 == 0, "tile alignment");
   // Each 64-entry group table starts on a 256-byte boundary, so a lookup
   // address is the table address plus the index byte (no carry).
@@ -84,9 +96,12 @@ __constant__ uint32_t c_mul[5] = {2u, 4u, 16u, 64u, 1u};
 // the compiler keeps the dot product.
 __constant__ uint32_t c_sel[4] = {0x1u, 0x100u, 0x10000u, 0x1000000u};
 
+// Shared load at a register plus a constant: scores of a pass differ only in the
+// constant, so one address serves all their lookups.
+template <uint32_t OFF>
 __device__ __forceinline__ int32_t lds_s32(uint32_t addr) {
   int32_t v;
-  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(addr));
+  asm volatile("ld.shared.s32 %0, [%1 + %2];" : "=r"(v) : "r"(addr), "n"(OFF));
   return v;
 }
 
@@ -133,10 +148,12 @@ __device__ __forceinline__ bool table_member(const TableArgs& a, uint64_t row) {
   return a.member == nullptr || a.member[a.row0 + row] != 0;
 }
 
-// grid.x = stages, block = kPlainGroups groups x 64 entries.
+// grid = stages x scores, block = kPlainGroups groups x 64 entries.
 __global__ void __launch_bounds__(kPlainGroups * 64) gnm_plain_tables(TableArgs a) {
   __shared__ float s_max[kPlainGroups * 2];
   const uint64_t stage = blockIdx.x;
+  if (a.records) a.records += blockIdx.y * a.record_stride;
+  a.tables += blockIdx.y * a.table_stride;
   const uint32_t e = threadIdx.x, g = e >> 6, idx = e & 63u;
   const uint32_t lc = (idx >> 5) & 1u;
   const uint32_t code[3] = {(idx & 3u) ^ lc, ((idx >> 2) & 3u) ^ lc, ((idx >> 3) & 2u) | lc};
@@ -166,8 +183,9 @@ __global__ void __launch_bounds__(kPlainGroups * 64) gnm_plain_tables(TableArgs 
     const bool mem = e < kPlainRows && row < a.num_rows && table_member(a, row);
     const uint32_t bits = __ballot_sync(0xFFFFFFFFu, mem);
     if (e < 4)
-      reinterpret_cast<uint32_t*>(tab + kPlainGroups * 256)[e] =
+      reinterpret_cast<uint32_t*>(tab + kPlainTailOff)[e] =
           e == 0 ? bits : (e == 1 ? __float_as_uint(q) : 0u);
+    reinterpret_cast<uint32_t*>(tab + kPlainRowsOff)[e] = mem ? 1u : 0u;
   }
 }
 
@@ -175,58 +193,63 @@ __global__ void __launch_bounds__(kPlainGroups * 64) gnm_plain_tables(TableArgs 
 
 // Copies of one stage: the tile's first `boxes` row boxes (the ones that hold
 // row bytes) and the stage table, on the buffer's mbarrier.
-template <uint32_t TILE>
-__device__ __forceinline__ void plain_issue_stage(const CUtensorMap* map, const uint8_t* tables,
+template <uint32_t TILE, uint32_t NS>
+__device__ __forceinline__ void plain_issue_stage(const CUtensorMap* map, const PlainArgs& a,
                                                   uint32_t smem_base, uint32_t buf,
                                                   int32_t tile_x, int32_t row0, uint64_t stage,
                                                   uint32_t boxes) {
-  using L = PlainSmem<TILE>;
+  using L = PlainSmem<TILE, NS>;
   const uint32_t bar = smem_base + L::kBarOff + 8 * buf;
-  mbar_arrive_expect_tx(bar, boxes * L::kBoxBytes + kPlainTableBytes);
+  mbar_arrive_expect_tx(bar, boxes * L::kBoxBytes + NS * kPlainTableBytes);
   const uint32_t tile = smem_base + L::kTileOff + buf * L::kStageBytes;
   for (uint32_t b = 0; b < boxes; ++b)
     tma_load_2d(tile + b * L::kBoxBytes, map, tile_x + int32_t(b * kPlainBoxBytes), row0, bar);
-  bulk_load(smem_base + L::kTabOff + buf * L::kTabStride, tables + stage * kPlainTableBytes,
-            kPlainTableBytes, bar);
+#pragma unroll
+  for (uint32_t s = 0; s < NS; ++s)
+    bulk_load(smem_base + L::kTabOff + buf * L::kTabStride + s * L::kTabOne,
+              a.tables + s * a.table_stride + stage * kPlainTableBytes, kPlainTableBytes, bar);
 }
 
-template <uint32_t TILE, bool WS>
+template <uint32_t TILE, bool WS, uint32_t NS>
 struct PlainShape {
   static constexpr uint32_t kThreads = TILE / 4 + (WS ? 32u : 0u);
-  static constexpr uint32_t kMinBlocks = TILE >= 2048 ? 1u : 2048u / TILE;
+  // as many CTAs as 227 KB of shared memory hold
+  static constexpr uint32_t kFit = 227u * 1024u / (PlainSmem<TILE, NS>::kTotal + 1024u);
+  static constexpr uint32_t kMinBlocks = kFit > 4u ? 4u : kFit;
 };
 
-// One CTA per (people tile, variant split).  The grid is 1D: the first
-// (tiles - 1) * splits CTAs cover the full tiles, `splits` each, and the last
-// tile (often only partly populated by people) has its own stages-per-split
-// field; the host gives it the same split count as the others, because a
-// CTA's time per stage is set by each warp's dependency chains, not by how
-// many of its warps hold people.  block = TILE / 4 scoring threads, plus (WS) one
-// producer warp that issues every stage's copies once the scoring warps have
-// released its buffer (they arrive on an mbarrier and never wait for one
-// another); without it the scoring warp that releases a buffer last issues
+// One CTA per (people tile, variant split), for NS score columns.  The last tile
+// (often only partly populated by people) has as many splits as the others,
+// because a CTA's time per stage is set by each warp's dependency chains, not
+// by how many of its warps hold people.  block = TILE / 4 scoring threads, plus
+// (WS) one producer warp that issues every stage's copies once the scoring
+// warps have released its buffer (they arrive on an mbarrier and never wait for
+// one another); without it the scoring warp that releases a buffer last issues
 // the refill.
-template <uint32_t TILE, bool WS>
-__global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TILE, WS>::kMinBlocks)
+//
+// Registers: the FP64 sums live in tensor memory (a lane per thread, two
+// columns per person and score) and are read, added to and written back once
+// per stage; the 32-bit missing counts live in the partials and are added to
+// every eight stages.  What is left, 16 stage sums per score, lets NS scores
+// share a pass: its row words, index transposes, lookup addresses and (where
+// every row is a member of all its scores) missing counts are computed once.
+// Per 3 rows x 16 people a pass of one score takes 81 instructions, of three
+// 43 per score, and the table lookups' shared-memory wavefronts become the
+// bound (18.1 of 19 per score).
+template <uint32_t TILE, bool WS, uint32_t NS>
+__global__ void __launch_bounds__(PlainShape<TILE, WS, NS>::kThreads,
+                                  PlainShape<TILE, WS, NS>::kMinBlocks)
     gnm_plain_accumulate(const __grid_constant__ CUtensorMap map, PlainArgs a) {
-  using L = PlainSmem<TILE>;
+  using L = PlainSmem<TILE, NS>;
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const uint32_t tid = threadIdx.x, lane = tid & 31u;
   const bool producer = WS && tid >= L::kThreads;
-  const uint32_t full_ctas = (a.tiles - 1) * a.splits;
-  uint32_t tile, split, sps;
-  if (blockIdx.x < full_ctas) {
-    tile = blockIdx.x / a.splits;
-    split = blockIdx.x % a.splits;
-    sps = a.stages_per_split;
-  } else {
-    tile = a.tiles - 1;
-    split = blockIdx.x - full_ctas;
-    sps = a.last_stages_per_split;
-  }
+  // tiles fastest: the CTAs that run together read whole rows, and share the
+  // stage tables of their splits in L2
+  const uint32_t tile = blockIdx.x % a.tiles, split = a.split0 + blockIdx.x / a.tiles;
 
-  const uint64_t rows_per_split = uint64_t(sps) * kPlainRows;
+  const uint64_t rows_per_split = uint64_t(a.stages_per_split) * kPlainRows;
   const uint64_t r_begin = uint64_t(split) * rows_per_split;
   if (r_begin >= a.num_rows) return;
   // table addresses are formed by byte replacement: the window must be aligned
@@ -260,7 +283,13 @@ __global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TIL
     }
     fence_mbar_init();
   }
+  if (tid < 32) {
+    tmem_alloc(sbase + L::kHolder, L::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
   if (WS && producer) {
     // ---- producer warp: every stage's copies, each once its buffer is free
     bool ok = true;
@@ -268,7 +297,7 @@ __global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TIL
       for (uint32_t st = 0; st < nstages; ++st) {
         const uint32_t buf = st % L::kStages;
         if (st >= L::kStages) {
-          // the scoring warps released stage st - 3 of this buffer
+          // the scoring warps released this buffer's last stage
           if (!mbar_wait_bounded(empty0 + 8 * buf, ((st / L::kStages) - 1) & 1u)) {
             atomicOr(a.err, kErrTmaTimeout);
             ok = false;
@@ -277,8 +306,9 @@ __global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TIL
           fence_proxy_async_smem();
         }
         last_issued[buf] = st;
-        plain_issue_stage<TILE>(&map, a.tables, sbase, buf, tile_x,
-                                int32_t(r_begin + uint64_t(st) * kPlainRows), stage0 + st, boxes);
+        plain_issue_stage<TILE, NS>(&map, a, sbase, buf, tile_x,
+                                    int32_t(r_begin + uint64_t(st) * kPlainRows), stage0 + st,
+                                    boxes);
       }
     }
     // every warp of the CTA meets here (the scoring warps at the end of their loop)
@@ -293,37 +323,45 @@ __global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TIL
   if (!WS && tid == 0) {
     for (uint32_t s = 0; s < L::kStages && s < nstages; ++s) {
       last_issued[s] = s;
-      plain_issue_stage<TILE>(&map, a.tables, sbase, s, tile_x,
-                              int32_t(r_begin + s * kPlainRows), stage0 + s, boxes);
+      plain_issue_stage<TILE, NS>(&map, a, sbase, s, tile_x, int32_t(r_begin + s * kPlainRows),
+                                  stage0 + s, boxes);
     }
   }
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + L::kHolder);
+  const uint32_t warp = tid >> 5;
+  // this warp's sums: its lane quadrant, kWarpCols columns
+  const uint32_t sums = tmem + ((32 * (warp & 3u)) << 16) + (warp >> 2) * L::kWarpCols;
 
-  // int32 fixed-point sums of the current stage: iacc[4j + q] is person
+  // int32 fixed-point sums of the current stage: iacc[s][4j + q] is person
   // 4j + q of this thread's 16 (exact: <= 10 lookups of |entry| <= 2^27 + 1).
-  int32_t iacc[16];
-  double acc64[16];
-  uint32_t cnt[16];
-  uint32_t by[4] = {0u, 0u, 0u, 0u};   // byte counters: byte j = person 4j+q
+  int32_t iacc[NS][16];
+  // byte counters of the stages since the last flush (byte j of [q] = person
+  // 4j + q): stages whose rows are all members of every score count once for
+  // all of them, other stages per score
+  uint32_t all[4] = {0u, 0u, 0u, 0u};
+  uint32_t by[NS][4];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    acc64[i] = 0.0;
-    cnt[i] = 0u;
+  for (uint32_t s = 0; s < NS; ++s) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) iacc[s][i] = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) by[s][q] = 0u;
   }
-#pragma unroll
-  for (int i = 0; i < 16; ++i) iacc[i] = 0;
 
   // Each thread reads word column `tid` of the TILE-byte stage row; the stage
   // is stored as TILE / 256 TMA boxes of [kPlainRows rows][256 bytes].
   const uint32_t word_off = (tid / (kPlainBoxBytes / 4)) * L::kBoxBytes +
                             (tid % (kPlainBoxBytes / 4)) * 4;
   // warps whose 128 bytes all lie past the row's last byte only hold padding
-  const bool warp_active = (tid >> 5) < active_warps;
+  const bool warp_active = warp < active_warps;
+  const uint64_t person0 = uint64_t(tile) * (TILE * 4) + uint64_t(tid) * 16;
+  const uint64_t slot0 = uint64_t(split) * a.part_stride + person0;
 
   bool failed = false;
   for (uint32_t st = 0; st < (warp_active ? nstages : 0u); ++st) {
     const uint32_t buf = st % L::kStages;
     const uint32_t parity = (st / L::kStages) & 1u;
-    if (!mbar_wait_bounded(bar0 + 8 * buf, parity)) {
+    if (!mbar_wait_warp(bar0 + 8 * buf, parity)) {   // (the warp stays whole: tensor memory)
       if (lane == 0) atomicOr(a.err, kErrTmaTimeout);
       failed = true;
       break;
@@ -334,18 +372,23 @@ __global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TIL
     // wait above clobbers memory, so none moves above it); table lookups go
     // through 32-bit shared addresses.
     const uint8_t* tbase = smem + L::kTileOff + buf * L::kStageBytes + word_off;
+    const uint8_t* tab = smem + L::kTabOff + buf * L::kTabStride;
     const uint32_t lbase = sbase + L::kTabOff + buf * L::kTabStride;
-    const uint64_t members = *reinterpret_cast<const uint32_t*>(
-        smem + L::kTabOff + buf * L::kTabStride + kPlainGroups * 256);
-    // the stage's grid step, read before the buffer is released
-    const float stage_q = *reinterpret_cast<const float*>(
-        smem + L::kTabOff + buf * L::kTabStride + kPlainGroups * 256 + 4);
+    // the stage's member words and grid steps, read before the buffer is released
+    float stage_q[NS];
+    uint32_t every = 0xFFFFFFFFu, some = 0u;
+#pragma unroll
+    for (uint32_t s = 0; s < NS; ++s) {
+      const uint32_t* tail =
+          reinterpret_cast<const uint32_t*>(tab + s * L::kTabOne + kPlainTailOff);
+      stage_q[s] = __uint_as_float(tail[1]);
+      every &= tail[0];
+      some |= tail[0];
+    }
 
-    uint32_t ev = 0, od = 0;             // nibble counters (people 2j / 2j+1)
-    // Row words of group g -> four index words; returns the group's missing
-    // calls (code 01 of member rows) summed into 2-bit fields.
-    auto index = [&](uint32_t g, uint32_t (&ix)[4], uint32_t ma, uint32_t mb,
-                     uint32_t mc) -> uint32_t {
+    // Row words of group g -> four index words and the rows' missing calls
+    // (code 01, at the low bit of each field).
+    auto index = [&](uint32_t g, uint32_t (&ix)[4], uint32_t (&m)[3]) {
       const uint32_t xa = *reinterpret_cast<const uint32_t*>(tbase + (3 * g + 0) * kPlainBoxBytes);
       const uint32_t xb = *reinterpret_cast<const uint32_t*>(tbase + (3 * g + 1) * kPlainBoxBytes);
       const uint32_t xc = *reinterpret_cast<const uint32_t*>(tbase + (3 * g + 2) * kPlainBoxBytes);
@@ -361,58 +404,99 @@ __global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TIL
       ix[1] = ((O * c_mul[1]) & 0x3C3C3C3Cu) | ((xs * c_mul[2]) & 0xC0C0C0C0u);
       ix[2] = ((E >> 2) & 0x3C3C3C3Cu) | ((xs * c_mul[1]) & 0xC0C0C0C0u);
       ix[3] = ((O >> 2) & 0x3C3C3C3Cu) | (xs & 0xC0C0C0C0u);
-      return (xa & ~(xa >> 1) & ma) + (xb & ~(xb >> 1) & mb) + (xc & ~(xc >> 1) & mc);
+      m[0] = xa & ~(xa >> 1) & 0x55555555u;
+      m[1] = xb & ~(xb >> 1) & 0x55555555u;
+      m[2] = xc & ~(xc >> 1) & 0x55555555u;
     };
     // Groups g and g + 1 together: each person's two lookups go into its
-    // stage sum with one three-input add.  Nibble counters take four groups
-    // (<= 12 calls) before they are flushed to the byte counters.
-    auto pair = [&](uint32_t g, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3,
-                    uint32_t m4, uint32_t m5) {
-      uint32_t i0[4], i1[4];
-      const uint32_t c0 = index(g, i0, m0, m1, m2);
-      const uint32_t c1 = index(g + 1, i1, m3, m4, m5);
+    // stage sum with one three-input add.
+    auto lookups = [&](uint32_t g, const uint32_t (&i0)[4], const uint32_t (&i1)[4]) {
       const uint32_t l0 = lbase + g * 256, l1 = l0 + 256;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          iacc[4 * j + q] = int32_t(uint32_t(iacc[4 * j + q]) +
-                                    uint32_t(lds_s32(__dp4a(i0[q], c_sel[j], l0))) +
-                                    uint32_t(lds_s32(__dp4a(i1[q], c_sel[j], l1))));
-      }
-      ev = (c0 & 0x33333333u) + (c1 & 0x33333333u) + ev;
-      od = ((c0 >> 2) & 0x33333333u) + ((c1 >> 2) & 0x33333333u) + od;
-      if ((g / 2) % 2 == 1 || g + 2 == kPlainGroups) {
-        by[0] += ev & 0x0F0F0F0Fu;
-        by[2] += (ev >> 4) & 0x0F0F0F0Fu;
-        by[1] += od & 0x0F0F0F0Fu;
-        by[3] += (od >> 4) & 0x0F0F0F0Fu;
-        ev = 0u;
-        od = 0u;
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t a0 = __dp4a(i0[q], c_sel[j], l0), a1 = __dp4a(i1[q], c_sel[j], l1);
+          auto add = [&](int32_t& t, int32_t u, int32_t v) {
+            t = int32_t(uint32_t(t) + uint32_t(u) + uint32_t(v));
+          };
+          add(iacc[0][4 * j + q], lds_s32<0>(a0), lds_s32<0>(a1));
+          if (NS > 1) add(iacc[NS > 1 ? 1 : 0][4 * j + q], lds_s32<L::kTabOne>(a0),
+                          lds_s32<L::kTabOne>(a1));
+          if (NS > 2) add(iacc[NS > 2 ? 2 : 0][4 * j + q], lds_s32<2 * L::kTabOne>(a0),
+                          lds_s32<2 * L::kTabOne>(a1));
+        }
       }
     };
-    if (!warp_active) {
-      // padding-only warp: nothing to score
-    } else if (members == (uint64_t(1) << kPlainRows) - 1) {
-      // every row of the stage is a member of this score (the common case)
-#pragma unroll
-      for (uint32_t g = 0; g < kPlainGroups; g += 2)
-        pair(g, 0x55555555u, 0x55555555u, 0x55555555u, 0x55555555u, 0x55555555u, 0x55555555u);
-    } else {
+    // nibble counters (people 2j / 2j + 1) -> byte counters
+    auto widen = [&](uint32_t (&to)[4], uint32_t ev, uint32_t od) {
+      to[0] += ev & 0x0F0F0F0Fu;
+      to[2] += (ev >> 4) & 0x0F0F0F0Fu;
+      to[1] += od & 0x0F0F0F0Fu;
+      to[3] += (od >> 4) & 0x0F0F0F0Fu;
+    };
+    constexpr uint32_t kAll = (1u << kPlainRows) - 1;
+    if (every == kAll) {
+      // every row of the stage is a member of every score (the common case):
+      // missing calls of a group add into 2-bit fields, of four groups into
+      // nibbles (<= 12)
+      uint32_t ev = 0, od = 0;
 #pragma unroll
       for (uint32_t g = 0; g < kPlainGroups; g += 2) {
-        uint32_t m[6];
+        uint32_t i0[4], i1[4], m0[3], m1[3];
+        index(g, i0, m0);
+        index(g + 1, i1, m1);
+        lookups(g, i0, i1);
+        const uint32_t c0 = m0[0] + m0[1] + m0[2], c1 = m1[0] + m1[1] + m1[2];
+        ev = (c0 & 0x33333333u) + (c1 & 0x33333333u) + ev;
+        od = ((c0 >> 2) & 0x33333333u) + ((c1 >> 2) & 0x33333333u) + od;
+        if ((g / 2) % 2 == 1 || g + 2 == kPlainGroups) {
+          widen(all, ev, od);
+          ev = 0u;
+          od = 0u;
+        }
+      }
+    } else {
+      // scores with different members (some may have none).  A row's calls are
+      // split into nibbles once for all scores, and a score adds them times its
+      // 0 / 1 membership word of the row: multiply-adds, on the FMA pipe.
+#pragma unroll 1
+      for (uint32_t g = 0; g < kPlainGroups; g += 2) {
+        uint32_t i0[4], i1[4], m[6];
+        {
+          uint32_t m0[3], m1[3];
+          index(g, i0, m0);
+          index(g + 1, i1, m1);
 #pragma unroll
-        for (uint32_t r = 0; r < 6; ++r)
-          m[r] = (0u - uint32_t((members >> (3 * g + r)) & 1u)) & 0x55555555u;
-        pair(g, m[0], m[1], m[2], m[3], m[4], m[5]);
+          for (int r = 0; r < 3; ++r) {
+            m[r] = m0[r];
+            m[3 + r] = m1[r];
+          }
+        }
+        lookups(g, i0, i1);
+        if (some == 0u) continue;   // no score counts (projection tables)
+        uint32_t ev[NS], od[NS];
+#pragma unroll
+        for (uint32_t s = 0; s < NS; ++s) ev[s] = od[s] = 0u;
+#pragma unroll
+        for (uint32_t r = 0; r < 6; r += 2) {
+#pragma unroll
+          for (uint32_t s = 0; s < NS; ++s) {
+            const uint2 b = *reinterpret_cast<const uint2*>(tab + s * L::kTabOne + kPlainRowsOff +
+                                                            4 * (3 * g + r));
+            ev[s] += (m[r] & 0x11111111u) * b.x + (m[r + 1] & 0x11111111u) * b.y;
+            od[s] += ((m[r] >> 2) & 0x11111111u) * b.x + ((m[r + 1] >> 2) & 0x11111111u) * b.y;
+          }
+        }
+#pragma unroll
+        for (uint32_t s = 0; s < NS; ++s) widen(by[s], ev[s], od[s]);
       }
     }
 
     // Release the buffer.  __syncwarp orders this warp's reads before lane
     // 0's release-add; the warp that completes the count acquires every
     // warp's release, so all reads of the buffer are done before it hands the
-    // buffer to the async proxy for the stage three ahead.
+    // buffer to the async proxy for its next stage.
     __syncwarp();
     if (WS) {
       if (lane == 0) mbar_arrive(empty0 + 8 * buf);
@@ -424,81 +508,128 @@ __global__ void __launch_bounds__(PlainShape<TILE, WS>::kThreads, PlainShape<TIL
         if (nxt < nstages) {
           last_issued[buf] = nxt;
           fence_proxy_async_smem();
-          plain_issue_stage<TILE>(&map, a.tables, sbase, buf, tile_x,
-                                  int32_t(r_begin + uint64_t(nxt) * kPlainRows), stage0 + nxt,
-                                  boxes);
+          plain_issue_stage<TILE, NS>(&map, a, sbase, buf, tile_x,
+                                      int32_t(r_begin + uint64_t(nxt) * kPlainRows), stage0 + nxt,
+                                      boxes);
         }
       }
     }
+    __syncwarp();
 
-    // The stage's exact integer sums go to FP64 with the stage's grid step;
-    // byte counters span eight stages (<= 240 calls per byte) before they
-    // are flushed to 32-bit counts.
-    {
-      const double q = double(stage_q);
+    // The stage's exact integer sums go to the FP64 sums with the stage's grid
+    // step, eight people at a time.
+    if (st > 0) tmem_st_wait();
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        acc64[i] = fma(double(iacc[i]), q, acc64[i]);
-        iacc[i] = 0;
-      }
-      if ((st & 7u) == 7u || st + 1 == nstages) {
+    for (uint32_t s = 0; s < NS; ++s) {
+      const double q = double(stage_q[s]);
 #pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) {
+      for (uint32_t h = 0; h < 2; ++h) {
+        uint32_t d[16];
+        if (st > 0) {
+          tmem_ld16(sums + 32 * s + 16 * h, d);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) cnt[4 * j + q4] += (by[q4] >> (8 * j)) & 0xFFu;
-          by[q4] = 0u;
+          for (int i = 0; i < 16; ++i) d[i] = 0u;
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const double t = fma(double(iacc[s][8 * h + i]), q,
+                               __hiloint2double(int(d[2 * i + 1]), int(d[2 * i])));
+          d[2 * i] = uint32_t(__double2loint(t));
+          d[2 * i + 1] = uint32_t(__double2hiint(t));
+          iacc[s][8 * h + i] = 0;
+        }
+        tmem_st16(sums + 32 * s + 16 * h, d);
       }
+    }
+    // Byte counters span eight stages (<= 240 calls per byte) before they go to
+    // the partials (the first launch since a reset writes them at its first
+    // flush).
+    if ((st & 7u) == 7u || st + 1 == nstages) {
+      const bool write = a.store && st < 8u;
+#pragma unroll
+      for (uint32_t s = 0; s < NS; ++s) {
+        uint4* pc = reinterpret_cast<uint4*>(a.part_cnt + s * a.score_stride + slot0);
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+          uint4 c = write ? make_uint4(0u, 0u, 0u, 0u) : pc[j];
+          c.x += ((by[s][0] + all[0]) >> (8 * j)) & 0xFFu;
+          c.y += ((by[s][1] + all[1]) >> (8 * j)) & 0xFFu;
+          c.z += ((by[s][2] + all[2]) >> (8 * j)) & 0xFFu;
+          c.w += ((by[s][3] + all[3]) >> (8 * j)) & 0xFFu;
+          pc[j] = c;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) by[s][q] = 0u;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) all[q] = 0u;
     }
   }
 
   // A warp that gave up on a TMA wait leaves stages other warps may still
   // wait for (bounded).  Once every warp is here, drain each buffer's last
   // issued copy (bounded) so no TMA is in flight when the CTA exits.
-  if (__syncthreads_or(failed)) {
-    if (!WS && tid == 0) {   // (WS: the producer warp drains)
-      for (uint32_t b = 0; b < L::kStages; ++b)
-        if (last_issued[b] != 0xFFFFFFFFu)
-          mbar_wait_bounded(bar0 + 8 * b, (last_issued[b] / L::kStages) & 1u);
-    }
-    return;
+  const bool any_failed = __syncthreads_or(failed);
+  if (any_failed && !WS && tid == 0) {   // (WS: the producer warp drains)
+    for (uint32_t b = 0; b < L::kStages; ++b)
+      if (last_issued[b] != 0xFFFFFFFFu)
+        mbar_wait_bounded(bar0 + 8 * b, (last_issued[b] / L::kStages) & 1u);
   }
 
   // FP64 partials for this (split, person) accumulate across calls; the first
   // launch after a reset writes them (every split of every tile has a CTA, so
   // every slot it covers is written).  Warps that only held padding added
   // nothing: their slots (people past the row) stay as they are.
-  if (!warp_active) return;
-  const uint64_t person0 = uint64_t(tile) * (TILE * 4) + uint64_t(tid) * 16;
-  double* ps = a.part_sum + uint64_t(split) * a.part_stride + person0;
-  uint32_t* pc = a.part_cnt + uint64_t(split) * a.part_stride + person0;
-  if (a.store) {
+  if (warp_active && !any_failed) {
+    tmem_st_wait();
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      ps[i] = acc64[i];
-      pc[i] = cnt[i];
-    }
-  } else {
+    for (uint32_t s = 0; s < NS; ++s) {
+      double2* ps = reinterpret_cast<double2*>(a.part_sum + s * a.score_stride + slot0);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      ps[i] += acc64[i];
-      pc[i] += cnt[i];
+      for (uint32_t h = 0; h < 2; ++h) {
+        uint32_t d[16];
+        tmem_ld16(sums + 32 * s + 16 * h, d);
+        tmem_ld_wait();
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+          double2 v = make_double2(__hiloint2double(int(d[4 * i + 1]), int(d[4 * i])),
+                                   __hiloint2double(int(d[4 * i + 3]), int(d[4 * i + 2])));
+          if (!a.store) {
+            const double2 o = ps[4 * h + i];
+            v.x += o.x;
+            v.y += o.y;
+          }
+          ps[4 * h + i] = v;
+        }
+      }
     }
+  }
+  tc_fence_before();
+  named_barrier(1, L::kThreads);   // the scoring warps: nobody reads tensor memory any more
+  if (tid < 32) {
+    tc_fence_after();
+    tmem_dealloc(tmem, L::kTmemCols);
   }
 }
 
 // out[o*K + k] = init + sum over splits of part[s][fam(o)], init = baseline[k]
-// (fresh run).  One launch per score column k.  A CTA takes 32 people; warp g
-// sums splits g, g + 8, g + 16, ... of each (a lane per person, so every
-// load is 32 consecutive people of one split) into eight independent
+// (fresh run), for score columns k = a.k + blockIdx.y.  A CTA takes 32 people;
+// warp g of W sums splits g, g + W, g + 2W, ... of each (a lane per person, so
+// every load is 32 consecutive people of one split) into eight independent
 // accumulators, so eight loads are in flight per thread; the accumulators,
-// then the eight warps' sums (lane o of warp 0, g = 0..7), are added in a
-// fixed order, so results are deterministic.
-constexpr uint32_t kFinWarps = 8;
+// then the warps' sums (lane o of warp 0, g = 0..W-1), are added in a fixed
+// order, so results are deterministic.  W = 32 for small cohorts: with few CTAs
+// the time is the longest chain of loads, and 148 splits are one round.
 constexpr uint32_t kFinLanes = 8;   // independent accumulators per thread
+template <uint32_t kFinWarps>
 __global__ void __launch_bounds__(32 * kFinWarps) gnm_finalize(FinalizeArgs a) {
   __shared__ double s_sum[kFinWarps][32];
   __shared__ uint32_t s_cnt[kFinWarps][32];
+  a.k += blockIdx.y;
+  a.part_sum += blockIdx.y * a.score_stride;
+  a.part_cnt += blockIdx.y * a.score_stride;
   const uint32_t lane = threadIdx.x & 31u, g = threadIdx.x >> 5;
   const uint64_t o = uint64_t(blockIdx.x) * 32 + lane;
   double s = 0.0;
@@ -641,45 +772,59 @@ cudaError_t launch_plain_tables(const TableArgs& a, cudaStream_t s) {
   const uint64_t stages = (a.num_rows + kPlainRows - 1) / kPlainRows;
   if (stages == 0) return cudaSuccess;
   if (stages > 0x7FFFFFFFull) return cudaErrorInvalidValue;
-  gnm_plain_tables<<<uint32_t(stages), kPlainGroups * 64, 0, s>>>(a);
+  gnm_plain_tables<<<dim3(uint32_t(stages), a.scores), kPlainGroups * 64, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+template <uint32_t TILE, bool WS, uint32_t NS>
+static cudaError_t launch_plain_pass(const CUtensorMap& map, const PlainArgs& a, uint32_t grid,
+                                     cudaStream_t s) {
+  using L = PlainSmem<TILE, NS>;
+  const cudaError_t e = raise_smem_limit(
+      reinterpret_cast<const void*>(gnm_plain_accumulate<TILE, WS, NS>), int(L::kTotal));
+  if (e != cudaSuccess) return e;
+  gnm_plain_accumulate<TILE, WS, NS>
+      <<<grid, PlainShape<TILE, WS, NS>::kThreads, L::kTotal, s>>>(map, a);
   return cudaGetLastError();
 }
 
 template <uint32_t TILE, bool WS>
-static cudaError_t launch_plain_tile(const CUtensorMap& map, const PlainArgs& a, uint32_t grid,
-                                     cudaStream_t s) {
-  using L = PlainSmem<TILE>;
-  const cudaError_t e = raise_smem_limit(
-      reinterpret_cast<const void*>(gnm_plain_accumulate<TILE, WS>), int(L::kTotal));
-  if (e != cudaSuccess) return e;
-  gnm_plain_accumulate<TILE, WS><<<grid, PlainShape<TILE, WS>::kThreads, L::kTotal, s>>>(map, a);
-  return cudaGetLastError();
+static cudaError_t launch_plain_tile(const CUtensorMap& map, const PlainArgs& a, uint32_t scores,
+                                     uint32_t grid, cudaStream_t s) {
+  switch (scores) {
+    case 1: return launch_plain_pass<TILE, WS, 1>(map, a, grid, s);
+    case 2: return launch_plain_pass<TILE, WS, 2>(map, a, grid, s);
+    case 3: return launch_plain_pass<TILE, WS, 3>(map, a, grid, s);
+    default: return cudaErrorInvalidValue;
+  }
 }
 
 uint32_t plain_grid(const PlainArgs& a) {
-  const uint64_t stages = (a.num_rows + kPlainRows - 1) / kPlainRows;
-  const uint64_t last = (stages + a.last_stages_per_split - 1) / a.last_stages_per_split;
-  return uint32_t(uint64_t(a.tiles - 1) * a.splits + last);
+  return a.tiles * a.splits;   // every tile has the same split count
 }
 
 cudaError_t launch_plain_accumulate(const CUtensorMap& map, const PlainArgs& a, uint32_t kernel,
-                                    cudaStream_t s) {
-  if (a.tiles == 0 || a.splits == 0 || a.stages_per_split == 0 || a.last_stages_per_split == 0)
+                                    uint32_t scores, cudaStream_t s) {
+  if (a.tiles == 0 || a.splits == 0 || a.stages_per_split == 0)
     return cudaErrorInvalidValue;
   const uint32_t grid = plain_grid(a);
   switch (kernel) {
-    case kPlain512: return launch_plain_tile<512, false>(map, a, grid, s);
-    case kPlain512Ws: return launch_plain_tile<512, true>(map, a, grid, s);
-    case kPlain1024: return launch_plain_tile<1024, false>(map, a, grid, s);
-    case kPlain1024Ws: return launch_plain_tile<1024, true>(map, a, grid, s);
-    case kPlain2048Ws: return launch_plain_tile<2048, true>(map, a, grid, s);
+    case kPlain512: return launch_plain_tile<512, false>(map, a, scores, grid, s);
+    case kPlain512Ws: return launch_plain_tile<512, true>(map, a, scores, grid, s);
+    case kPlain1024: return launch_plain_tile<1024, false>(map, a, scores, grid, s);
+    case kPlain1024Ws: return launch_plain_tile<1024, true>(map, a, scores, grid, s);
+    case kPlain2048Ws: return launch_plain_tile<2048, true>(map, a, scores, grid, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t launch_finalize(const FinalizeArgs& a, cudaStream_t s) {
-  const uint32_t blocks = uint32_t((a.num_people + 31) / 32);
-  gnm_finalize<<<blocks ? blocks : 1, 32 * kFinWarps, 0, s>>>(a);
+  const dim3 grid(uint32_t(a.num_people ? (a.num_people + 31) / 32 : 1), a.scores);
+  // 32 warps per 32 people while two such CTAs per SM hold the whole grid
+  if (uint64_t(grid.x) * grid.y <= 296 && a.num_splits > 8)
+    gnm_finalize<32><<<grid, 1024, 0, s>>>(a);
+  else
+    gnm_finalize<8><<<grid, 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 

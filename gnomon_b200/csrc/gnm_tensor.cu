@@ -1603,7 +1603,7 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
     const uint64_t valid = *reinterpret_cast<volatile uint32_t*>(a.state);
     for (uint64_t u = u0; u < u1; ++u, ++n) {
       const uint32_t s = n % ST, ph = (n / ST) & 1u;
-      if (!mbar_wait_bounded(full(s), ph)) {
+      if (!mbar_wait_warp(full(s), ph)) {
         give_up(kErrTmaTimeout);
         break;
       }
@@ -1640,7 +1640,7 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
         // arithmetic below it)
 #pragma unroll
         for (uint32_t i = 0; i < 16; ++i) asm volatile("" : "+r"(lo[i]), "+r"(hi[i]));
-        if (!mbar_wait_bounded(sfree(slot, pairm), sph ^ 1u)) {
+        if (!mbar_wait_warp(sfree(slot, pairm), sph ^ 1u)) {
           give_up(kErrMmaTimeout);
           ok = false;
           break;
@@ -1670,7 +1670,7 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
       if (tile_end || inblk == kT8NrFlush || u + 1 == u1) {
         // ---- epilogue: drain one 128-person block of the tile ----
         inblk = 0;
-        if (!mbar_wait_bounded(accfull, blk & 1u)) {
+        if (!mbar_wait_warp(accfull, blk & 1u)) {
           give_up(kErrMmaTimeout);
           break;
         }
@@ -2484,7 +2484,7 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
     for (uint32_t k = 0; k < kBwScores; ++k) acc[k] = 0.0;
     for (uint64_t u = u0; u < u1; ++u, ++n) {
       const uint32_t s = n % ST, ph = (n / ST) & 1u;
-      if (!mbar_wait_bounded(full(s), ph)) {
+      if (!mbar_wait_warp(full(s), ph)) {
         give_up(kErrTmaTimeout);
         break;
       }
@@ -2519,7 +2519,7 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
         for (uint32_t i = 0; i < (CORR ? 32u : 16u); ++i) asm volatile("" : "+r"(v[i]));
         // a stage is two turns of the ring, so slots and phases are constants
         const uint32_t op = op0 + (2 * (j % 2)) * kBw8SlotCols;
-        if (!mbar_wait_bounded(sfree0 + 16 * (j % 2), (j / 2) ^ 1u)) {
+        if (!mbar_wait_warp(sfree0 + 16 * (j % 2), (j / 2) ^ 1u)) {
           give_up(kErrMmaTimeout);
           ok = false;
           break;
@@ -2544,7 +2544,7 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
       }
       if (tile_end || inblk == kBw8Flush || u + 1 == u1) {
         inblk = 0;
-        if (!mbar_wait_bounded(accfull, blk & 1u)) {
+        if (!mbar_wait_warp(accfull, blk & 1u)) {
           give_up(kErrMmaTimeout);
           break;
         }
