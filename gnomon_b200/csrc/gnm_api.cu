@@ -22,6 +22,7 @@
 #include <exception>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -812,141 +813,203 @@ static bool is_pinned(const void* ptr) {
   return at.type == cudaMemoryTypeHost || at.type == cudaMemoryTypeManaged;
 }
 
-// Device -> host copy of a result array.  Large copies into pageable memory go
-// through a cached pinned ring (two 64 MB chunks): the DMA fills one chunk at
-// the link rate while host threads copy the other out (a direct pageable copy
-// of the batched workload's 0.6 GB of results ran at ~4 GB/s).
+// ---- pinned staging ----------------------------------------------------------
+// Pageable memory reaches the link's rate only through pinned buffers, and
+// pinning costs: two 128 MB buffers took 105 ms to allocate and 30 ms to free, of
+// 149 ms for a whole run over 272 MB of rows.  So pinned memory is kept: 32 MB
+// chunks, each borrowed by one transfer at a time, at most kPinnedKept of them
+// held between calls (gnm_release_cached_memory frees those).
 namespace {
-std::mutex g_ring_mu;
-uint8_t* g_ring[2] = {nullptr, nullptr};
-constexpr uint64_t kRingChunk = uint64_t(64) << 20;
+constexpr uint64_t kPinnedChunk = uint64_t(32) << 20;
+constexpr size_t kPinnedKept = 4;
+std::mutex g_pinned_mu;
+std::vector<uint8_t*> g_pinned;
 }  // namespace
 
-static void release_result_ring() {
-  std::lock_guard<std::mutex> lock(g_ring_mu);
-  for (auto*& r : g_ring) {
-    if (r) cudaFreeHost(r);
-    r = nullptr;
+static void release_pinned() {
+  std::lock_guard<std::mutex> lock(g_pinned_mu);
+  for (auto* p : g_pinned) cudaFreeHost(p);
+  g_pinned.clear();
+}
+
+// One pinned buffer of at least `bytes`; goes back (or is freed) at the end of
+// its scope, when every copy from or to it must have finished.
+struct PinnedBuffer {
+  uint8_t* p = nullptr;
+  bool kept = false;
+  explicit PinnedBuffer(uint64_t bytes) : kept(bytes <= kPinnedChunk) {
+    if (kept) {
+      std::lock_guard<std::mutex> lock(g_pinned_mu);
+      if (!g_pinned.empty()) {
+        p = g_pinned.back();
+        g_pinned.pop_back();
+        return;
+      }
+    }
+    check_cuda(cudaHostAlloc(&p, std::max(bytes, kPinnedChunk), cudaHostAllocDefault),
+               "cudaHostAlloc");
+  }
+  ~PinnedBuffer() {
+    if (kept) {
+      std::lock_guard<std::mutex> lock(g_pinned_mu);
+      if (g_pinned.size() < kPinnedKept) {
+        g_pinned.push_back(p);
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+  PinnedBuffer(const PinnedBuffer&) = delete;
+  PinnedBuffer& operator=(const PinnedBuffer&) = delete;
+};
+
+// Moves `pieces` pieces of at most `piece` bytes through pinned memory: host threads
+// take them in turn, each with two buffers of its own, so that one thread's host
+// work (filling a buffer, or emptying it) runs while others' copies are on the
+// link.  work(i, buf, done) does piece i: for an upload it fills buf and queues its
+// copy; for a download it queues the copy, calls done() to wait for it, and
+// empties buf.  Returns when every copy has finished; the first failure is rethrown.
+template <class W>
+static void staged_pieces(uint64_t pieces, uint64_t piece, cudaStream_t s, W work) {
+  if (pieces == 0) return;
+  const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+  const uint64_t nt = std::min<uint64_t>(hw, pieces);
+  PinnedBuffer pinned(2 * nt * piece);
+  int device = 0;
+  check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+  std::atomic<uint64_t> next{0};
+  std::mutex mu;
+  std::exception_ptr failure;
+  auto run = [&](uint64_t t) {
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+    bool pending[2] = {false, false};
+    try {
+      check_cuda(cudaSetDevice(device), "cudaSetDevice");
+      for (auto& e : ev)
+        check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+      for (uint64_t n = 0;; ++n) {
+        const uint64_t i = next.fetch_add(1);
+        if (i >= pieces) break;
+        const int b = int(n & 1);
+        uint8_t* buf = pinned.p + (2 * t + b) * piece;
+        if (pending[b]) check_cuda(cudaEventSynchronize(ev[b]), "staged copy");
+        pending[b] = false;
+        work(i, buf, [&] {
+          check_cuda(cudaEventRecord(ev[b], s), "event");
+          check_cuda(cudaEventSynchronize(ev[b]), "staged copy");
+        });
+        check_cuda(cudaEventRecord(ev[b], s), "event");
+        pending[b] = true;
+      }
+    } catch (...) {
+      std::lock_guard<std::mutex> lock(mu);
+      if (!failure) failure = std::current_exception();
+      next = pieces;   // the others stop
+    }
+    for (int b = 0; b < 2; ++b) {   // this thread's copies leave its buffers alone
+      if (pending[b]) cudaEventSynchronize(ev[b]);
+      if (ev[b]) cudaEventDestroy(ev[b]);
+    }
+  };
+  if (nt == 1) {
+    run(0);
+  } else {
+    std::vector<std::thread> th;
+    try {
+      for (uint64_t t = 1; t < nt; ++t) th.emplace_back(run, t);
+    } catch (const std::system_error&) {
+      // fewer threads: the ones there are take every piece
+    }
+    run(0);
+    for (auto& x : th) x.join();
+  }
+  if (failure) {
+    cudaStreamSynchronize(s);   // a copy that failed to record may still be queued
+    std::rethrow_exception(failure);
   }
 }
 
+// Pieces of 1 MB up to 32 MB of data in flight; copies below 4 MB go directly.
+constexpr uint64_t kStagedPiece = uint64_t(1) << 20;
+constexpr uint64_t kStagedMin = uint64_t(4) << 20;
+
+// Synchronous device -> host copy of a result array.
 static void copy_to_host(void* dst, const void* src, uint64_t bytes, cudaStream_t s) {
   if (bytes == 0) return;
-  if (bytes < 2 * kRingChunk || is_pinned(dst)) {
+  if (bytes < kStagedMin || is_pinned(dst)) {
     check_cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s), "D2H results");
     check_cuda(cudaStreamSynchronize(s), "D2H results");
     return;
   }
-  std::lock_guard<std::mutex> lock(g_ring_mu);
-  for (auto*& r : g_ring)
-    if (!r) check_cuda(cudaHostAlloc(&r, kRingChunk, cudaHostAllocDefault), "cudaHostAlloc");
-  cudaEvent_t landed[2] = {nullptr, nullptr};
-  struct Ev {
-    cudaEvent_t* e;
-    ~Ev() {
-      for (int i = 0; i < 2; ++i)
-        if (e[i]) cudaEventDestroy(e[i]);
-    }
-  } ev{landed};
-  for (auto& e : landed) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-  const uint64_t n = (bytes + kRingChunk - 1) / kRingChunk;
-  auto issue = [&](uint64_t i) {
-    const uint64_t off = i * kRingChunk, len = std::min(kRingChunk, bytes - off);
-    check_cuda(cudaMemcpyAsync(g_ring[i % 2], static_cast<const uint8_t*>(src) + off, len,
-                               cudaMemcpyDeviceToHost, s),
-               "D2H results");
-    check_cuda(cudaEventRecord(landed[i % 2], s), "event");
-  };
-  issue(0);
-  for (uint64_t i = 0; i < n; ++i) {
-    check_cuda(cudaEventSynchronize(landed[i % 2]), "D2H results");
-    if (i + 1 < n) issue(i + 1);   // the other chunk was copied out last iteration
-    const uint64_t off = i * kRingChunk, len = std::min(kRingChunk, bytes - off);
-    const uint8_t* from = g_ring[i % 2];
-    uint8_t* to = static_cast<uint8_t*>(dst) + off;
-    parallel_chunks(len, uint64_t(4) << 20, [&](uint64_t b, uint64_t e, uint64_t) {
-      std::memcpy(to + b, from + b, e - b);
-    });
-  }
+  staged_pieces((bytes + kStagedPiece - 1) / kStagedPiece, kStagedPiece, s,
+                [&](uint64_t i, uint8_t* buf, auto done) {
+                  const uint64_t off = i * kStagedPiece;
+                  const uint64_t len = std::min(kStagedPiece, bytes - off);
+                  check_cuda(cudaMemcpyAsync(buf, static_cast<const uint8_t*>(src) + off, len,
+                                             cudaMemcpyDeviceToHost, s),
+                             "D2H results");
+                  done();
+                  std::memcpy(static_cast<uint8_t*>(dst) + off, buf, len);
+                });
 }
 
-// Host -> device copy of a large pageable array (the tensor plan's CSR)
-// through the same pinned ring: host threads fill one chunk while the DMA
-// sends the other (a direct pageable copy of the batched workload's 1.6 GB
-// CSR ran at ~10 GB/s).
+// Synchronous host -> device copy.
 void copy_to_device(void* dst, const void* src, uint64_t bytes, cudaStream_t s) {
   if (bytes == 0) return;
-  if (bytes < 2 * kRingChunk || is_pinned(src)) {
+  if (bytes < kStagedMin || is_pinned(src)) {
     check_cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "H2D upload");
     check_cuda(cudaStreamSynchronize(s), "H2D upload");
     return;
   }
-  std::lock_guard<std::mutex> lock(g_ring_mu);
-  for (auto*& r : g_ring)
-    if (!r) check_cuda(cudaHostAlloc(&r, kRingChunk, cudaHostAllocDefault), "cudaHostAlloc");
-  cudaEvent_t sent[2] = {nullptr, nullptr};
-  struct Ev {
-    cudaEvent_t* e;
-    ~Ev() {
-      for (int i = 0; i < 2; ++i)
-        if (e[i]) cudaEventDestroy(e[i]);
-    }
-  } ev{sent};
-  for (auto& e : sent) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-  const uint64_t n = (bytes + kRingChunk - 1) / kRingChunk;
-  for (uint64_t i = 0; i < n; ++i) {
-    const int slot = int(i % 2);
-    if (i >= 2) check_cuda(cudaEventSynchronize(sent[slot]), "H2D upload");
-    const uint64_t off = i * kRingChunk, len = std::min(kRingChunk, bytes - off);
-    const uint8_t* from = static_cast<const uint8_t*>(src) + off;
-    uint8_t* to = g_ring[slot];
-    parallel_chunks(len, uint64_t(4) << 20, [&](uint64_t b, uint64_t e, uint64_t) {
-      std::memcpy(to + b, from + b, e - b);
-    });
-    check_cuda(cudaMemcpyAsync(static_cast<uint8_t*>(dst) + off, to, len, cudaMemcpyHostToDevice, s),
-               "H2D upload");
-    check_cuda(cudaEventRecord(sent[slot], s), "event");
-  }
-  check_cuda(cudaStreamSynchronize(s), "H2D upload");
+  staged_pieces((bytes + kStagedPiece - 1) / kStagedPiece, kStagedPiece, s,
+                [&](uint64_t i, uint8_t* buf, auto) {
+                  const uint64_t off = i * kStagedPiece;
+                  const uint64_t len = std::min(kStagedPiece, bytes - off);
+                  std::memcpy(buf, static_cast<const uint8_t*>(src) + off, len);
+                  check_cuda(cudaMemcpyAsync(static_cast<uint8_t*>(dst) + off, buf, len,
+                                             cudaMemcpyHostToDevice, s),
+                             "H2D upload");
+                });
 }
 
-// Copy rows [v0, v0+n) into dst (pitch layout); zero the padding.
-static void gather_rows(const HostRun& r, uint64_t v0, uint64_t n, uint8_t* dst) {
+// Rows [v0, v0 + n) into dst (pitch layout), padding zeroed: 0, 1 if a row lies past
+// the end of the data, 2 if the callback failed.
+static int gather_rows(const HostRun& r, uint64_t v0, uint64_t n, uint8_t* dst) {
   const uint64_t bpv = r.bpv;
   const uint64_t* map = r.prep->required_bim_indices;
-  const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  const unsigned nt = unsigned(std::min<uint64_t>(hw, std::max<uint64_t>(1, n / 256)));
-  std::atomic<int> bad{0};
-  auto work = [&](unsigned t) {
-    for (uint64_t i = t; i < n; i += nt) {
-      uint8_t* d = dst + i * r.pitch;
-      if (v0 + i < r.zero_before) {  // already folded into the resume state
-        std::memset(d, 0, r.pitch);
-        continue;
-      }
-      const uint64_t row = map ? map[v0 + i] : v0 + i;
-      if (r.bed->data) {
-        if ((row + 1) * bpv > r.bed->data_len) {
-          bad = 1;
-          return;
-        }
-        std::memcpy(d, r.bed->data + row * bpv, bpv);
-      } else if (r.bed->read_at(r.bed->user_ctx, row * bpv, d, bpv) != 0) {
-        bad = 2;
-        return;
-      }
-      std::memset(d + bpv, 0, r.pitch - bpv);
+  for (uint64_t i = 0; i < n; ++i) {
+    uint8_t* d = dst + i * r.pitch;
+    if (v0 + i < r.zero_before) {  // already folded into the resume state
+      std::memset(d, 0, r.pitch);
+      continue;
     }
-  };
-  if (nt == 1) {
-    work(0);
-  } else {
-    std::vector<std::thread> th;
-    for (unsigned t = 0; t < nt; ++t) th.emplace_back(work, t);
-    for (auto& x : th) x.join();
+    const uint64_t row = map ? map[v0 + i] : v0 + i;
+    if (r.bed->data) {
+      if ((row + 1) * bpv > r.bed->data_len) return 1;
+      std::memcpy(d, r.bed->data + row * bpv, bpv);
+    } else if (r.bed->read_at(r.bed->user_ctx, row * bpv, d, bpv) != 0) {
+      return 2;
+    }
+    std::memset(d + bpv, 0, r.pitch - bpv);
   }
-  if (bad == 1) fail(GNM_ERR_IO, "truncated .bed: a required row lies past the end of the data");
-  if (bad == 2) fail(GNM_ERR_PRODUCER, "read_at callback failed");
+  return 0;
+}
+
+// Rows [v0, v0 + n) into device memory d_rows through pinned buffers.
+static void upload_rows(const HostRun& r, uint64_t v0, uint64_t n, uint8_t* d_rows,
+                        cudaStream_t s) {
+  const uint64_t per =   // rows per piece
+      std::max<uint64_t>(1, kStagedPiece / std::max<uint64_t>(1, r.pitch));
+  staged_pieces((n + per - 1) / per, per * r.pitch, s, [&](uint64_t i, uint8_t* buf, auto) {
+    const uint64_t c0 = i * per, nc = std::min(per, n - c0);
+    const int bad = gather_rows(r, v0 + c0, nc, buf);
+    if (bad == 1)
+      fail(GNM_ERR_IO, "truncated .bed: a required row lies past the end of the data");
+    if (bad == 2) fail(GNM_ERR_PRODUCER, "read_at callback failed");
+    check_cuda(cudaMemcpyAsync(d_rows + c0 * r.pitch, buf, nc * r.pitch, cudaMemcpyHostToDevice,
+                               s),
+               "H2D rows");
+  });
 }
 
 // Streams and pool buffers of one host run.  Whatever way the run ends, the
@@ -1062,37 +1125,24 @@ static void host_run_impl(const gnm_prep_view* prep, const gnm_bed_view* bed,
   if (repitch)
     for (int i = 0; i < 2; ++i) staging[i] = res.alloc<uint8_t>(rpc * bpv, "staging");
   const uint64_t chunk = std::max<uint64_t>(1, std::min<uint64_t>(block, (uint64_t(128) << 20) / pitch));
-  uint8_t* pinned[2] = {nullptr, nullptr};
-  struct Pinned {
-    uint8_t** p;
-    ~Pinned() {
-      cudaFreeHost(p[0]);
-      cudaFreeHost(p[1]);
-    }
-  } pin_owner{pinned};
-  if (!direct)
-    for (int i = 0; i < 2; ++i)
-      check_cuda(cudaHostAlloc(&pinned[i], chunk * pitch, cudaHostAllocDefault), "cudaHostAlloc");
   check_cuda(cudaStreamSynchronize(cs), "pool allocations");
 
-  // copied: block rows are in dbuf; consumed: compute done with dbuf;
-  // staged: host staging buffer free; landed / repitched: device staging
-  // buffer filled / drained
-  cudaEvent_t copied[2], consumed[2], staged[2], landed[2], repitched[2];
+  // copied: block rows are in dbuf; consumed: compute done with dbuf; landed /
+  // repitched: device staging buffer filled / drained
+  cudaEvent_t copied[2], consumed[2], landed[2], repitched[2];
   struct Events {
-    cudaEvent_t* e[5];
+    cudaEvent_t* e[4];
     ~Events() {
       for (auto* a : e)
         for (int i = 0; i < 2; ++i)
           if (a[i]) cudaEventDestroy(a[i]);
     }
-  } ev_owner{{copied, consumed, staged, landed, repitched}};
+  } ev_owner{{copied, consumed, landed, repitched}};
   for (auto* a : ev_owner.e) a[0] = a[1] = nullptr;
   for (int i = 0; i < 2; ++i) {
     for (auto* a : ev_owner.e)
       check_cuda(cudaEventCreateWithFlags(&a[i], cudaEventDisableTiming), "event");
     check_cuda(cudaEventRecord(consumed[i], cs), "event");
-    check_cuda(cudaEventRecord(staged[i], xs), "event");
     check_cuda(cudaEventRecord(landed[i], xs), "event");
     check_cuda(cudaEventRecord(repitched[i], rs), "event");
   }
@@ -1132,16 +1182,7 @@ static void host_run_impl(const gnm_prep_view* prep, const gnm_bed_view* bed,
       check_cuda(cudaEventRecord(copied[slot], repitch ? rs : xs), "event");
     } else {
       check_cuda(cudaStreamWaitEvent(xs, consumed[slot], 0), "wait");
-      for (uint64_t c0 = 0; c0 < nb; c0 += chunk, ++stage_idx) {
-        const uint64_t nc = std::min(chunk, nb - c0);
-        const int ps = int(stage_idx & 1);
-        check_cuda(cudaEventSynchronize(staged[ps]), "wait pinned buffer");
-        gather_rows(r, b0 + c0, nc, pinned[ps]);
-        check_cuda(cudaMemcpyAsync(dbuf[slot] + c0 * pitch, pinned[ps], nc * pitch,
-                                   cudaMemcpyHostToDevice, xs),
-                   "H2D rows");
-        check_cuda(cudaEventRecord(staged[ps], xs), "event");
-      }
+      upload_rows(r, b0, nb, dbuf[slot], xs);
       check_cuda(cudaEventRecord(copied[slot], xs), "event");
     }
   };
@@ -1407,11 +1448,18 @@ static void project_block_impl(gnm_projector* pj, const uint8_t* packed, uint64_
   plan_reset_impl(plan.get(), b.s);
   accumulate_impl(plan.get(), rows, pitch, 0, filled, b.s);
   finalize_impl(plan.get(), d_sums, d_counts, true, b.s);
-  std::vector<double> s(pj->n * pj->K);
-  check_cuda(cudaMemcpyAsync(s.data(), d_sums, s.size() * 8, cudaMemcpyDeviceToHost, b.s), "sums");
   sync_impl(plan.get(), b.s);
   trace.mark("project: accumulate");
-  for (uint64_t i = 0; i < s.size(); ++i) pj->acc[i] += s[i];
+  // the sums come back piece by piece and are added as they land
+  const uint64_t n = pj->n * pj->K, per = kStagedPiece / sizeof(double);
+  double* acc = pj->acc.data();
+  staged_pieces((n + per - 1) / per, kStagedPiece, b.s, [&](uint64_t i, uint8_t* buf, auto done) {
+    const uint64_t c0 = i * per, nc = std::min(per, n - c0);
+    check_cuda(cudaMemcpyAsync(buf, d_sums + c0, nc * 8, cudaMemcpyDeviceToHost, b.s), "sums");
+    done();
+    const double* from = reinterpret_cast<const double*>(buf);
+    for (uint64_t x = 0; x < nc; ++x) acc[c0 + x] += from[x];
+  });
   trace.mark("project: add");
 }
 
@@ -1708,7 +1756,7 @@ gnm_status gnm_release_cached_memory(int device, gnm_error* err) {
     device = resolve_device(device);
     DeviceGuard g(device);
     check_cuda(cudaMemPoolTrimTo(run_pool(device), 0), "cudaMemPoolTrimTo");
-    release_result_ring();
+    release_pinned();
   });
 }
 
