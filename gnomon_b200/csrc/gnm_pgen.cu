@@ -55,6 +55,9 @@ enum : uint32_t { kPgErrBounds = 1u, kPgErrPair = 2u, kPgErrPatch = 4u };
 
 constexpr uint32_t kNoAnchor = 0xFFFFFFFFu;
 
+constexpr uint64_t kPgSmem = 227 * 1024;      // shared memory of an SM
+constexpr uint64_t kPgRowMax = 200 * 1024;    // rows up to 819,200 samples are patched there
+
 struct PgArgs {
   const uint8_t* pgen;         // whole file
   const uint64_t* offsets;     // [V] record offsets
@@ -69,6 +72,8 @@ struct PgArgs {
   uint8_t* scratch;            // anchor rows outside the output: [extra_rows][spitch]
   uint64_t spitch;
   uint32_t extra_rows;         // scratch rows the direct kernel decodes
+  const uint32_t* direct;      // range mode: its variants that are not LD-compressed (else null)
+  uint32_t ndirect;
   // list mode (null in range mode): the variant of output row i (rows count ..
   // count + extra_rows - 1 are scratch rows) and the row holding its anchor
   const uint32_t* vids;
@@ -490,6 +495,359 @@ __global__ void __launch_bounds__(kPgThreads, 8) gnm_pgen_ld(PgArgs a) {
   __syncwarp();
   warp_difflist(a, r, 0, row, src, v, swap);
   warp_fix_tail(a, row);
+}
+
+// Records decoded with the row in shared memory: one CTA per record, W = blockDim /
+// 32 warps (a power of two) sharing it.  LD: an LD-compressed record (CTAs of
+// others return at once); the anchor row is copied in, type 3 swapping REF and ALT
+// homozygotes on the way.  Otherwise a record of its own: the 2-bit or 1-bit array
+// turned into .bed codes sixteen fields at a time, or a fill.  The difflist
+// patches the shared row, which is written out once, so rows touch L2 once each
+// way.
+//
+// What bounds the global-memory forms (gnm_pgen_direct, gnm_pgen_ld) is instruction
+// issue: a lane walks a difflist group's 64 entries one after the other, 19,300 warp
+// instructions per record of 5,100 entries.  Here a group whose 63 deltas are one
+// byte each (its stored length says so; id gaps below 128) is decoded by eight lanes
+// at once, four groups per step: a lane takes eight entries, their deltas in two
+// 32-bit words and their values in two bytes, an eight-lane scan turns deltas into
+// ids (byte sums by dot product), and each entry xors its field of the shared row
+// (ids differ, so a field is touched once and its old value may be read beside
+// other lanes' xors).  A group with some two-byte deltas (gaps of 128 and more)
+// takes the whole warp: a byte's bits are shifted by seven where the byte before
+// goes on, and one scan gives both the ids and the entries' ranks.  Groups with
+// longer deltas are walked by one lane each.
+//
+// 50,000 samples x 16,384 variants (15,128 LD records): LD kernel 413 -> 227 us.
+template <bool LD>
+__global__ void __launch_bounds__(512) gnm_pgen_row(PgArgs a) {
+  extern __shared__ uint4 s_row[];
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wi = tid >> 5;
+  const uint32_t warp_mask = (blockDim.x >> 5) - 1;
+  uint32_t at_row = blockIdx.x;
+  if (!LD && a.direct)   // the range's records of their own, then the scratch row
+    at_row = blockIdx.x < a.ndirect ? a.direct[blockIdx.x] - a.begin
+                                    : a.count + blockIdx.x - a.ndirect;
+  const uint32_t v = variant_at(a, at_row);
+  const uint32_t anchor = a.anchor_of[v];
+  if ((anchor != kNoAnchor) != LD) return;
+  const Rec r{a.pgen + a.offsets[v], a.lens[v]};
+  const uint32_t kind = a.types[v] & 7u;
+  const bool swap = LD && kind == 3u;
+  uint8_t* row = row_at(a, at_row);
+  const uint32_t bpv = uint32_t((a.n + 3) / 4);   // the host bounds rows to shared memory
+  const uint32_t vecs = bpv / 16, words = bpv / 4;
+  uint8_t* s8 = reinterpret_cast<uint8_t*>(s_row);
+  // the record as aligned words: byte o is byte (o + skew) % 4 of word (o + skew) / 4
+  const uint32_t skew = uint32_t(reinterpret_cast<uintptr_t>(r.p) & 3u);
+  const uint32_t* p32 = reinterpret_cast<const uint32_t*>(r.p - skew);
+  // the `count` (1 to 4) bytes from record offset `off`, in one or two aligned words
+  // (each holds a byte that is asked for); higher bytes of the result are undefined
+  auto load_bytes = [&](uint32_t off, uint32_t count) {
+    const uint32_t o = skew + off;
+    const uint32_t w0 = p32[o >> 2];
+    const uint32_t w1 = ((o + count - 1) >> 2) != (o >> 2) ? p32[(o >> 2) + 1] : 0u;
+    return __funnelshift_r(w0, w1, (o & 3u) * 8u);
+  };
+  // sixteen categories -> .bed codes: 0, 1, 2, 3 -> 11, 10, 00, 01, with the REF / ALT
+  // swap 00, 10, 11, 01
+  auto codes_of = [&](uint32_t c) {
+    const uint32_t hi = (c >> 1) & 0x55555555u, diff = (c ^ (c >> 1)) & 0x55555555u;
+    return swap ? (diff << 1) | hi : ((hi ^ 0x55555555u) << 1) | (diff ^ 0x55555555u);
+  };
+  uint32_t cur = 0;      // where the difflist starts
+  bool difflist = true;
+  if (LD) {
+    const uint32_t ar =
+        a.arow ? a.arow[at_row] : anchor >= a.begin ? anchor - a.begin : a.count;
+    const uint8_t* src = row_at(a, ar);
+    const uint4* s16 = reinterpret_cast<const uint4*>(src);
+    for (uint32_t j = tid; j < vecs; j += 4 * blockDim.x) {   // four loads in flight
+      uint4 q[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (j + k * blockDim.x < vecs) q[k] = s16[j + k * blockDim.x];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (j + k * blockDim.x < vecs) {
+          if (swap) {
+            q[k].x = swap_homs(q[k].x);
+            q[k].y = swap_homs(q[k].y);
+            q[k].z = swap_homs(q[k].z);
+            q[k].w = swap_homs(q[k].w);
+          }
+          s_row[j + k * blockDim.x] = q[k];
+        }
+    }
+    for (uint32_t b = 16 * vecs + tid; b < bpv; b += blockDim.x)
+      s8[b] = uint8_t(swap ? swap_homs(src[b]) : src[b]);
+  } else if (kind == 0) {
+    if (r.len < bpv) {
+      if (tid == 0) flag(a, kPgErrBounds, v);
+      return;
+    }
+    uint32_t* s32 = reinterpret_cast<uint32_t*>(s_row);
+    for (uint32_t j = tid; j < words; j += 4 * blockDim.x) {
+      uint32_t x[4];
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (j + k * blockDim.x < words) x[k] = load_bytes(4 * (j + k * blockDim.x), 4);
+#pragma unroll
+      for (uint32_t k = 0; k < 4; ++k)
+        if (j + k * blockDim.x < words) s32[j + k * blockDim.x] = codes_of(x[k]);
+    }
+    for (uint32_t b = 4 * words + tid; b < bpv; b += blockDim.x) s8[b] = uint8_t(codes_of(r.p[b]));
+    difflist = false;
+  } else if (kind == 1) {
+    // pair code -> (low, high) categories; bit set = high
+    uint32_t pc = 0;
+    const bool okb = r.byte(0, pc);
+    const int low = okb && pc < 16 ? kPairLow[pc] : -1;
+    const int high = okb && pc < 16 ? kPairHigh[pc] : -1;
+    const uint32_t nb = uint32_t((a.n + 7) / 8);
+    if (!okb || low < 0 || r.len < 1 + nb) {
+      if (tid == 0) flag(a, !okb || low < 0 ? kPgErrPair : kPgErrBounds, v);
+      return;
+    }
+    const uint32_t clear = kCatToBed[low], diff = clear ^ kCatToBed[high];
+    // sixteen bits -> sixteen fields: the bits spread to the fields' low bits, times
+    // what the set bit changes
+    auto expand = [&](uint32_t b) {
+      b = (b | (b << 8)) & 0x00FF00FFu;
+      b = (b | (b << 4)) & 0x0F0F0F0Fu;
+      b = (b | (b << 2)) & 0x33333333u;
+      b = (b | (b << 1)) & 0x55555555u;
+      return (clear * 0x55555555u) ^ (b * diff);
+    };
+    uint32_t* s32 = reinterpret_cast<uint32_t*>(s_row);
+    for (uint32_t j = tid; j < words; j += blockDim.x)
+      s32[j] = expand(load_bytes(1 + 2 * j, 2) & 0xFFFFu);
+    for (uint32_t b = 4 * words + tid; b < bpv; b += blockDim.x)
+      s8[b] = uint8_t(expand((uint32_t(r.p[1 + b / 2]) >> (4 * (b % 2))) & 15u));
+    cur = 1 + nb;
+  } else if (kind == 4 || kind == 6 || kind == 7) {
+    const uint32_t w = kCatToBed[kind == 4 ? 0 : kind == 6 ? 2 : 3] * 0x55555555u;
+    for (uint32_t j = tid; j < vecs; j += blockDim.x) s_row[j] = make_uint4(w, w, w, w);
+    for (uint32_t b = 16 * vecs + tid; b < bpv; b += blockDim.x) s8[b] = uint8_t(w);
+  } else {
+    if (tid == 0) flag(a, kPgErrPair, v);
+    return;
+  }
+  __syncthreads();
+
+  uint32_t* row32 = reinterpret_cast<uint32_t*>(s_row);
+  const uint32_t n32 = uint32_t(a.n);
+  // category -> .bed code as a packed 2-bit table, with or without the swap
+  const uint32_t code_of = swap ? 0x78u : 0x4Bu;
+  auto patch = [&](uint32_t id, uint32_t val) {
+    if (id >= n32) return;   // skipped, as the reference skips them
+    const uint32_t sh = 2 * (id & 15u);
+    const uint32_t old = row32[id >> 4] >> sh, code = code_of >> (2 * val);
+    atomicXor(row32 + (id >> 4), ((old ^ code) & 3u) << sh);
+  };
+  uint64_t l = 0;
+  bool bad = difflist && (!r.varint(cur, l) || l > a.n);
+  if (!bad && l > 0) {
+    const uint32_t len = uint32_t(l), groups = (len + 63) / 64;
+    const uint32_t wid = a.n <= (1u << 8) ? 1 : a.n <= (1u << 16) ? 2 : a.n <= (1u << 24) ? 3 : 4;
+    const uint32_t first_at = cur, glen_at = first_at + groups * wid;
+    const uint32_t vals_at = glen_at + groups - 1;
+    uint32_t deltas = vals_at + (len + 3) / 4;   // the first group's deltas
+    const uint8_t* p = r.p;
+    const uint32_t rlen = r.len;
+    bad = deltas > rlen;
+    auto first_id = [&](uint32_t g) {
+      uint32_t id = 0;
+      for (uint32_t k = 0; k < wid; ++k) id |= uint32_t(p[first_at + g * wid + k]) << (8 * k);
+      return id;
+    };
+    // every warp lays out all groups, 32 at a time, and patches every W-th step's
+    uint32_t step = 0;
+    for (uint32_t c0 = 0; !bad && c0 < groups; c0 += 32) {
+      const uint32_t g = c0 + lane;
+      const bool have = g < groups, ends = g + 1 == groups;
+      const uint32_t mine = g + 1 < groups ? uint32_t(p[glen_at + g]) + 63u : 0u;
+      uint32_t incl = mine;
+#pragma unroll
+      for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += y;
+      }
+      const uint32_t at = deltas + incl - mine;
+      deltas += __shfl_sync(0xFFFFFFFFu, incl, 31);
+      const uint32_t count = ends ? len - 64u * (groups - 1) : 64u;
+      const uint32_t fid = have ? first_id(g) : 0u;
+      // 63 one-byte deltas that lie inside the record; ids that cannot wrap
+      const bool quick = have && !ends && mine == 63u && at <= rlen && 63u <= rlen - at &&
+                         fid < 0xFFE00000u;
+      bool mixed = have && !quick && (g & warp_mask) == wi;
+      // every id lies below the next group's first
+      const uint32_t nfid = have && !ends ? first_id(g + 1) : 0xFFFFFFFFu;
+      // four quick groups per step, eight lanes each, eight entries per lane
+      uint32_t todo = __ballot_sync(0xFFFFFFFFu, quick);
+      while (todo) {
+        uint32_t from = 32;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          if (todo && lane / 8 == k) from = __ffs(todo) - 1;
+          todo &= todo - 1;   // (0 stays 0)
+        }
+        if ((step++ & warp_mask) != wi) continue;
+        const uint32_t i = lane & 7u;
+        const bool on = from < 32;
+        const uint32_t gat = __shfl_sync(0xFFFFFFFFu, at, from & 31u);
+        const uint32_t gid = __shfl_sync(0xFFFFFFFFu, fid, from & 31u);
+        const uint32_t gnext = __shfl_sync(0xFFFFFFFFu, nfid, from & 31u);
+        // the deltas of entries 8i .. 8i + 7 (entry 0 has none): eight bytes from
+        // gat + 8i - 1, in two or three aligned words, each with a byte of them
+        uint32_t x0 = 0x01010101u, x1 = 0x01010101u, codes = 0;
+        if (on) {
+          const uint32_t off = skew + gat + 8 * i - 1, sh = (off & 3u) * 8u;
+          const uint32_t* al = p32 + (off >> 2);
+          const uint32_t w0 = al[0], w1 = al[1], w2 = sh ? al[2] : 0u;
+          x0 = __funnelshift_r(w0, w1, sh);
+          x1 = __funnelshift_r(w1, w2, sh);
+          if (i == 0) x0 = (x0 & ~0xFFu) | 1u;
+          const uint8_t* vals = p + vals_at + 16 * (c0 + from) + 2 * i;
+          codes = codes_of(uint32_t(vals[0]) | (uint32_t(vals[1]) << 8));
+        }
+        // a continuation bit or a zero delta
+        bool odd = ((x0 | ((x0 - 0x01010101u) & ~x0) | x1 | ((x1 - 0x01010101u) & ~x1)) &
+                    0x80808080u) != 0u;
+        if (i == 0) x0 &= ~0xFFu;
+        const uint32_t mine8 = __dp4a(x1, 0x01010101u, __dp4a(x0, 0x01010101u, 0u));
+        uint32_t sum = mine8;
+#pragma unroll
+        for (uint32_t d = 1; d < 8; d <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, sum, d, 8);
+          if (i >= d) sum += y;
+        }
+        const uint32_t last = gid + __shfl_sync(0xFFFFFFFFu, sum, 7, 8);
+        odd |= on && last >= gnext;
+        if (on && !odd) {
+          const uint32_t base = gid + sum - mine8;
+          const uint32_t mid = __dp4a(x0, 0x01010101u, base);
+          const uint32_t id[8] = {__dp4a(x0, 0x00000001u, base), __dp4a(x0, 0x00000101u, base),
+                                  __dp4a(x0, 0x00010101u, base), mid,
+                                  __dp4a(x1, 0x00000001u, mid),  __dp4a(x1, 0x00000101u, mid),
+                                  __dp4a(x1, 0x00010101u, mid),  __dp4a(x1, 0x01010101u, mid)};
+#pragma unroll
+          for (uint32_t k = 0; k < 8; ++k)
+            if (id[k] < n32) {   // others are skipped, as the reference skips them
+              const uint32_t sh = 2 * (id[k] & 15u);
+              const uint32_t old = row32[id[k] >> 4] >> sh;
+              atomicXor(row32 + (id[k] >> 4), ((old ^ (codes >> (2 * k))) & 3u) << sh);
+            }
+        }
+        bad |= odd;   // its length says one byte per delta
+      }
+      // groups with some two-byte deltas, in at most 128 bytes (the last group's
+      // length is not stored: it ends with its last entry)
+      const uint32_t room = at <= rlen ? rlen - at : 0u;
+      const uint32_t span = ends ? min(128u, room) : mine;
+      todo = __ballot_sync(0xFFFFFFFFu, mixed && span <= 128u && span <= room && fid < 0xFFE00000u);
+      while (todo) {
+        const uint32_t l0 = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t gat = __shfl_sync(0xFFFFFFFFu, at, l0);
+        const uint32_t gcount = __shfl_sync(0xFFFFFFFFu, count, l0);
+        const uint32_t gid = __shfl_sync(0xFFFFFFFFu, fid, l0);
+        const uint32_t gnext = __shfl_sync(0xFFFFFFFFu, nfid, l0);
+        const uint32_t bytes = __shfl_sync(0xFFFFFFFFu, span, l0);
+        const uint32_t gg = c0 + l0;
+        const bool g_ends = gg + 1 == groups;
+        // lane: bytes 4 lane .. of the group's deltas
+        const uint32_t act = bytes > 4 * lane ? min(4u, bytes - 4 * lane) : 0u;
+        const uint32_t in = act < 4 ? (1u << (8 * act)) - 1u : 0xFFFFFFFFu;
+        const uint32_t x = act ? load_bytes(gat + 4 * lane, act) & in : 0u;
+        const uint32_t cont = x & 0x80808080u;            // a delta goes on
+        const uint32_t end = ~x & 0x80808080u & in;       // a delta ends
+        const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, x >> 31, 1);
+        const uint32_t second = (cont << 8) | (lane ? up << 7 : 0u);   // second byte of a delta
+        const uint32_t zero = (x - 0x01010101u) & ~x & 0x80808080u & in;
+        // three bytes, or a byte of zero bits (a zero or a padded delta): walked below
+        const bool odd = ((cont & second) | zero) != 0u;
+        uint32_t c[4], sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          const uint32_t b = (x >> (8 * k)) & 0x7Fu;
+          sum += ((second >> (8 * k)) & 0x80u) ? b << 7 : b;
+          c[k] = sum;
+        }
+        // one scan for the ids (at most 128 x 16,256) and the entries' ranks
+        uint32_t scan = sum | (uint32_t(__popc(end)) << 24);
+        const uint32_t own = scan;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, scan, d);
+          if (lane >= d) scan += y;
+        }
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, scan, 31);
+        const uint32_t found = total >> 24;
+        const uint32_t tail = __ballot_sync(0xFFFFFFFFu, act && bytes - 4 * lane <= 4 &&
+                                                             ((end >> (8 * act - 1)) & 1u));
+        if (__any_sync(0xFFFFFFFFu, odd && (!g_ends || (scan - own) >> 24 < gcount - 1)) ||
+            (g_ends ? found < gcount - 1 : found != gcount - 1 || !tail))
+          continue;   // left to the walk, which says what is wrong
+        const uint8_t* vals = p + vals_at + 16 * gg;
+        const uint32_t base = gid + ((scan - own) & 0xFFFFFFu);
+        uint32_t e = 1 + ((scan - own) >> 24);
+        if (lane == 0) patch(gid, vals[0] & 3u);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+          if ((end >> (8 * k)) & 0x80u) {
+            if (e < gcount) patch(base + c[k], (vals[e / 4] >> (2 * (e & 3u))) & 3u);
+            ++e;
+          }
+        if (!g_ends && gid + (total & 0xFFFFFFu) >= gnext) bad = true;
+        if (lane == l0) mixed = false;
+      }
+      if (mixed) {   // one lane walks the group
+        const uint8_t* vals = p + vals_at + 16 * g;
+        uint32_t id = fid, pos = at;
+        patch(id, vals[0] & 3u);
+        for (uint32_t e = 1; e < count && !bad; ++e) {
+          // a delta of any length; a read past the record gives 0, which ends the
+          // walk as a zero delta
+          uint32_t d = pos < rlen ? p[pos] : 0u;
+          ++pos;
+          if (d & 0x80u) {
+            uint64_t d64 = d & 0x7Fu;
+            uint32_t b = 0x80u, shift = 7;
+            while (b & 0x80u) {
+              if (pos >= rlen || shift > 56) {
+                bad = true;
+                break;
+              }
+              b = p[pos++];
+              d64 |= uint64_t(b & 0x7Fu) << shift;
+              shift += 7;
+            }
+            d = uint32_t(min(d64, uint64_t(0xFFFFFFFFu)));
+          }
+          if (d == 0) bad = true;
+          if (bad) break;
+          id = id > 0xFFFFFFFFu - d ? 0xFFFFFFFFu : id + d;   // saturates
+          patch(id, (vals[e / 4] >> (2 * (e & 3u))) & 3u);
+        }
+        if (!bad && !ends && (pos != at + mine || id >= nfid)) bad = true;
+      }
+      bad = __any_sync(0xFFFFFFFFu, bad);
+    }
+  }
+  if (bad && lane == 0) flag(a, kPgErrBounds, v);
+  __syncthreads();
+  // padding fields of the last byte -> 01 (missing), as the reference packs them
+  const uint32_t rem = uint32_t(a.n % 4);
+  if (tid == 0 && rem) {
+    uint32_t b = s8[bpv - 1];
+    for (uint32_t k = rem; k < 4; ++k) b = (b & ~(3u << (2 * k))) | (1u << (2 * k));
+    s8[bpv - 1] = uint8_t(b);
+  }
+  __syncthreads();
+  uint4* d16 = reinterpret_cast<uint4*>(row);
+  for (uint32_t j = tid; j < vecs; j += blockDim.x) d16[j] = s_row[j];
+  for (uint32_t b = 16 * vecs + tid; b < bpv; b += blockDim.x) row[b] = s8[b];
 }
 
 
@@ -1131,6 +1489,8 @@ struct gnm_pgen {
   int device = 0;
   uint64_t variants = 0, samples = 0, file_bytes = 0, device_bytes = 0;
   std::vector<uint32_t> anchor_of;   // host copy: which anchors a decode needs
+  std::vector<uint32_t> direct;      // variants that are not LD-compressed, ascending
+  uint32_t* d_direct = nullptr;      // the same on the device
   std::vector<uint32_t> alt_counts;  // host copy (empty: every variant biallelic)
   std::vector<void*> bufs;
   gnm::PgArgs base{};
@@ -1227,6 +1587,10 @@ gnm_pgen* pgen_open_impl(const uint8_t* pgen, uint64_t pgen_len, int device,
   pg->device_bytes += a.spitch;
   a.scratch = pg->scratch;
   a.n = ix.samples;
+  for (uint64_t v = 0; v < m; ++v)
+    if (anchor_of[v] == kNoAnchor) pg->direct.push_back(uint32_t(v));
+  pg->d_direct =
+      static_cast<uint32_t*>(up(pg->direct.data(), pg->direct.size() * 4, ".pgen index"));
   pg->anchor_of = std::move(anchor_of);
   return pg.release();
 }
@@ -1256,9 +1620,26 @@ static void check_rows(const gnm_pgen* pg, const uint8_t* d_rows, uint64_t pitch
 }
 
 static void launch_decode(const PgArgs& a, cudaStream_t s) {
-  gnm_pgen_direct<<<a.count + a.extra_rows, kPgThreads, 0, s>>>(a);
-  check_cuda(cudaGetLastError(), "pgen decode launch");
-  gnm_pgen_ld<<<uint32_t((uint64_t(a.count) + kPgWarps - 1) / kPgWarps), kPgThreads, 0, s>>>(a);
+  const uint64_t row_bytes = ((a.n + 3) / 4 + 15) / 16 * 16;
+  if (row_bytes <= kPgRowMax) {
+    // Rows that fit shared memory.  Records of their own are few: eight warps each.
+    // LD records: enough warps for 32 per SM (50,000 samples, two: 124 us, one: 190
+    // us for 4,096 variants; four: no faster).
+    for (const void* k : {reinterpret_cast<const void*>(gnm_pgen_row<false>),
+                          reinterpret_cast<const void*>(gnm_pgen_row<true>)})
+      check_cuda(raise_smem_limit(k, int(kPgRowMax)), "pgen row shared memory");
+    const uint32_t own = (a.direct ? a.ndirect : a.count) + a.extra_rows;
+    if (own) gnm_pgen_row<false><<<own, 256, uint32_t(row_bytes), s>>>(a);
+    check_cuda(cudaGetLastError(), "pgen decode launch");
+    const uint64_t per_sm = std::min<uint64_t>(32, kPgSmem / (row_bytes + 1024));
+    uint32_t warps = 1;
+    while (warps < 16 && warps * per_sm < 32) warps *= 2;
+    gnm_pgen_row<true><<<a.count, 32 * warps, uint32_t(row_bytes), s>>>(a);
+  } else {
+    gnm_pgen_direct<<<a.count + a.extra_rows, kPgThreads, 0, s>>>(a);
+    check_cuda(cudaGetLastError(), "pgen decode launch");
+    gnm_pgen_ld<<<uint32_t((uint64_t(a.count) + kPgWarps - 1) / kPgWarps), kPgThreads, 0, s>>>(a);
+  }
   check_cuda(cudaGetLastError(), "pgen LD decode launch");
   if (a.any_dosage || a.any_multi) {   // patches and dosages, on the finished rows
     if (a.ma_smem > 48 * 1024)
@@ -1367,6 +1748,10 @@ static void pgen_decode_impl(gnm_pgen* pg, uint64_t begin, uint64_t count, uint8
       break;
     }
   a.extra_rows = a.extra != kNoAnchor ? 1u : 0u;
+  const auto lo = std::lower_bound(pg->direct.begin(), pg->direct.end(), uint32_t(begin));
+  const auto hi = std::lower_bound(lo, pg->direct.end(), uint32_t(begin + count));
+  a.direct = pg->d_direct + (lo - pg->direct.begin());
+  a.ndirect = uint32_t(hi - lo);
   DeviceGuard g(pg->device);
   launch_decode(a, s);
 }
