@@ -1603,17 +1603,16 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
     const uint64_t valid = *reinterpret_cast<volatile uint32_t*>(a.state);
     for (uint64_t u = u0; u < u1; ++u, ++n) {
       const uint32_t s = n % ST, ph = (n / ST) & 1u;
-      if (!mbar_wait_warp(full(s), ph)) {
-        give_up(kErrTmaTimeout);
-        break;
-      }
+      // Waits that run out are remembered, not acted on: the tensor-memory stores
+      // need the whole warp, and a vote per wait costs 10 % of the kernel.  The
+      // stage's end leaves the loop for the warp as one.
+      uint32_t late = mbar_wait_bounded(full(s), ph) ? 0u : kErrTmaTimeout;
       constexpr uint32_t kTurns = 4 / kEvery;   // this warp's slots of the stage
       uint32_t x[kTurns][4];   // [16 variants each][byte columns 0-7, 8-15]
 #pragma unroll
       for (uint32_t j = 0; j < kTurns; ++j)
         ldmatrix_t_b8(pk0 + s * L::kTma + j * (32 * kEvery * L::kPkRow), x[j]);
       const uint32_t aborted = lds_volatile_u32(abort_addr);
-      bool ok = true;
 #pragma unroll
       for (uint32_t j = 0; j < kTurns; ++j) {
         // columns of block h: dosage of variants 0-15, 16-31, missing likewise;
@@ -1640,11 +1639,8 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
         // arithmetic below it)
 #pragma unroll
         for (uint32_t i = 0; i < 16; ++i) asm volatile("" : "+r"(lo[i]), "+r"(hi[i]));
-        if (!mbar_wait_warp(sfree(slot, pairm), sph ^ 1u)) {
-          give_up(kErrMmaTimeout);
-          ok = false;
-          break;
-        }
+        if (!mbar_wait_bounded(sfree(slot, pairm), sph ^ 1u)) late |= kErrMmaTimeout;
+        __syncwarp();
         tc_fence_after();
         const uint32_t op = op0 + slot * L::kSlotCols;
         tmem_st_16x128b_x8(op, lo);
@@ -1659,7 +1655,10 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
           sph ^= 1u;
         }
       }
-      if (!ok || aborted) break;
+      if (__any_sync(0xFFFFFFFFu, (late | aborted) != 0u)) {
+        if (late) give_up(late);
+        break;
+      }
       ++inblk;
       const uint32_t tile_now = tile;
       const bool tile_end = ++st == a.stages;
@@ -2302,11 +2301,12 @@ struct Bw8Args {
 // The missing term of one variant over people [p0, p1) of a score whose largest
 // |dS| is an infinity or NaN, which limbs cannot hold: the sum of the dS values
 // themselves, so that only variants at which such a person is missing get one.
-__device__ __noinline__ double bw_missing_sum(const Bw8Args& a, uint64_t v, uint64_t k, uint64_t p0,
-                                              uint64_t p1) {
+// (`row`: the variant's packed row, `ds`: the score's column of dS, `K` apart.)
+__device__ __noinline__ double bw_missing_sum(const uint8_t* row, const float* ds, uint64_t K,
+                                              uint64_t p0, uint64_t p1) {
   double s = 0.0;
-  for (uint64_t p = p0; p < p1 && p < a.people; ++p)
-    if (((a.rows[v * a.pitch + p / 4] >> (2 * (p % 4))) & 3u) == 1u) s += double(a.ds[p * a.K + k]);
+  for (uint64_t p = p0; p < p1; ++p)
+    if (((row[p / 4] >> (2 * (p % 4))) & 3u) == 1u) s += double(ds[p * K]);
   return s;
 }
 
@@ -2484,12 +2484,9 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
     for (uint32_t k = 0; k < kBwScores; ++k) acc[k] = 0.0;
     for (uint64_t u = u0; u < u1; ++u, ++n) {
       const uint32_t s = n % ST, ph = (n / ST) & 1u;
-      if (!mbar_wait_warp(full(s), ph)) {
-        give_up(kErrTmaTimeout);
-        break;
-      }
+      // waits that run out are acted on at the stage's end (see gnm_t8_narrow)
+      uint32_t late = mbar_wait_bounded(full(s), ph) ? 0u : kErrTmaTimeout;
       const uint32_t aborted = lds_volatile_u32(abort_addr);
-      bool ok = true;
       uint4 x4 = lds_u128(pk0 + s * L::kStage + ((mine ^ (r & 7u)) << 4));
 #pragma unroll
       for (uint32_t j = 0; j < kBw8K / 128; ++j) {
@@ -2519,11 +2516,8 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
         for (uint32_t i = 0; i < (CORR ? 32u : 16u); ++i) asm volatile("" : "+r"(v[i]));
         // a stage is two turns of the ring, so slots and phases are constants
         const uint32_t op = op0 + (2 * (j % 2)) * kBw8SlotCols;
-        if (!mbar_wait_warp(sfree0 + 16 * (j % 2), (j / 2) ^ 1u)) {
-          give_up(kErrMmaTimeout);
-          ok = false;
-          break;
-        }
+        if (!mbar_wait_bounded(sfree0 + 16 * (j % 2), (j / 2) ^ 1u)) late |= kErrMmaTimeout;
+        __syncwarp();
         tc_fence_after();
         if (CORR)
           tmem_st_32x32b_x32(op, v);
@@ -2534,7 +2528,10 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(ready0 + 16 * (j % 2));
       }
-      if (!ok || aborted) break;
+      if (__any_sync(0xFFFFFFFFu, (late | aborted) != 0u)) {
+        if (late) give_up(late);
+        break;
+      }
       ++inblk;
       const uint32_t tile_now = tile;
       const bool tile_end = ++st == a.stages;
@@ -2581,7 +2578,8 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
 #pragma unroll
             for (uint32_t k = 0; k < kBwScores; ++k)
               if (k0 + k < a.K && !isfinite(a.quanta[k0 + k]))
-                acc[k] = -bw_missing_sum(a, v, k0 + k, s0 * kBw8K, (u + 1 - t0) * kBw8K);
+                acc[k] = -bw_missing_sum(a.rows + v * a.pitch, a.ds + k0 + k, a.K, s0 * kBw8K,
+                                         min(a.people, (u + 1 - t0) * kBw8K));
           }
           if (CORR || mine == 0) {
             if (t0 >= u0 && tile_end) {   // the whole tile is this CTA's
