@@ -78,7 +78,7 @@ struct TensorPlan {
   uint64_t P_nar = 0;                     // narrow: people rounded up to 512
   uint64_t nslot = 0;                     // narrow: elements per slot (K16 * P_nar)
   uint32_t nalloc = 0;                    // narrow: slots allocated
-  uint32_t ncta = 1;                      // narrow 8-bit: CTAs per score tile
+  uint32_t sms = 1;
   uint32_t* d_state = nullptr;            // narrow: slot state (slots_written)
   bool wide_clear = false;                // wide partials cleared since the last reset
   CUtensorMap map_dos, map_mis;
@@ -94,6 +94,7 @@ struct TensorPlan {
   bool can_narrow = false;                // K <= 64: either kernel can run the plan
   CUtensorMap nmap_dos, nmap_mis;         // narrow boxes: 16 scores x 4 planes
   CUtensorMap nmap8_dos, nmap8_mis;       // narrow 8-bit boxes: 128 variants x 16 scores x 4 / 5 planes
+  CUtensorMap nmap8_dos2, nmap8_mis2;     // the same with 32 scores
 };
 
 struct TcArgs {
@@ -1324,35 +1325,44 @@ __global__ void __launch_bounds__(kNrThreads, 1)
 // columns) beside a three-slot ring of operands (64 columns per 32 variants),
 // and every 18 KB of limbs staged from L2 feeds 512 people instead of 128.
 // NMT = 2 (256 people, eight slots) takes the cohorts and calls too small to
-// fill the chip with 512-person tiles.
+// fill the chip with 512-person tiles.  With 32 scores per CTA (NS = 2, the same
+// 320 columns as 2 x 160, six slots) a genotype is expanded once for twice the
+// scores: two tiles of 16 ran the expansion, which the MMAs of 16 scores do not
+// cover, twice.
 //
-// Work is split evenly, not by tiles: a CTA takes `quota` consecutive
-// (people tile, stage) units of its score tile, so one CTA covers the tail of
-// one tile and the head of the next and every SM finishes together; each of
-// a tile's few segments writes its own FP64 slot.  CTAs of different score
-// tiles walk the rows in step and share them in L2.
+// Work is split evenly, not by tiles: first whole people tiles, all CTAs at the
+// same stage, then of the last one to two tiles per CTA `quota` consecutive
+// (people tile, stage) units each, so one CTA covers the tail of one tile and
+// the head of the next and every SM finishes together; each of a tile's few
+// segments writes its own FP64 slot.  CTAs of different score tiles walk the
+// rows in step and share them in L2; whole tiles let the people tiles share the
+// limbs too, which even shares alone, each at its own variants, read from HBM
+// once they overflow L2 (200,000 people x 60,000 variants x 64 scores: 3.84 ms
+// on 16 scores per CTA, 3.76 on 32, 3.39 on 32 with whole tiles).
 //
 // S32 sums are exact for 2^17 variants: |limb x 4^q x dosage| <= 127 x 128.
-constexpr uint32_t kT8NrScoreRows = 4 * kNrScores;   // limb rows of one operand
-constexpr uint32_t kT8NrCols = 5 * kNrScores;        // accumulator columns per 128 people
 constexpr uint32_t kT8NrFlush = 1024;                // stages per exact S32 block (2^17 variants)
 constexpr uint32_t kT8NrGroups = 4;                  // expansion warps per TMEM lane quadrant
 constexpr uint32_t kT8NrThreads = 128 + 128 * kT8NrGroups;   // TMA, two MMA warps, one idle
 
-template <int NMT>
+template <int NMT, int NS>
 struct T8NrSmem {
-  static constexpr uint32_t kStages = NMT == 4 ? 6 : 8;
-  static constexpr uint32_t kSlots = NMT == 4 ? 3 : 8;      // operand ring, 32 variants each
+  static constexpr uint32_t kScores = kNrScores * NS;       // scores per CTA
+  static constexpr uint32_t kRows = 4 * kScores;            // limb rows of the dosage operand
+  static constexpr uint32_t kCols = 5 * kScores;            // accumulator columns per 128 people
+  static constexpr uint32_t kStages = NS == 2 ? 5 : NMT == 4 ? 6 : 8;
+  // operand ring, 32 variants each
+  static constexpr uint32_t kSlots = NS == 2 ? 6 : NMT == 4 ? 3 : 8;
   static constexpr uint32_t kSlotCols = 16 * NMT;           // 8 dosage + 8 missing per block
   static constexpr uint32_t kParts = NMT / 2;               // a slot's parts: two blocks each
-  static constexpr uint32_t kRing0 = kT8NrCols * NMT;       // first operand column
+  static constexpr uint32_t kRing0 = kCols * NMT;           // first operand column
   static constexpr uint32_t kPeople = kNrM * NMT;
   static constexpr uint32_t kPkRow = kPeople / 4;           // packed bytes per variant row
   static constexpr uint32_t kPk = kT8K * kPkRow;
   static constexpr uint32_t kBDos = 0;                      // offsets inside a TMA stage
-  static constexpr uint32_t kBMis = kT8NrScoreRows * kT8K;  // 8 KB
-  static constexpr uint32_t kPkIn = kBMis + kT8NrCols * kT8K;   // + 10 KB
-  static constexpr uint32_t kTma = kPkIn + kPk;             // 34 / 26 KB
+  static constexpr uint32_t kBMis = kRows * kT8K;           // 8 KB (NS = 1)
+  static constexpr uint32_t kPkIn = kBMis + kCols * kT8K;   // + 10 KB
+  static constexpr uint32_t kTma = kPkIn + kPk;             // 34, 26 or 44 KB
   static constexpr uint32_t kBarOff = kStages * kTma;
   static constexpr uint32_t kBars = 2 * kStages + 2 * kSlots * kParts + 4;
   static constexpr uint32_t kHolder = kBarOff + 8 * kBars;
@@ -1399,19 +1409,59 @@ struct T8NrArgs {
   uint32_t* err;
   uint32_t stages;         // stages of the block (128 variants each)
   uint32_t ptiles;         // people tiles
-  uint32_t quota;          // (people tile, stage) units per CTA
+  uint32_t rounds;         // whole people tiles per CTA, before its share of the rest
+  uint32_t quota;          // (people tile, stage) units per share
   uint32_t slots;          // slots of every tile; those without a segment are zeroed
   uint32_t* state;         // {slots written since the reset, CTAs done}: see SlotState
   const double* quanta;    // [kT8Planes][K_pad]
   uint64_t K_pad;
+  uint64_t K16;            // scores the partials hold
 };
 
-template <int NMT>
+// The (people tile, stage) units of a CTA in order: `rounds` whole tiles, CTA c the
+// tiles c, c + CTAs, ..., then units [u0, u1) of the tiles left.
+struct T8NrWalk {
+  uint32_t tile, st, round, units;   // the current unit; units in all
+  uint32_t u0_tile, u0_st;
+  __device__ explicit T8NrWalk(const T8NrArgs& a) {
+    const uint32_t base = a.rounds * gridDim.x;
+    const uint64_t rest = uint64_t(a.ptiles - base) * a.stages;
+    const uint64_t u0 = min(uint64_t(blockIdx.x) * a.quota, rest);
+    const uint64_t u1 = min(u0 + a.quota, rest);
+    units = a.rounds * a.stages + uint32_t(u1 - u0);
+    u0_tile = base + uint32_t(u0 / a.stages);
+    u0_st = uint32_t(u0 % a.stages);
+    round = 0;
+    tile = a.rounds ? blockIdx.x : u0_tile;
+    st = a.rounds ? 0u : u0_st;
+  }
+  __device__ void next(const T8NrArgs& a) {
+    if (++st < a.stages) return;
+    st = 0;
+    if (round >= a.rounds) {
+      ++tile;
+    } else if (++round < a.rounds) {
+      tile += gridDim.x;
+    } else {
+      tile = u0_tile;
+      st = u0_st;
+    }
+  }
+  // the slot of the current unit's segment: its share's place among the tile's
+  __device__ uint32_t slot(const T8NrArgs& a) const {
+    if (round < a.rounds) return 0u;
+    const uint64_t t0 = uint64_t(tile - a.rounds * gridDim.x) * a.stages;
+    return blockIdx.x - uint32_t(t0 / a.quota);
+  }
+};
+
+template <int NMT, int NS>
 __global__ void __launch_bounds__(kT8NrThreads, 1)
     gnm_t8_narrow(const __grid_constant__ CUtensorMap dmap,
                   const __grid_constant__ CUtensorMap mmap,
                   const __grid_constant__ CUtensorMap pmap, T8NrArgs a) {
-  using L = T8NrSmem<NMT>;
+  static_assert(NS == 1 || NMT == 2, "accumulator columns");
+  using L = T8NrSmem<NMT, NS>;
   constexpr uint32_t ST = L::kStages, R = L::kSlots, RP = R * L::kParts;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
@@ -1419,10 +1469,11 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
   const uint32_t sb = smem_u32(smem);
   const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t stile = blockIdx.y;
-  const uint64_t units = uint64_t(a.ptiles) * a.stages;
-  const uint64_t u0 = uint64_t(blockIdx.x) * a.quota;
-  const uint64_t u1 = u0 + a.quota < units ? u0 + a.quota : units;
-  if (u0 >= u1) return;   // uniform per CTA (the host launches none such)
+  T8NrWalk w(a);
+  if (w.units == 0) {   // uniform per CTA
+    if (threadIdx.x == 0) slots_written(a.state, a.slots, gridDim.x * gridDim.y);
+    return;
+  }
   auto full = [&](uint32_t s) { return sb + L::kBarOff + 8 * s; };           // TMA landed
   auto tempty = [&](uint32_t s) { return sb + L::kBarOff + 8 * (ST + s); };  // stage free
   // part p of operand slot b: filled by its four warps / read by its MMAs
@@ -1474,9 +1525,8 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       uint32_t n = 0;            // stages issued
-      uint32_t tile = uint32_t(u0 / a.stages), st = uint32_t(u0 % a.stages);
       bool ok = true;
-      for (uint64_t u = u0; u < u1; ++u, ++n) {
+      for (; n < w.units; ++n, w.next(a)) {
         const uint32_t s = n % ST, ph = (n / ST) & 1u;
         if (!mbar_wait_bounded(tempty(s), ph ^ 1u)) {
           give_up(kErrMmaTimeout);
@@ -1489,14 +1539,11 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
         }
         const uint32_t at = sb + s * L::kTma;
         mbar_arrive_expect_tx(full(s), L::kTma);
-        const int32_t x = a.a_x0 + int32_t(st * kT8K);
-        tma_load_2d(at + L::kPkIn, &pmap, int32_t(tile * L::kPkRow), int32_t(st * kT8K), full(s));
-        tma_load_3d(at + L::kBMis, &mmap, x, int32_t(stile * kNrScores), 4, full(s));
-        tma_load_3d(at + L::kBDos, &dmap, x, int32_t(stile * kNrScores), 0, full(s));
-        if (++st == a.stages) {
-          st = 0;
-          ++tile;
-        }
+        const int32_t x = a.a_x0 + int32_t(w.st * kT8K);
+        tma_load_2d(at + L::kPkIn, &pmap, int32_t(w.tile * L::kPkRow), int32_t(w.st * kT8K),
+                    full(s));
+        tma_load_3d(at + L::kBMis, &mmap, x, int32_t(stile * L::kScores), 4, full(s));
+        tma_load_3d(at + L::kBDos, &dmap, x, int32_t(stile * L::kScores), 0, full(s));
       }
       if (!ok)   // nothing may still be in flight when the CTA exits (bounded)
         for (uint32_t i = n > ST ? n - ST : 0; i < n; ++i)
@@ -1513,16 +1560,15 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
     // descriptors then stay in uniform registers, which tcgen05.mma reads (a
     // loop that only lane 0 runs moves each over per instruction: 60 clocks per
     // MMA).
-    constexpr uint32_t idesc_d = idesc_u8s8_s32(kNrM, kT8NrScoreRows);
-    constexpr uint32_t idesc_m = idesc_u8s8_s32(kNrM, kT8NrCols);
+    constexpr uint32_t idesc_d = idesc_u8s8_s32(kNrM, L::kRows);
+    constexpr uint32_t idesc_m = idesc_u8s8_s32(kNrM, L::kCols);
     constexpr uint32_t kMine = NMT / 2;                  // blocks of this warp
     const uint32_t b0 = (warp - 1) * kMine;
     const uint32_t part = NMT == 4 ? warp - 1 : 0u;
-    uint32_t st = uint32_t(u0 % a.stages), blk = 0, inblk = 0, n = 0, slot = 0, sph = 0;
-    const uint32_t left = uint32_t(u1 - u0);
+    uint32_t blk = 0, inblk = 0, n = 0, slot = 0, sph = 0;
     const uint32_t utmem = __shfl_sync(0xFFFFFFFFu, tmem, 0);
     bool ok = true;
-    for (; n < left && ok; ++n) {
+    for (; n < w.units && ok; ++n, w.next(a)) {
       const uint32_t s = n % ST;
       if (inblk == 0 && blk > 0 && !mbar_wait_warp(accempty, (blk - 1) & 1u)) {
         give_up(kErrMmaTimeout);
@@ -1532,7 +1578,7 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
       const uint32_t at = sb + s * L::kTma;
       const uint64_t bm0 = desc_kmajor_sw128(at + L::kBMis);
       const uint64_t bd0 = desc_kmajor_sw128(at + L::kBDos);
-      const bool last = st + 1 == a.stages || inblk + 1 == kT8NrFlush || n + 1 == left;
+      const bool last = w.st + 1 == a.stages || inblk + 1 == kT8NrFlush || n + 1 == w.units;
 #pragma unroll
       for (uint32_t kk = 0; kk < kT8K / 32; ++kk) {   // 32 variants per slot and MMA
         // the warps that filled the slot waited for the stage's limbs too
@@ -1545,15 +1591,15 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
         if (elect_one()) {
           const uint64_t bm = bm0 + 2 * kk, bd = bd0 + 2 * kk;   // 32 bytes further
           const uint32_t op = utmem + L::kRing0 + slot * L::kSlotCols + 16 * b0;
-          const uint32_t d = utmem + kT8NrCols * b0;
-          // the missing product covers all 80 columns, so it starts a block
+          const uint32_t d = utmem + L::kCols * b0;
+          // the missing product covers all columns, so it starts a block
           const uint32_t acc = (inblk == 0 && kk == 0) ? 0u : 1u;
 #pragma unroll
           for (uint32_t t = 0; t < kMine; ++t)
-            tc_mma_i8_ta(d + t * kT8NrCols, op + 16 * t + 8, bm, idesc_m, acc);
+            tc_mma_i8_ta(d + t * L::kCols, op + 16 * t + 8, bm, idesc_m, acc);
 #pragma unroll
           for (uint32_t t = 0; t < kMine; ++t)
-            tc_mma_i8_ta(d + t * kT8NrCols, op + 16 * t, bd, idesc_d, 1u);
+            tc_mma_i8_ta(d + t * L::kCols, op + 16 * t, bd, idesc_d, 1u);
           tc_commit(sfree(slot, part));
           if (kk == kT8K / 32 - 1) {
             tc_commit(tempty(s));
@@ -1567,7 +1613,6 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
         }
       }
       ++inblk;
-      if (++st == a.stages) st = 0;
       if (last) {   // end of a block
         ++blk;
         inblk = 0;
@@ -1597,11 +1642,10 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
     const uint32_t pk0 = sb + L::kPkIn + row * L::kPkRow +
                          ((NMT == 4 ? (chunk ^ (row & 7u)) : (chunk ^ ((row >> 1) & 3u))) << 4);
     const uint32_t op0 = tmem + ((32 * quad) << 16) + L::kRing0 + 32 * pairm;
-    uint32_t tile = uint32_t(u0 / a.stages), st = uint32_t(u0 % a.stages);
     uint32_t blk = 0, inblk = 0, n = 0, slot = mine, sph = 0;
     bool first = true;   // the segment's first block
     const uint64_t valid = *reinterpret_cast<volatile uint32_t*>(a.state);
-    for (uint64_t u = u0; u < u1; ++u, ++n) {
+    for (; n < w.units; ++n, w.next(a)) {
       const uint32_t s = n % ST, ph = (n / ST) & 1u;
       // Waits that run out are remembered, not acted on: the tensor-memory stores
       // need the whole warp, and a vote per wait costs 10 % of the kernel.  The
@@ -1660,13 +1704,8 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
         break;
       }
       ++inblk;
-      const uint32_t tile_now = tile;
-      const bool tile_end = ++st == a.stages;
-      if (tile_end) {
-        st = 0;
-        ++tile;
-      }
-      if (tile_end || inblk == kT8NrFlush || u + 1 == u1) {
+      const bool tile_end = w.st + 1 == a.stages;
+      if (tile_end || inblk == kT8NrFlush || n + 1 == w.units) {
         // ---- epilogue: drain one 128-person block of the tile ----
         inblk = 0;
         if (!mbar_wait_warp(accfull, blk & 1u)) {
@@ -1679,19 +1718,20 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
         const uint32_t q = lane >> 3;        // row scale 4^q
         // TMEM lane 8q + r of quadrant `quad`, block t: person q of the
         // quadrant's packed byte 8t + r
-        const uint64_t person = uint64_t(tile_now) * L::kPeople +
+        const uint64_t person = uint64_t(w.tile) * L::kPeople +
                                 4 * (8 * NMT * quad + 8 * t + (lane & 7u)) + q;
-        const uint32_t base = tmem + ((32 * quad) << 16) + t * kT8NrCols;
+        const uint32_t base = tmem + ((32 * quad) << 16) + t * L::kCols;
         const double scale = 1.0 / double(1u << (2 * q));
-        const uint64_t first_cta = uint64_t(tile_now) * a.stages / a.quota;
-        const uint64_t sl = blockIdx.x - first_cta;
+        const uint64_t sl = w.slot(a);
         const bool write = sl >= valid && first;
         const bool in = person < a.P_pad;
-        constexpr uint32_t kHalves = NMT == 4 ? 2 : 1;   // 256 people: two warps share a block
+        // scores eight at a time; with 256 people two warps share a block's scores
+        constexpr uint32_t kOcts = 2 * NS / (NMT == 4 ? 1 : 2);
 #pragma unroll 1
-        for (uint32_t i = 0; i < kHalves; ++i) {
-          const uint32_t half = NMT == 4 ? i : (grp >> 1);
-          const uint64_t k0 = uint64_t(stile) * kNrScores + 8 * half;
+        for (uint32_t i = 0; i < kOcts; ++i) {
+          const uint32_t oct = NMT == 4 ? i : (grp >> 1) * kOcts + i;
+          const uint64_t k0 = uint64_t(stile) * L::kScores + 8 * oct;
+          if (k0 >= a.K16) break;   // (the same for the whole warp)
           double acc[8];
           uint32_t cnt[8];
 #pragma unroll
@@ -1699,7 +1739,7 @@ __global__ void __launch_bounds__(kT8NrThreads, 1)
 #pragma unroll
           for (uint32_t g = 0; g < 5; ++g) {
             uint32_t d[8];
-            tmem_ld8(base + 16 * g + 8 * half, d);
+            tmem_ld8(base + L::kScores * g + 8 * oct, d);
             tmem_ld_wait();
 #pragma unroll
             for (uint32_t k = 0; k < 8; ++k) {
@@ -2914,6 +2954,12 @@ static uint32_t narrow_splits(uint64_t base_ctas, uint64_t stages, int sms) {
   return best;
 }
 
+// CTAs per score tile, tiles of 16 * ns scores sharing the SMs.
+static uint32_t narrow_ctas(const TensorPlan* t, uint64_t K, uint32_t ns) {
+  const uint64_t stiles = (K + kNrScores * ns - 1) / (kNrScores * ns);
+  return std::max<uint32_t>(1, uint32_t(t->sms / stiles));
+}
+
 void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trace) {
   auto mark = [&](const char* what) {
     if (trace) trace->mark(what);
@@ -2959,10 +3005,14 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
     t->nsplits = narrow_splits(base, t->V_pad / kTcK, std::max(1, sms));
     t->P_nar = std::max<uint64_t>(1, (p->fam + 4 * kNrM - 1) / (4 * kNrM)) * (4 * kNrM);
     t->nslot = k16 * t->P_nar;
+    t->sms = uint32_t(std::max(1, sms));
     // a tile of S stages meets at most S / quota + 2 CTAs' shares, and quota >=
-    // ptiles * S / ncta
-    t->ncta = std::max<uint32_t>(1, uint32_t(std::max(1, sms)) / uint32_t(k16 / kNrScores));
-    t->nalloc = std::max(t->nsplits, t->ncta / uint32_t(t->P_nar / (4 * kNrM)) + 2);
+    // ptiles * S / (CTAs per score tile)
+    const uint32_t ns = p->K > kNrScores ? 2 : 1;
+    const uint64_t people = ns == 2 ? 2 * kNrM : 4 * kNrM;   // of the widest tile in use
+    t->nalloc = std::max(t->nsplits, narrow_ctas(t, p->K, ns) /
+                                         uint32_t(std::max<uint64_t>(1, (p->fam + people - 1) /
+                                                                            people)) + 2);
     t->part_elems = std::max(t->part_elems, uint64_t(t->nalloc) * t->nslot);
     t->d_state = p->d_err + 1;   // cleared with the error word by every reset
   }
@@ -3038,6 +3088,8 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
     t->nmap_mis = make_plane_map(t->d_planes_mis, t->V_pad, t->K_pad, kNrScores, 4);
     t->nmap8_dos = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, kNrScores, 4);
     t->nmap8_mis = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, kNrScores, 5);
+    t->nmap8_dos2 = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, 2 * kNrScores, 4);
+    t->nmap8_mis2 = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, 2 * kNrScores, 5);
   }
 }
 
@@ -3092,23 +3144,32 @@ void tensor_reset(gnm_plan* p, cudaStream_t s) {
   t->pass_valid = false;   // the next SM-pair accumulate writes its pass arrays
 }
 
-template <int NMT>
-static void launch_t8_narrow(const TensorPlan* t, const uint8_t* d_rows, uint64_t pitch,
-                             uint64_t bpv, uint64_t nv, uint32_t stiles, T8NrArgs a,
-                             cudaStream_t s) {
-  using L = T8NrSmem<NMT>;
+template <int NMT, int NS>
+static void launch_t8_narrow(const gnm_plan* p, const uint8_t* d_rows, uint64_t pitch,
+                             uint64_t nv, T8NrArgs a, cudaStream_t s) {
+  using L = T8NrSmem<NMT, NS>;
+  const TensorPlan* t = p->tensor;
   const CUtensorMap pmap =
-      make_row_map(d_rows, bpv, nv, pitch, L::kPkRow, kT8K,
+      make_row_map(d_rows, p->bpv, nv, pitch, L::kPkRow, kT8K,
                    NMT == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
-  check_cuda(raise_smem_limit(reinterpret_cast<const void*>(gnm_t8_narrow<NMT>), int(L::kTotal)),
+  check_cuda(raise_smem_limit(reinterpret_cast<const void*>(gnm_t8_narrow<NMT, NS>),
+                              int(L::kTotal)),
              "narrow 8-bit shared memory");
-  a.ptiles = uint32_t(std::max<uint64_t>(1, (bpv + L::kPkRow - 1) / L::kPkRow));
-  const uint64_t units = uint64_t(a.ptiles) * a.stages;
-  a.quota = uint32_t((units + t->ncta - 1) / t->ncta);
+  const uint32_t ncta = narrow_ctas(t, p->K, NS);
+  a.ptiles = uint32_t(std::max<uint64_t>(1, (p->bpv + L::kPkRow - 1) / L::kPkRow));
+  // Whole tiles while at least two rounds of CTAs are left: those CTAs start every
+  // tile at its first variant together and share the limbs in L2, which long rows'
+  // limbs overflow (50,000 x 100,000 x 512, 460 MB of them: 15.2 ms with shares
+  // only).  The one to two rounds that remain go in even shares.
+  a.rounds = a.ptiles >= 2 * ncta ? a.ptiles / ncta - 1 : 0u;
+  const uint64_t units = uint64_t(a.ptiles - a.rounds * ncta) * a.stages;
+  a.quota = uint32_t((units + ncta - 1) / ncta);
   a.slots = (a.stages + a.quota - 2) / a.quota + 1;
   if (a.slots > t->nalloc) fail(GNM_ERR_COMPUTE, "narrow engine: more slots than allocated");
-  const dim3 grid(uint32_t((units + a.quota - 1) / a.quota), stiles);
-  gnm_t8_narrow<NMT><<<grid, kT8NrThreads, L::kTotal, s>>>(t->nmap8_dos, t->nmap8_mis, pmap, a);
+  const dim3 grid(a.rounds ? ncta : uint32_t((units + a.quota - 1) / a.quota),
+                  uint32_t((p->K + L::kScores - 1) / L::kScores));
+  gnm_t8_narrow<NMT, NS><<<grid, kT8NrThreads, L::kTotal, s>>>(
+      NS == 2 ? t->nmap8_dos2 : t->nmap8_dos, NS == 2 ? t->nmap8_mis2 : t->nmap8_mis, pmap, a);
   check_cuda(cudaGetLastError(), "narrow 8-bit tensor launch");
 }
 
@@ -3118,9 +3179,9 @@ static void launch_t8_narrow(const TensorPlan* t, const uint8_t* d_rows, uint64_
 // 512: half the limb traffic per person.  100,000 variants x 16 scores,
 // 20,000 people: 191 us on 512-person tiles, 266 us on 256-person ones; 10,000
 // variants: 44 and 50 us.
-static bool narrow_small_tiles(const TensorPlan* t, uint64_t people, uint64_t stages) {
+static bool narrow_small_tiles(uint32_t ncta, uint64_t people, uint64_t stages) {
   const uint64_t u4 = (people + 511) / 512 * stages, u2 = (people + 255) / 256 * stages;
-  const uint64_t q4 = (u4 + t->ncta - 1) / t->ncta, q2 = (u2 + t->ncta - 1) / t->ncta;
+  const uint64_t q4 = (u4 + ncta - 1) / ncta, q2 = (u2 + ncta - 1) / ncta;
   return 8 * q4 > 5 * q2;
 }
 
@@ -3142,11 +3203,14 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
     a.state = t->d_state;
     a.quanta = t->d_quanta8;
     a.K_pad = t->K_pad;
-    const uint32_t stiles = uint32_t((p->K + kNrScores - 1) / kNrScores);
-    if (narrow_small_tiles(t, p->fam, a.stages))
-      launch_t8_narrow<2>(t, d_rows, pitch, p->bpv, nv, stiles, a, s);
+    a.K16 = (p->K + kNrScores - 1) / kNrScores * kNrScores;
+    // Over 16 scores: 32 per CTA, so that half as many CTAs expand the same rows.
+    if (p->K > kNrScores)
+      launch_t8_narrow<2, 2>(p, d_rows, pitch, nv, a, s);
+    else if (narrow_small_tiles(narrow_ctas(t, p->K, 1), p->fam, a.stages))
+      launch_t8_narrow<2, 1>(p, d_rows, pitch, nv, a, s);
     else
-      launch_t8_narrow<4>(t, d_rows, pitch, p->bpv, nv, stiles, a, s);
+      launch_t8_narrow<4, 1>(p, d_rows, pitch, nv, a, s);
     p->launches += 1;
     return;
   }

@@ -90,3 +90,15 @@ def test_blocks_at_the_s32_limit(cuda, byte, code):
     np.testing.assert_allclose(s, np.broadcast_to(want, s.shape), rtol=0, atol=TOL * variants)
     np.testing.assert_array_equal(c, variants if code == 1 else 0)
     plan.close()
+
+
+@pytest.mark.parametrize("people,variants,scores,blocks", [
+    (38_000, 257, 40, None), (57_000, 140, 64, [(0, 128), (128, 12)]),
+    (76_000, 300, 17, [(0, 128), (128, 172)]), (152_000, 130, 3, None)])
+def test_whole_tiles_then_shares(cuda, people, variants, scores, blocks):
+    """Two and more rounds of people tiles per CTA: whole tiles first, then even
+    shares of the rest, with each of the kernel's tile sizes; a second call adds
+    to the slots of both."""
+    _, prep, rows, _ = synth_case(people, variants, scores=scores,
+                                  config="batched_100k_x_500k_k512")
+    check(prep, rows, run(prep, rows, blocks))
