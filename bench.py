@@ -474,7 +474,10 @@ def gpu_arm(args, rank, world, local_rank):
         # over 256-person x 128-score tiles (256-score tiles on SM pairs) and
         # 128-variant stages; the integer peak is taken as twice the BF16 one
         # (the nominal dense ratio, 4.5 / 2.25)
-        mt = 256 if tshape & 8 else 128
+        # (in the shape a plan starts with, 13 or 5, people are the M: 256 people x
+        # 32 scores, 5 + 4 planes)
+        people_m = tshape == (13 if K > 128 else 5) and K > 64
+        mt = 32 if people_m else 256 if tshape & 8 else 128
         ptiles, kpad, vpad = -(-P // 256), -(-K // mt) * mt, -(-V // 128) * 128
         executed = 2.0 * ptiles * 256 * vpad * kpad * 9
         flops = 2.0 * P * nnz * 3
@@ -483,7 +486,9 @@ def gpu_arm(args, rank, world, local_rank):
         roof = {"bound": "tensor", "achieved": achieved, "peak": pk, "unit": "TFLOP/s",
                 "frac": achieved / pk, "traffic": None,
                 "peak_kind": peak_kind + " (bf16 sustained)",
-                "kernel": ("gnm_t8_pair (8-bit limbs on SM pairs, cta_group::2; "
+                "kernel": ("gnm_t8_narrow (8-bit limbs, people as M; "
+                           if people_m else
+                           "gnm_t8_pair (8-bit limbs on SM pairs, cta_group::2; "
                            if tshape & 8 else "gnm_t8_accumulate (8-bit limbs, ")
                 + "dosage + missing + count passes)",
                 "kernel_ms": kernel_ms, "algorithmic_flops_per_launch": flops,

@@ -760,36 +760,32 @@ static void autotune_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, ui
     plain_shape(p, best_kernel, best_mult);
   } else {
     // shape bit 0: raster order of the wide kernel; bit 1: the narrow kernel;
-    // bit 2: 8-bit limbs; bit 3: the 8-bit wide kernel over SM pairs
+    // bit 2: 8-bit limbs; bit 3: the 8-bit wide kernel over SM pairs.  Over 64
+    // scores the plan's first shape (13; 5 up to 128 scores) runs people as M
+    const uint32_t people = tensor_default_shape(p);
     std::vector<uint32_t> cand = {0u, 1u, 4u, 5u, 12u, 13u};
     if (tensor_can_narrow(p)) cand.insert(cand.begin(), {2u, 6u});
-    uint32_t best = (tensor_is_narrow(p) ? 2u : 0u) | (tensor_is_i8(p) ? 4u : 0u) |
-                    (tensor_is_pair(p) ? 8u : 0u) | p->raster;
+    uint32_t best = tensor_shape(p);
     const char* tr = std::getenv("GNM_TRACE");
     const bool trace = tr && std::strcmp(tr, "0") != 0;
     for (uint32_t c : cand) {
-      tensor_set_narrow(p, (c & 2u) != 0);
-      tensor_set_i8(p, (c & 4u) != 0);
-      tensor_set_pair(p, (c & 8u) != 0);
-      p->raster = c & 1u;
+      tensor_set_shape(p, c);
       const float ms = time_best();
       if (trace)
         std::fprintf(stderr, "[gnm autotune] tensor %s kernel%s: %.4f ms\n",
-                     (c & 2u) ? ((c & 4u) ? "narrow 8-bit (people as M)" : "narrow (people as M)")
+                     c == people ? "8-bit (people as M)"
+                     : (c & 2u)  ? ((c & 4u) ? "narrow 8-bit (people as M)" : "narrow (people as M)")
                               : ((c & 8u) ? "wide 8-bit on SM pairs (scores as M)"
                                           : ((c & 4u) ? "wide 8-bit (scores as M)"
                                                       : "wide (scores as M)")),
-                     (c & 2u) ? "" : ((c & 1u) ? ", score tiles fastest" : ", people tiles fastest"),
+                     (c & 2u) || c == people ? "" : ((c & 1u) ? ", score tiles fastest" : ", people tiles fastest"),
                      ms);
       if (ms < best_ms) {
         best_ms = ms;
         best = c;
       }
     }
-    tensor_set_narrow(p, (best & 2u) != 0);
-    tensor_set_i8(p, (best & 4u) != 0);
-    tensor_set_pair(p, (best & 8u) != 0);
-    p->raster = best & 1u;
+    tensor_set_shape(p, best);
   }
   plan_reset_impl(p, s);
   sync_impl(p, s);
@@ -1706,10 +1702,7 @@ gnm_status gnm_plan_set_shape(gnm_plan* p, uint32_t shape, gnm_error* err) {
         fail(GNM_ERR_INVALID,
              "tensor engine shape is raster | (narrow << 1) | (8-bit limbs << 2) | "
              "(8-bit wide kernel on SM pairs << 3)");
-      tensor_set_narrow(p, (shape & 2u) != 0);
-      tensor_set_i8(p, (shape & 4u) != 0);
-      tensor_set_pair(p, (shape & 8u) != 0);
-      p->raster = shape & 1u;
+      tensor_set_shape(p, shape);
       return;
     }
     const uint32_t kernel = shape >> 16;
@@ -1735,9 +1728,7 @@ gnm_status gnm_plan_set_shape(gnm_plan* p, uint32_t shape, gnm_error* err) {
 uint32_t gnm_plan_tuned_shape(const gnm_plan* p) {
   if (!p) return 0;
   return p->engine == GNM_ENGINE_PLAIN ? (p->kernel << 16) | std::min<uint32_t>(p->splits, 0xFFFFu)
-                                       : (p->raster | (tensor_is_narrow(p) ? 2u : 0u) |
-                                          (tensor_is_i8(p) ? 4u : 0u) |
-                                          (tensor_is_pair(p) ? 8u : 0u));
+                                       : tensor_shape(p);
 }
 
 gnm_status gnm_decode_device(const uint8_t* d_rows, uint64_t pitch, uint64_t nv, uint64_t np,

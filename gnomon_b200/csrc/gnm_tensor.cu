@@ -4,8 +4,11 @@
 //   gnm_tc_accumulate / gnm_t8_accumulate  wide: scores as M, one SM per tile
 //   gnm_t8_pairs                           wide, 8-bit, SM pairs (cta_group::2),
 //                                          one persistent launch per call
-//   gnm_tc_narrow / gnm_t8_narrow          narrow: people as M (<= 64 scores)
-//   gnm_tc_backward / gnm_t8_backward      dW = G^T dS, dC on CUDA cores
+//   gnm_t8_narrow                          8-bit, people as M: the default for
+//                                          every score count
+//   gnm_tc_narrow                          the same on BF16 limbs (<= 64 scores)
+//   gnm_tc_backward                        dW = G^T dS, dC on CUDA cores
+//   gnm_t8_backward                        dW and dC on the tensor cores (default)
 // The BF16 forms come first below; each 8-bit form states what it changes.
 //
 // Scoring as a GEMM (the reference does this with three cuBLAS SGEMMs per
@@ -71,10 +74,13 @@ struct TensorPlan {
   uint32_t ptiles = 0, stiles = 0;
   __nv_bfloat16* d_planes_dos = nullptr;  // [4][K_pad][V_pad] W' limbs
   __nv_bfloat16* d_planes_mis = nullptr;  // [4][K_pad][V_pad] -corr limbs, member
-  double* d_part_sum = nullptr;           // wide: [K_pad][P_pad]; narrow: [slots][K16][P_nar]
+  double* d_part_sum = nullptr;           // wide kernels: [K_pad][P_pad]
   uint32_t* d_part_cnt = nullptr;
-  uint64_t part_elems = 0;                // elements of d_part_sum / d_part_cnt
+  double* d_slot_sum = nullptr;           // people as M: [slots][K16][P_nar]; up to 64 scores
+  uint32_t* d_slot_cnt = nullptr;         //   the same memory as d_part_sum / d_part_cnt
+  bool slots_used = false;                // over 64 scores: slots written since the last reset
   uint32_t nsplits = 1;                   // narrow BF16: variant splits (grid z)
+  uint32_t nscores = 1;                   // narrow 8-bit: 16-score groups per CTA (narrow_scores)
   uint64_t P_nar = 0;                     // narrow: people rounded up to 512
   uint64_t nslot = 0;                     // narrow: elements per slot (K16 * P_nar)
   uint32_t nalloc = 0;                    // narrow: slots allocated
@@ -90,11 +96,10 @@ struct TensorPlan {
   bool pair = false;                      // ... over SM pairs (gnm_t8_pairs)
   double* d_part_pass = nullptr;          // SM pairs, passes 1-3: [3][K_pad][P_pad]
   bool pass_valid = false;                // d_part_pass written since the last reset
-  bool narrow = false;                    // few scores: gnm_tc_narrow (people as M)
+  bool narrow = false;                    // up to 64 scores: people as M (8-bit or BF16 limbs)
   bool can_narrow = false;                // K <= 64: either kernel can run the plan
   CUtensorMap nmap_dos, nmap_mis;         // narrow boxes: 16 scores x 4 planes
-  CUtensorMap nmap8_dos, nmap8_mis;       // narrow 8-bit boxes: 128 variants x 16 scores x 4 / 5 planes
-  CUtensorMap nmap8_dos2, nmap8_mis2;     // the same with 32 scores
+  CUtensorMap nmap8_dos, nmap8_mis;       // 8-bit boxes: 128 variants x 16 nscores x 4 / 5 planes
 };
 
 struct TcArgs {
@@ -1053,7 +1058,7 @@ __global__ void gnm_t8_build_planes(const float* w, const float* corr, const uin
 // chain of dependent byte loads and permutes set the stage time.  Sums of a
 // 16384-variant block are exact in FP32 (same limb argument) and are added to
 // the FP64 partials of the CTA's variant split in natural person order at
-// block ends; gnm_tc_finalize adds the split slots in a fixed order.
+// block ends; gnm_tc_finalize_slots adds the split slots in a fixed order.
 constexpr uint32_t kNrM = 128;                // people per CTA
 constexpr uint32_t kNrScores = 16;            // scores per CTA
 constexpr uint32_t kNrN = 4 * kNrScores;      // accumulator columns per operand
@@ -1295,8 +1300,8 @@ __global__ void __launch_bounds__(kNrThreads, 1)
   }
 }
 
-// ---- narrow engine on 8-bit limbs -------------------------------------------------
-// Few score columns on tcgen05.mma kind::i8 with people as M: the genotype
+// ---- people as M on 8-bit limbs ---------------------------------------------------
+// Every score count on tcgen05.mma kind::i8 with people as M: the genotype
 // operand A is expanded straight into TENSOR MEMORY, never into shared memory.
 //
 // What bounds it: with A in shared memory (the form this kernel replaced) a
@@ -1870,6 +1875,19 @@ __global__ void gnm_tc_build_planes(const float* w, const float* corr, const uin
 // [3][pass_stride]) in pass order.  Nothing accumulated since the reset
 // (`empty`): the initial value.
 constexpr uint32_t kFinTile = 32;
+
+struct WideSums {          // the wide kernels' partials, sum null without any
+  const double* sum;
+  const uint32_t* cnt;
+  const double* pass;      // passes 1-3 of the SM pairs, or null
+  uint64_t P_pad, pass_stride;
+};
+
+__device__ __forceinline__ uint64_t wide_slot(uint64_t f) {
+  const uint64_t r = f % kTcN, rr = r % 128;
+  return f / kTcN * kTcN + 128 * (r / 128) + 32 * (rr % 4) + rr / 4;
+}
+
 __global__ void __launch_bounds__(256)
     gnm_tc_finalize(const double* part_sum, const uint32_t* part_cnt, uint64_t P_pad,
                     const double* init, const uint32_t* out_to_fam, uint64_t P, uint64_t K,
@@ -1883,8 +1901,7 @@ __global__ void __launch_bounds__(256)
   const uint64_t o = o0 + lane;
   const bool in = o < P && !empty;
   const uint64_t f = !in ? 0 : (out_to_fam ? out_to_fam[o] : o);
-  const uint64_t fr = f % kTcN, h = fr / 128, rr = fr % 128;
-  const uint64_t at = (f / kTcN) * kTcN + 128 * h + 32 * (rr % 4) + rr / 4;
+  const uint64_t at = wide_slot(f);
 #pragma unroll
   for (uint32_t i = 0; i < kPer; ++i) {
     const uint64_t k = k0 + w + 8 * i;
@@ -1918,12 +1935,13 @@ __global__ void __launch_bounds__(256)
 // CTA takes 32 people x 8 scores; two warps share a score, even and odd slots
 // four at a time, so the sum over a small cohort's many slots (48 of them: one
 // per CTA that met the tile) is a few memory latencies, and its order is fixed.
+// `wide` holds what blocks of the same run left in the wide partials.
 constexpr uint32_t kSlotScores = 8, kSlotWarps = 2 * kSlotScores;
 __global__ void __launch_bounds__(32 * kSlotWarps)
     gnm_tc_finalize_slots(const double* part_sum, const uint32_t* part_cnt, uint64_t P_pad,
                           const double* init, const uint32_t* out_to_fam, uint64_t P, uint64_t K,
-                          const uint32_t* state, uint64_t slot_stride, double* sums,
-                          uint32_t* counts) {
+                          const uint32_t* state, uint64_t slot_stride, WideSums wide,
+                          double* sums, uint32_t* counts) {
   __shared__ double s_sum[kSlotWarps][33];
   __shared__ uint32_t s_cnt[kSlotWarps][33];
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
@@ -1943,6 +1961,14 @@ __global__ void __launch_bounds__(32 * kSlotWarps)
           acc[i] += ps[(z + 2 * i) * slot_stride];
           cnt += pc[(z + 2 * i) * slot_stride];
         }
+    }
+    if (wide.sum && part == 0) {
+      const uint64_t at = k * wide.P_pad + wide_slot(f);
+      acc[1] += wide.sum[at];
+      cnt += wide.cnt[at];
+      if (wide.pass)
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) acc[1] += wide.pass[j * wide.pass_stride + at];
     }
   }
   s_sum[w][lane] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
@@ -2287,10 +2313,10 @@ __global__ void __launch_bounds__(kBwThreads, 1)
 //   * gnm_bw_build8 lays dS out in that order of people, so nothing is
 //     transposed; tcgen05.st.32x32b writes 64 people of both operands.
 //
-// Both operands meet the same limbs (two MMAs of N = 64 per 32 people: 37
-// clocks each, the tensor core's floor for M = 128 at these N); the dense
-// missing product costs less than the sparse FP32 sums did and is exact to the
-// limbs.  256 variants per CTA share each limb tile (2 x 128 accumulator
+// Both operands meet the same limbs (two MMAs of N = 64 per 32 people, at least
+// 32 clocks each: 0.22 of the 0.44 ms at 20,000 x 200,000 x 16; the operand ring's
+// latency takes the rest); the dense missing product costs less than the sparse
+// FP32 sums did and is exact to the limbs.  256 variants per CTA share each limb tile (2 x 128 accumulator
 // columns + 256 of operand ring).  CTAs take equal shares of (variant tile,
 // 512-person stage) units; a tile inside one share is written by its CTA, the
 // segments of a tile that spans shares go through FP64 slots that gnm_bw_join
@@ -2960,6 +2986,21 @@ static uint32_t narrow_ctas(const TensorPlan* t, uint64_t K, uint32_t ns) {
   return std::max<uint32_t>(1, uint32_t(t->sms / stiles));
 }
 
+// 16-score groups per CTA.  32 scores halve the CTAs that expand the same rows
+// (20,000 people x 100,000 variants x 32: 337 us on 16, 324 on 32; 20,000 x 40,000
+// x 256: 1123 and 1034), unless 16 pad enough fewer scores per CTA in use: 15 %,
+// the expansion's share (40 scores, 48 against 64 padded: 71 and 77 us at 3,000 x
+// 60,000; 100 scores, 112 against 128: 493 and 484 us at 20,000 x 40,000).
+static uint32_t narrow_scores(const TensorPlan* t, uint64_t K) {
+  if (K <= kNrScores) return 1;
+  double cost[2];
+  for (uint32_t ns : {1u, 2u}) {
+    const uint64_t tiles = (K + kNrScores * ns - 1) / (kNrScores * ns);
+    cost[ns - 1] = double(tiles * ns) / double(tiles * narrow_ctas(t, K, ns));
+  }
+  return 1.15 * cost[0] < cost[1] ? 1 : 2;
+}
+
 void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trace) {
   auto mark = [&](const char* what) {
     if (trace) trace->mark(what);
@@ -2973,9 +3014,9 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   t->P_pad = uint64_t(t->ptiles) * kTcN;
   t->can_narrow = p->K <= kNarrowMaxScores;
   t->narrow = t->can_narrow;
-  // the wide kernel runs on 8-bit limbs unless a shape says otherwise: 1.4x
-  // the BF16 limbs' speed on the batched workload, errors below 2.3e-7 at full
-  // length on every workload
+  // 8-bit limbs unless a shape says otherwise: 1.4x the BF16 limbs' speed in the
+  // wide kernels on the batched workload, errors below 2.3e-7 at full length on
+  // every workload
   t->i8 = true;
   // SM pairs when the plan fills pairs of 128-score tiles (with one tile the
   // pair's second CTA would hold no scores)
@@ -2993,34 +3034,38 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   };
   alloc(reinterpret_cast<void**>(&t->d_planes_dos), 4 * plane * 2, "cudaMalloc(limb planes)");
   alloc(reinterpret_cast<void**>(&t->d_planes_mis), 4 * plane * 2, "cudaMalloc(limb planes)");
-  // partials hold either kernel's layout when both can run the plan (the
-  // autotuner chooses between them)
-  t->part_elems = t->K_pad * t->P_pad;
-  if (t->can_narrow) {
-    const uint64_t k16 = (p->K + kNrScores - 1) / kNrScores * kNrScores;
-    const uint64_t base = ((p->fam + kNrM - 1) / kNrM) * (k16 / kNrScores);
-    int sms = 0;
-    check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device),
-               "cudaDeviceGetAttribute");
+  const uint64_t k16 = (p->K + kNrScores - 1) / kNrScores * kNrScores;
+  const uint64_t base = ((p->fam + kNrM - 1) / kNrM) * (k16 / kNrScores);
+  int sms = 0;
+  check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device),
+             "cudaDeviceGetAttribute");
+  t->P_nar = std::max<uint64_t>(1, (p->fam + 4 * kNrM - 1) / (4 * kNrM)) * (4 * kNrM);
+  t->nslot = k16 * t->P_nar;
+  t->sms = uint32_t(std::max(1, sms));
+  t->d_state = p->d_err + 1;   // cleared with the error word by every reset
+  // a tile of S stages meets at most S / quota + 2 CTAs' shares, and quota >=
+  // ptiles * S / (CTAs per score tile); after whole tiles, quota >= S
+  t->nscores = narrow_scores(t, p->K);
+  const uint64_t people = t->nscores == 2 ? 2 * kNrM : 4 * kNrM;   // of the widest tile in use
+  t->nalloc = narrow_ctas(t, p->K, t->nscores) /
+                  uint32_t(std::max<uint64_t>(1, (p->fam + people - 1) / people)) + 2;
+  uint64_t part_elems = t->K_pad * t->P_pad;
+  if (t->can_narrow) {   // one buffer for either layout: a run uses one of the two
     t->nsplits = narrow_splits(base, t->V_pad / kTcK, std::max(1, sms));
-    t->P_nar = std::max<uint64_t>(1, (p->fam + 4 * kNrM - 1) / (4 * kNrM)) * (4 * kNrM);
-    t->nslot = k16 * t->P_nar;
-    t->sms = uint32_t(std::max(1, sms));
-    // a tile of S stages meets at most S / quota + 2 CTAs' shares, and quota >=
-    // ptiles * S / (CTAs per score tile)
-    const uint32_t ns = p->K > kNrScores ? 2 : 1;
-    const uint64_t people = ns == 2 ? 2 * kNrM : 4 * kNrM;   // of the widest tile in use
-    t->nalloc = std::max(t->nsplits, narrow_ctas(t, p->K, ns) /
-                                         uint32_t(std::max<uint64_t>(1, (p->fam + people - 1) /
-                                                                            people)) + 2);
-    t->part_elems = std::max(t->part_elems, uint64_t(t->nalloc) * t->nslot);
-    t->d_state = p->d_err + 1;   // cleared with the error word by every reset
+    t->nalloc = std::max(t->nalloc, t->nsplits);
+    part_elems = std::max(part_elems, uint64_t(t->nalloc) * t->nslot);
   }
-  alloc(reinterpret_cast<void**>(&t->d_part_sum), t->part_elems * 8, "cudaMalloc(partials)");
-  alloc(reinterpret_cast<void**>(&t->d_part_cnt), t->part_elems * 4, "cudaMalloc(partials)");
-  if (t->pair)   // the SM-pair kernel's passes 1-3 (written before being read)
-    alloc(reinterpret_cast<void**>(&t->d_part_pass), 3 * t->K_pad * t->P_pad * 8,
-          "cudaMalloc(pass partials)");
+  alloc(reinterpret_cast<void**>(&t->d_part_sum), part_elems * 8, "cudaMalloc(partials)");
+  alloc(reinterpret_cast<void**>(&t->d_part_cnt), part_elems * 4, "cudaMalloc(partials)");
+  t->d_slot_sum = t->d_part_sum;
+  t->d_slot_cnt = t->d_part_cnt;
+  if (!t->can_narrow) {   // blocks that start off a 128-variant boundary add to the wide sums
+    const uint64_t n = uint64_t(t->nalloc) * t->nslot;
+    t->d_slot_sum = nullptr;
+    t->d_slot_cnt = nullptr;
+    alloc(reinterpret_cast<void**>(&t->d_slot_sum), n * 8, "cudaMalloc(slots)");
+    alloc(reinterpret_cast<void**>(&t->d_slot_cnt), n * 4, "cudaMalloc(slots)");
+  }
   check_cuda(cudaMemset(t->d_planes_dos, 0, 4 * plane * 2), "memset planes");
   check_cuda(cudaMemset(t->d_planes_mis, 0, 4 * plane * 2), "memset planes");
   t->V_pad8 = std::max<uint64_t>(kT8K, (p->V + kT8K - 1) / kT8K * kT8K);
@@ -3083,14 +3128,10 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   t->map8_1 = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, kTcM, 1);
   t->map_dos = make_plane_map(t->d_planes_dos, t->V_pad, t->K_pad, kTcM, kTcPlanes);
   t->map_mis = make_plane_map(t->d_planes_mis, t->V_pad, t->K_pad, kTcM, kTcPlanes);
-  if (t->can_narrow) {
-    t->nmap_dos = make_plane_map(t->d_planes_dos, t->V_pad, t->K_pad, kNrScores, 4);
-    t->nmap_mis = make_plane_map(t->d_planes_mis, t->V_pad, t->K_pad, kNrScores, 4);
-    t->nmap8_dos = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, kNrScores, 4);
-    t->nmap8_mis = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, kNrScores, 5);
-    t->nmap8_dos2 = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, 2 * kNrScores, 4);
-    t->nmap8_mis2 = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, 2 * kNrScores, 5);
-  }
+  t->nmap_dos = make_plane_map(t->d_planes_dos, t->V_pad, t->K_pad, kNrScores, 4);
+  t->nmap_mis = make_plane_map(t->d_planes_mis, t->V_pad, t->K_pad, kNrScores, 4);
+  t->nmap8_dos = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, kNrScores * t->nscores, 4);
+  t->nmap8_mis = make_plane_map8(t->d_planes8, t->V_pad8, t->K_pad, kNrScores * t->nscores, 5);
 }
 
 void tensor_plan_destroy(gnm_plan* p) {
@@ -3100,6 +3141,10 @@ void tensor_plan_destroy(gnm_plan* p) {
   pool_free(t->d_planes_mis);
   pool_free(t->d_planes8);
   pool_free(t->d_quanta8);
+  if (t->d_slot_sum != t->d_part_sum) {
+    pool_free(t->d_slot_sum);
+    pool_free(t->d_slot_cnt);
+  }
   pool_free(t->d_part_sum);
   pool_free(t->d_part_cnt);
   pool_free(t->d_part_pass);
@@ -3107,25 +3152,44 @@ void tensor_plan_destroy(gnm_plan* p) {
   p->tensor = nullptr;
 }
 
+// The plan's shape is its default one: 8-bit limbs with people as M (score tiles
+// fastest, and over 64 scores the bit of SM pairs where the plan fills them).
+uint32_t tensor_default_shape(const gnm_plan* p) {
+  return p->tensor->can_narrow ? 7u : (p->tensor->stiles >= 2 ? 13u : 5u);
+}
+// gnm_t8_narrow runs the plan's 8-bit blocks: always up to 64 scores when the
+// shape says narrow; over 64 in the default shape (the wide kernels' bits
+// otherwise, below).  Against SM pairs, the better wide kernel: 100,000 people x
+// 40,000 variants x 512 scores 10.5 against 12.2 ms, 50,000 x 100,000 x 512 12.9
+// against 13.3, 8,000 x 40,000 x 512 0.99 against 1.04; with a last score tile to
+// fill, 20,000 x 40,000 x 256, 1.03 against 1.53, 3,000 x 20,000 x 100, 61 against
+// 882 us.
+static bool people_as_m(const gnm_plan* p) {
+  const TensorPlan* t = p->tensor;
+  return t->can_narrow ? t->narrow && t->i8 : tensor_shape(p) == tensor_default_shape(p);
+}
+
 bool tensor_can_narrow(const gnm_plan* p) { return p->tensor && p->tensor->can_narrow; }
-bool tensor_is_narrow(const gnm_plan* p) { return p->tensor && p->tensor->narrow; }
-bool tensor_is_i8(const gnm_plan* p) { return p->tensor && p->tensor->i8; }
-void tensor_set_i8(gnm_plan* p, bool i8) { p->tensor->i8 = i8; }
-bool tensor_is_pair(const gnm_plan* p) { return p->tensor && p->tensor->pair; }
-void tensor_set_pair(gnm_plan* p, bool pair) {
+uint32_t tensor_shape(const gnm_plan* p) {
+  const TensorPlan* t = p->tensor;
+  return p->raster | (t->narrow ? 2u : 0u) | (t->i8 ? 4u : 0u) | (t->pair ? 8u : 0u);
+}
+void tensor_set_shape(gnm_plan* p, uint32_t shape) {
   TensorPlan* t = p->tensor;
-  if (pair && !t->d_part_pass) {   // the pass arrays of the SM-pair kernel, on first use
+  if ((shape & 2u) && !t->can_narrow)
+    fail(GNM_ERR_INVALID, "the narrow tensor kernel serves at most 64 scores");
+  const bool pair = (shape & 8u) != 0;
+  if (pair && !t->d_part_pass && (t->can_narrow || shape != tensor_default_shape(p))) {
+    // the pass arrays of the SM-pair kernel, on first use
     const uint64_t bytes = 3 * t->K_pad * t->P_pad * 8;
     t->d_part_pass = static_cast<double*>(pool_alloc(p->device, bytes, "pass partials"));
     p->device_bytes += bytes;
     t->pass_valid = false;
   }
+  t->narrow = (shape & 2u) != 0;
+  t->i8 = (shape & 4u) != 0;
   t->pair = pair;
-}
-void tensor_set_narrow(gnm_plan* p, bool narrow) {
-  if (narrow && !tensor_can_narrow(p))
-    fail(GNM_ERR_INVALID, "the narrow tensor kernel serves at most 64 scores");
-  p->tensor->narrow = narrow;
+  p->raster = shape & 1u;
 }
 
 // The wide partials start from zero; the narrow engine's slots are written, not
@@ -3140,7 +3204,8 @@ static void clear_wide(TensorPlan* t, cudaStream_t s) {
 void tensor_reset(gnm_plan* p, cudaStream_t s) {
   TensorPlan* t = p->tensor;
   t->wide_clear = false;
-  if (!t->narrow) clear_wide(t, s);
+  t->slots_used = false;
+  if (!t->narrow && !people_as_m(p)) clear_wide(t, s);
   t->pass_valid = false;   // the next SM-pair accumulate writes its pass arrays
 }
 
@@ -3169,7 +3234,7 @@ static void launch_t8_narrow(const gnm_plan* p, const uint8_t* d_rows, uint64_t 
   const dim3 grid(a.rounds ? ncta : uint32_t((units + a.quota - 1) / a.quota),
                   uint32_t((p->K + L::kScores - 1) / L::kScores));
   gnm_t8_narrow<NMT, NS><<<grid, kT8NrThreads, L::kTotal, s>>>(
-      NS == 2 ? t->nmap8_dos2 : t->nmap8_dos, NS == 2 ? t->nmap8_mis2 : t->nmap8_mis, pmap, a);
+      t->nmap8_dos, t->nmap8_mis, pmap, a);
   check_cuda(cudaGetLastError(), "narrow 8-bit tensor launch");
 }
 
@@ -3190,12 +3255,12 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
   TensorPlan* t = p->tensor;
   if (v0 % kTcK != 0)
     fail(GNM_ERR_INVALID, "tensor engine blocks must start at a multiple of 64 variants");
-  if (t->narrow && t->i8 && v0 % kT8K == 0) {
+  if (people_as_m(p) && v0 % kT8K == 0) {
     T8NrArgs a{};
     a.num_rows = nv;
     a.a_x0 = int32_t(v0);
-    a.part_sum = t->d_part_sum;
-    a.part_cnt = t->d_part_cnt;
+    a.part_sum = t->d_slot_sum;
+    a.part_cnt = t->d_slot_cnt;
     a.P_pad = t->P_nar;
     a.slot_stride = t->nslot;
     a.err = p->d_err;
@@ -3204,13 +3269,13 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
     a.quanta = t->d_quanta8;
     a.K_pad = t->K_pad;
     a.K16 = (p->K + kNrScores - 1) / kNrScores * kNrScores;
-    // Over 16 scores: 32 per CTA, so that half as many CTAs expand the same rows.
-    if (p->K > kNrScores)
+    if (t->nscores == 2)
       launch_t8_narrow<2, 2>(p, d_rows, pitch, nv, a, s);
     else if (narrow_small_tiles(narrow_ctas(t, p->K, 1), p->fam, a.stages))
       launch_t8_narrow<2, 1>(p, d_rows, pitch, nv, a, s);
     else
       launch_t8_narrow<4, 1>(p, d_rows, pitch, nv, a, s);
+    t->slots_used = true;
     p->launches += 1;
     return;
   }
@@ -3223,12 +3288,12 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
     a.a_x0 = int32_t(v0);
     const uint32_t nall = uint32_t((nv + kTcK - 1) / kTcK);
     a.stages_per_split = (nall + t->nsplits - 1) / t->nsplits;
-    a.part_sum = t->d_part_sum;
-    a.part_cnt = t->d_part_cnt;
+    a.part_sum = t->d_slot_sum;
+    a.part_cnt = t->d_slot_cnt;
     a.P_pad = t->P_nar;
     a.slot_stride = t->nslot;
     a.err = p->d_err;
-    gnm_tc_open_slots<<<296, 256, 0, s>>>(t->d_part_sum, t->d_part_cnt, t->nslot, t->nsplits,
+    gnm_tc_open_slots<<<296, 256, 0, s>>>(t->d_slot_sum, t->d_slot_cnt, t->nslot, t->nsplits,
                                           t->d_state);
     check_cuda(cudaGetLastError(), "narrow slots launch");
     const dim3 grid(uint32_t((p->fam + kNrM - 1) / kNrM),
@@ -3238,8 +3303,8 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
     p->launches += 2;
     return;
   }
-  if (!t->wide_clear) clear_wide(t, s);   // the reset met a narrow plan
-  if (t->i8 && v0 % kT8K == 0) {
+  if (!t->wide_clear) clear_wide(t, s);   // the reset met a plan that runs people as M
+  if (t->i8 && v0 % kT8K == 0) {   // a pinned wide shape
     // dosage limbs 0-1 and 2-3, correction limbs 0-1 and 2-3, then the counts
     const CUtensorMap pmap8 = make_row_map(d_rows, p->bpv, nv, pitch, kTcN / 4, kT8K);
     T8Args b;
@@ -3334,16 +3399,22 @@ void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_b
   if (n == 0) return;
   const double* init = add_baseline ? p->d_baseline : p->d_zero_base;
   const uint32_t gx = uint32_t((p->P + 31) / 32);
-  if (t->narrow)
+  if (t->narrow || t->slots_used || people_as_m(p)) {
+    // over 64 scores, blocks that ran a wide kernel lie in the wide partials
+    const bool wide = !t->can_narrow && t->wide_clear;
+    const WideSums ws{wide ? t->d_part_sum : nullptr, t->d_part_cnt,
+                      wide && t->pass_valid ? t->d_part_pass : nullptr, t->P_pad,
+                      t->K_pad * t->P_pad};
     gnm_tc_finalize_slots<<<dim3(gx, uint32_t((p->K + kSlotScores - 1) / kSlotScores)),
-                            32 * kSlotWarps, 0, s>>>(t->d_part_sum, t->d_part_cnt, t->P_nar, init,
+                            32 * kSlotWarps, 0, s>>>(t->d_slot_sum, t->d_slot_cnt, t->P_nar, init,
                                                      p->d_out_to_fam, p->P, p->K, t->d_state,
-                                                     t->nslot, d_sums, d_counts);
-  else
+                                                     t->nslot, ws, d_sums, d_counts);
+  } else {
     gnm_tc_finalize<<<dim3(gx, uint32_t((p->K + kFinTile - 1) / kFinTile)), 256, 0, s>>>(
         t->d_part_sum, t->d_part_cnt, t->P_pad, init, p->d_out_to_fam, p->P, p->K,
         t->pass_valid ? t->d_part_pass : nullptr, t->K_pad * t->P_pad, t->wide_clear ? 0u : 1u,
         d_sums, d_counts);
+  }
   check_cuda(cudaGetLastError(), "tensor finalize launch");
   p->launches += 1;
 }

@@ -8,10 +8,10 @@ struct gnm_prep_view;
 
 namespace gnm {
 
-// AUTO picks the tensor engine from this many score columns on: one narrow
-// tensor pass (a 16-score tile) costs about as much as seven single-score plain
-// passes over the same rows (measured on B200: 20,000 x 200,000, 16 scores,
-// 2.25 ms against 16 x 0.33 ms).
+// AUTO picks the tensor engine from this many score columns on.  Its cost alone
+// would put the line lower (20,000 x 200,000: 16 scores take 0.37 ms, one score
+// on the plain engine 0.33); it stays where the plain engine's sums, on another
+// grid, have always ended, so that a call's result does not move.
 constexpr uint64_t kTensorMinScores = 8;
 
 // Smallest row block the end-to-end call splits the tensor engine's rows into.
@@ -22,17 +22,14 @@ struct PhaseTrace;
 void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trace);
 void tensor_plan_destroy(gnm_plan* p);
 void tensor_reset(gnm_plan* p, cudaStream_t s);
-// Up to 64 scores either tensor kernel can run a plan: the narrow one (people
-// as the MMA's M, the default) or the wide one (scores as M).
+// Up to 64 scores a shape chooses between people as the MMA's M (the default)
+// and the wide kernels (scores as M); over 64 see tensor_default_shape.
 bool tensor_can_narrow(const gnm_plan* p);
-bool tensor_is_narrow(const gnm_plan* p);
-void tensor_set_narrow(gnm_plan* p, bool narrow);
-// The wide GEMM on 8-bit limbs (gnm_t8_accumulate) instead of BF16 limbs.
-bool tensor_is_i8(const gnm_plan* p);
-void tensor_set_i8(gnm_plan* p, bool i8);
-// The 8-bit wide GEMM over SM pairs (gnm_t8_pair, cta_group::2).
-bool tensor_is_pair(const gnm_plan* p);
-void tensor_set_pair(gnm_plan* p, bool pair);
+// Shape codes: raster order of the wide kernels | narrow << 1 | 8-bit limbs << 2 |
+// SM pairs << 3 (gnm_plan_set_shape).
+uint32_t tensor_shape(const gnm_plan* p);
+uint32_t tensor_default_shape(const gnm_plan* p);
+void tensor_set_shape(gnm_plan* p, uint32_t shape);
 void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint64_t v0,
                        uint64_t nv, cudaStream_t s);
 void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_baseline,

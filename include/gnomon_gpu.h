@@ -227,11 +227,11 @@ uint64_t gnm_plan_launch_count(const gnm_plan* plan);
  * producer warp; 1024 bytes with 8 warps, with or without one; 2048 bytes
  * with 16 warps and a producer warp) times the variant-split count (0.5x to
  * 8x the SMs' CTA slots, the same count for every people tile);
- * tensor engine: up to 64 scores the narrow kernel (people as the MMA's M)
- * on BF16 and on 8-bit limbs, against the wide kernel (scores as M) on BF16
+ * tensor engine: the kernel with people as the MMA's M on 8-bit limbs and, up
+ * to 64 scores, on BF16 limbs, against the wide kernel (scores as M) on BF16
  * limbs, on 8-bit integer limbs, and on 8-bit limbs over SM pairs (one MMA
- * across the two CTAs of a cluster), each wide form in both CTA raster
- * orders — keeps the fastest, and
+ * across the two CTAs of a cluster), the wide forms in either CTA raster
+ * order — keeps the fastest, and
  * leaves the plan reset.  Blocks until done.  With the environment variable
  * GNM_TRACE set, every candidate's time is printed on stderr. */
 gnm_status gnm_plan_autotune(gnm_plan* plan, const uint8_t* d_rows, uint64_t pitch,
@@ -242,7 +242,9 @@ gnm_status gnm_plan_autotune(gnm_plan* plan, const uint8_t* d_rows, uint64_t pit
  * tensor engine: raster order | (2 if the narrow kernel runs the plan) |
  * (4 if it runs on 8-bit limbs; its blocks then start at multiples of 128
  * variants, others fall back to the BF16 limbs) | (8 if the wide kernel's
- * 8-bit MMAs span SM pairs; only with 4 and without 2). */
+ * 8-bit MMAs span SM pairs; only with 4 and without 2).  Over 64 scores the
+ * shape a plan starts with (13; 5 up to 128 scores) is the 8-bit kernel with
+ * people as M; every other shape with 4 is the wide kernel its bits name. */
 uint32_t gnm_plan_tuned_shape(const gnm_plan* plan);
 
 /* Pin a shape (a value gnm_plan_tuned_shape returned, e.g. saved from an

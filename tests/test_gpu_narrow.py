@@ -102,3 +102,55 @@ def test_whole_tiles_then_shares(cuda, people, variants, scores, blocks):
     _, prep, rows, _ = synth_case(people, variants, scores=scores,
                                   config="batched_100k_x_500k_k512")
     check(prep, rows, run(prep, rows, blocks))
+
+
+def default_run(prep, rows, steps):
+    """Over 64 scores: a plan in its default shape; a step is a block (v0, n) or a
+    shape to continue in.  Two runs, the second over the first one's sums."""
+    V, bpv = rows.shape[0], prep.bytes_per_variant
+    pitch = row_pitch(bpv)
+    d = torch.zeros((V, pitch), dtype=torch.uint8, device="cuda")
+    d[:, :bpv] = torch.from_numpy(np.ascontiguousarray(rows[:, :bpv])).cuda()
+    plan = DevicePlan(prep, engine=_lib.ENGINE_TENSOR)
+    shape = plan.shape
+    assert shape == (13 if prep.num_scores > 128 else 5)
+    for _ in range(2):
+        s, c = plan.outputs()
+        plan.set_shape(shape)
+        plan.reset()
+        for step in steps:
+            if isinstance(step, int):
+                plan.set_shape(step)
+            else:
+                plan.accumulate(d[step[0]:], pitch, *step)
+        plan.finalize(s, c)
+        plan.sync()
+    out = s.cpu().numpy(), c.cpu().numpy().astype(np.uint32)
+    plan.close()
+    return out
+
+
+@pytest.mark.parametrize("people,variants,scores", [
+    (1, 1, 65), (257, 129, 70), (700, 1_000, 97), (513, 385, 128), (5_000, 640, 129),
+    (255, 3_001, 200), (1_025, 300, 257), (12_801, 260, 96), (640, 513, 512), (300, 200, 530)])
+def test_people_as_m_over_64_scores(cuda, people, variants, scores):
+    _, prep, rows, _ = synth_case(people, variants, scores=scores,
+                                  config="batched_100k_x_500k_k512")
+    check(prep, rows, default_run(prep, rows, [(0, variants)]))
+
+
+@pytest.mark.parametrize("scores", [100, 150])
+def test_wide_blocks_in_the_same_run(cuda, scores):
+    """Blocks off a 128-variant boundary, and shapes changed on the way, add to the
+    wide partials; the finalize sums both."""
+    _, prep, rows, _ = synth_case(700, 3_000, scores=scores, config="batched_100k_x_500k_k512")
+    pair = 12
+    for steps in ([(0, 1_024), (1_024, 960), (1_984, 1_016)], [(0, 64), (64, 2_936)],
+                  [(0, 1_024), pair, (1_024, 1_024), 0, (2_048, 952)],
+                  [pair, (0, 1_024), 13 if scores > 128 else 5, (1_024, 1_976)], []):
+        got = default_run(prep, rows, steps)
+        if steps:
+            check(prep, rows, got)
+        else:                            # nothing accumulated: the baseline alone
+            sums = got[0].reshape(700, scores)
+            assert not got[1].any() and (sums == sums[0]).all()
