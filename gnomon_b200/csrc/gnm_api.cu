@@ -334,6 +334,14 @@ static void plain_shape(gnm_plan* p, uint32_t kernel, double mult) {
   p->split_mult = mult;
 }
 
+// The cost of a launch, in stages of one CTA: its waves of CTAs, 0.13 of one more
+// for the CTAs that finish last, times the stages of a CTA and about two for its
+// start and its partials.
+static double plain_cost(uint64_t tiles, uint64_t stages, uint64_t slots, uint64_t splits) {
+  const uint64_t waves = (tiles * splits + slots - 1) / slots;
+  return (double(waves) + 0.13) * (double((stages + splits - 1) / splits) + 2.0);
+}
+
 // The shape of a plan that is not tuned.  512-byte tiles (four scoring warps) for
 // every size: a cohort's last, partly filled tile wastes least, and several CTAs
 // per SM cover each other's waits.  Passes of three scores run best without the
@@ -343,20 +351,42 @@ static void plain_shape(gnm_plan* p, uint32_t kernel, double mult) {
 // under, since one CTA more costs a wave (78 splits of the 15 tiles above: 0.91
 // ms, 83: 0.97), as many as leave about 60 stages in a CTA and at most six, so
 // that uneven CTAs even out (50,000 x 1,000,000 x 1: 3.83 ms at one wave, 3.55
-// at six).  Where one wave has fewer than 12 stages per CTA, one CTA per SM: a
-// CTA's start and its partials would cost more than its stages (2,000 x 50,000:
-// 23 us at 139 splits, 48 us at 592).
+// at six); more where whole tiles leave such a wave part empty and 24 stages
+// remain (123 tiles: four splits fill 0.83 of a wave, nine 0.94 of two).  Where
+// one wave has fewer than 12 stages per CTA, one CTA per SM: a CTA's start and
+// its partials would cost more than its stages (2,000 x 50,000: 23 us at 139
+// splits, 48 us at 592).
+//
+// Two scores share a pass in two launches (accumulate_impl), each in waves of its
+// own, two at least (183,493 x 29,269: 907 us with 6 and 7 splits of 90 tiles, 956
+// with 6 and 6, 783 with 13 and 13), unless one by one costs less than 1.85 times
+// as many stages: a stage of two scores costs 1.6 to 1.9 of one score's (250,000 x
+// 9,000: 394 against 490 us; 20,000 x 50,000: 243 against 208).
 static void plain_shape_default(gnm_plan* p) {
   const uint32_t kernel = p->K >= 3 ? kPlain512 : kPlain512Ws;
   const uint64_t tiles = std::max<uint64_t>(1, (p->bpv + 511) / 512);
   const uint64_t stages = std::max<uint64_t>(1, (p->V + kPlainRows - 1) / kPlainRows);
   const uint64_t slots = uint64_t(plain_ctas_per_sm(kernel)) * uint64_t(p->num_sms);
-  const uint64_t waves =
-      std::min<uint64_t>(6, std::max<uint64_t>(1, (stages * tiles + 30 * slots) / (60 * slots)));
-  const uint64_t splits =
-      waves > 1 ? waves * slots / tiles
-                : std::max(std::min(stages, uint64_t(p->num_sms) / tiles),
-                           std::min(slots / tiles, (stages + 11) / 12));
+  auto fill = [&](uint64_t waves) {
+    const uint64_t s = waves > 1 ? waves * slots / tiles
+                                 : std::max(std::min(stages, uint64_t(p->num_sms) / tiles),
+                                            std::min(slots / tiles, (stages + 11) / 12));
+    return std::max<uint64_t>(1, s);
+  };
+  const uint64_t most = p->K == 2 ? 2 : 6;
+  uint64_t waves = std::max<uint64_t>(1, (stages * tiles + 30 * slots) / (60 * slots));
+  uint64_t splits = fill(std::min(most, waves));
+  for (uint64_t w = 2; w <= most; ++w)
+    if (stages >= 24 * fill(w) && plain_cost(tiles, stages, slots, fill(w)) <
+                                      0.95 * plain_cost(tiles, stages, slots, splits))
+      splits = fill(w);
+  if (p->K == 2) {
+    const uint64_t half = fill(std::min<uint64_t>(3, std::max<uint64_t>(2, (waves + 1) / 2)));
+    if (stages >= 24 * half &&
+        plain_cost(tiles, stages, slots, splits) >
+            1.85 * plain_cost(tiles, (stages + 1) / 2, slots, half))
+      splits = 2 * half;
+  }
   plain_shape_fixed(p, kernel,
                     uint32_t(std::min<uint64_t>(0xFFFFu, std::max<uint64_t>(1, splits))));
 }

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from gnomon_b200 import _lib, synth
+from gnomon_b200.autograd import prep_from_dense
 from gnomon_b200.device import DevicePlan, row_pitch
 from gnomon_b200.prepare import PreparationResult
 from helpers import synth_case
@@ -137,3 +138,36 @@ def test_calls_off_the_stage_grid(cuda):
     prep = uneven(prep, 5, 11)
     blocks = [(0, 100), (100, 511), (611, 389)]
     check(prep, rows, run(prep, rows, 512, 7, blocks), blocks)
+
+
+@pytest.mark.parametrize("people,variants,scores,splits", [
+    (183_493, 20_000, 2, 26),    # two launches of 13 splits, two waves each
+    (183_493, 9_400, 2, 13),     # too few stages for them: one by one
+    (250_001, 6_600, 1, 9)])     # 123 tiles: nine splits fill two waves
+def test_default_shape_of_many_tiles(cuda, people, variants, scores, splits):
+    """The default shape against other splits of the same rows: stage sums are exact,
+    their FP64 sum (<= variants / 30 terms of <= 30 x 2 max|w|) differs in order."""
+    rng = np.random.default_rng(people + variants)
+    w = rng.standard_normal((variants, scores)).astype(np.float32)
+    member = rng.random((variants, scores)) < np.linspace(1.0, 0.2, scores)
+    prep = prep_from_dense(np.where(member, w, 0), rng.random(w.shape) < 0.2, member, people)
+    bpv = prep.bytes_per_variant
+    pitch = row_pitch(bpv)
+    gen = torch.Generator(device="cuda").manual_seed(people)
+    d = torch.randint(0, 256, (variants, pitch), dtype=torch.uint8, device="cuda", generator=gen)
+    if people % 4:                   # padding people are code 00
+        d[:, bpv - 1] &= (1 << 2 * (people % 4)) - 1
+    out = []
+    for pinned in (None, 5):
+        plan = DevicePlan(prep, engine=_lib.ENGINE_PLAIN)
+        if pinned:
+            plan.set_shape((513 << 16) | pinned)
+        else:
+            assert plan.shape == (513 << 16) | splits
+        s, c = plan.score(d, pitch)
+        plan.sync()
+        out.append((s.cpu().numpy(), c.cpu().numpy()))
+        plan.close()
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    np.testing.assert_allclose(out[0][0], out[1][0], rtol=0,
+                               atol=2 * variants / 30 * 2.0**-53 * variants * 2 * np.abs(w).max())
