@@ -84,6 +84,7 @@ struct TensorPlan {
   uint64_t P_nar = 0;                     // narrow: people rounded up to 512
   uint64_t nslot = 0;                     // narrow: elements per slot (K16 * P_nar)
   uint32_t nalloc = 0;                    // narrow: slots allocated
+  uint32_t nslots8 = 0;                   // narrow 8-bit: the most slots a call uses
   uint32_t sms = 1;
   uint32_t* d_state = nullptr;            // narrow: slot state (slots_written)
   bool wide_clear = false;                // wide partials cleared since the last reset
@@ -1869,11 +1870,13 @@ __global__ void gnm_tc_build_planes(const float* w, const float* corr, const uin
 // read a different cache line per thread: 2.02 ms against 0.46 ms on 100,000
 // people x 512 scores, four FP64 arrays and the counts.)
 //
-// Wide engine: one value in operand-row order, slot(f) = tile (f / 256), row
+// People as M: the slots written since the reset (`*state`) in person order, two at
+// a time, four scores a thread (gnm_tc_finalize_slots, one score a thread, took 751
+// us for two slots of 100,000 people x 512 scores, this 361).
+// Wide kernels: one value in operand-row order, slot(f) = tile (f / 256), row
 // 128*h + 32*(r%4) + (r%128)/4 with r = f % 256 and h = r / 128, plus the
 // SM-pair kernel's partials of passes 1-3 (`pass`, may be null:
-// [3][pass_stride]) in pass order.  Nothing accumulated since the reset
-// (`empty`): the initial value.
+// [3][pass_stride]) in pass order.  Neither: the initial value.
 constexpr uint32_t kFinTile = 32;
 
 struct WideSums {          // the wide kernels' partials, sum null without any
@@ -1883,15 +1886,21 @@ struct WideSums {          // the wide kernels' partials, sum null without any
   uint64_t P_pad, pass_stride;
 };
 
+struct SlotSums {          // people as M, sum null without any
+  const double* sum;
+  const uint32_t* cnt;
+  uint64_t P_pad, stride;
+  const uint32_t* state;   // slots written
+};
+
 __device__ __forceinline__ uint64_t wide_slot(uint64_t f) {
   const uint64_t r = f % kTcN, rr = r % 128;
   return f / kTcN * kTcN + 128 * (r / 128) + 32 * (rr % 4) + rr / 4;
 }
 
 __global__ void __launch_bounds__(256)
-    gnm_tc_finalize(const double* part_sum, const uint32_t* part_cnt, uint64_t P_pad,
-                    const double* init, const uint32_t* out_to_fam, uint64_t P, uint64_t K,
-                    const double* pass, uint64_t pass_stride, uint32_t empty, double* sums,
+    gnm_tc_finalize(SlotSums slots, WideSums wide, const double* init,
+                    const uint32_t* out_to_fam, uint64_t P, uint64_t K, double* sums,
                     uint32_t* counts) {
   __shared__ double s_sum[kFinTile][kFinTile + 1];
   __shared__ uint32_t s_cnt[kFinTile][kFinTile + 1];
@@ -1899,23 +1908,43 @@ __global__ void __launch_bounds__(256)
   const uint64_t o0 = uint64_t(blockIdx.x) * kFinTile, k0 = uint64_t(blockIdx.y) * kFinTile;
   constexpr uint32_t kPer = kFinTile / 8;   // scores per warp
   const uint64_t o = o0 + lane;
-  const bool in = o < P && !empty;
-  const uint64_t f = !in ? 0 : (out_to_fam ? out_to_fam[o] : o);
-  const uint64_t at = wide_slot(f);
+  const uint64_t f = o >= P ? 0 : (out_to_fam ? out_to_fam[o] : o);
+  double acc[kPer] = {};
+  uint32_t cnt[kPer] = {};
+  if (slots.sum && o < P) {
+    const uint32_t n = *slots.state;
+    const uint64_t first = (k0 + w) * slots.P_pad + f;
+    for (uint32_t z = 0; z < n; z += 2) {
+#pragma unroll
+      for (uint32_t i = 0; i < kPer; ++i) {
+        if (k0 + w + 8 * i >= K) break;
+        const uint64_t at = z * slots.stride + first + 8 * i * slots.P_pad;
+        acc[i] += slots.sum[at];
+        cnt[i] += slots.cnt[at];
+        if (z + 1 < n) {
+          acc[i] += slots.sum[at + slots.stride];
+          cnt[i] += slots.cnt[at + slots.stride];
+        }
+      }
+    }
+  }
+  if (wide.sum && o < P) {
+    const uint64_t first = (k0 + w) * wide.P_pad + wide_slot(f);
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i) {
+      if (k0 + w + 8 * i >= K) break;
+      const uint64_t at = first + 8 * i * wide.P_pad;
+      acc[i] += wide.sum[at];
+      cnt[i] += wide.cnt[at];
+      if (wide.pass)
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j) acc[i] += wide.pass[j * wide.pass_stride + at];
+    }
+  }
 #pragma unroll
   for (uint32_t i = 0; i < kPer; ++i) {
-    const uint64_t k = k0 + w + 8 * i;
-    double acc = 0.0;
-    uint32_t cnt = 0;
-    if (in && k < K) {
-      acc = part_sum[k * P_pad + at];
-      cnt = part_cnt[k * P_pad + at];
-      if (pass)
-#pragma unroll
-        for (uint32_t j = 0; j < 3; ++j) acc += pass[j * pass_stride + k * P_pad + at];
-    }
-    s_sum[w + 8 * i][lane] = acc;
-    s_cnt[w + 8 * i][lane] = cnt;
+    s_sum[w + 8 * i][lane] = acc[i];
+    s_cnt[w + 8 * i][lane] = cnt[i];
   }
   __syncthreads();
   const uint64_t k = k0 + lane;
@@ -1931,35 +1960,33 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Narrow engine: person order, the slots written since the reset (`*state`).  A
-// CTA takes 32 people x 8 scores; two warps share a score, even and odd slots
+// The same from many slots (a cohort of few people tiles).  A CTA takes 32 people x 8 scores; two warps share a score, even and odd slots
 // four at a time, so the sum over a small cohort's many slots (48 of them: one
 // per CTA that met the tile) is a few memory latencies, and its order is fixed.
 // `wide` holds what blocks of the same run left in the wide partials.
 constexpr uint32_t kSlotScores = 8, kSlotWarps = 2 * kSlotScores;
 __global__ void __launch_bounds__(32 * kSlotWarps)
-    gnm_tc_finalize_slots(const double* part_sum, const uint32_t* part_cnt, uint64_t P_pad,
-                          const double* init, const uint32_t* out_to_fam, uint64_t P, uint64_t K,
-                          const uint32_t* state, uint64_t slot_stride, WideSums wide,
-                          double* sums, uint32_t* counts) {
+    gnm_tc_finalize_slots(SlotSums slots, WideSums wide, const double* init,
+                          const uint32_t* out_to_fam, uint64_t P, uint64_t K, double* sums,
+                          uint32_t* counts) {
   __shared__ double s_sum[kSlotWarps][33];
   __shared__ uint32_t s_cnt[kSlotWarps][33];
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
   const uint64_t o0 = uint64_t(blockIdx.x) * 32, k0 = uint64_t(blockIdx.y) * kSlotScores;
   const uint64_t o = o0 + lane, k = k0 + w % kSlotScores;
-  const uint32_t nslots = *state, part = w / kSlotScores;
+  const uint32_t nslots = *slots.state, part = w / kSlotScores;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   uint32_t cnt = 0;
   if (o < P && k < K) {
     const uint64_t f = out_to_fam ? out_to_fam[o] : o;
-    const double* ps = part_sum + k * P_pad + f;
-    const uint32_t* pc = part_cnt + k * P_pad + f;
+    const double* ps = slots.sum + k * slots.P_pad + f;
+    const uint32_t* pc = slots.cnt + k * slots.P_pad + f;
     for (uint32_t z = part; z < nslots; z += 8) {
 #pragma unroll
       for (uint32_t i = 0; i < 4; ++i)
         if (z + 2 * i < nslots) {
-          acc[i] += ps[(z + 2 * i) * slot_stride];
-          cnt += pc[(z + 2 * i) * slot_stride];
+          acc[i] += ps[(z + 2 * i) * slots.stride];
+          cnt += pc[(z + 2 * i) * slots.stride];
         }
     }
     if (wide.sum && part == 0) {
@@ -3049,6 +3076,7 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   const uint64_t people = t->nscores == 2 ? 2 * kNrM : 4 * kNrM;   // of the widest tile in use
   t->nalloc = narrow_ctas(t, p->K, t->nscores) /
                   uint32_t(std::max<uint64_t>(1, (p->fam + people - 1) / people)) + 2;
+  t->nslots8 = t->nalloc;
   uint64_t part_elems = t->K_pad * t->P_pad;
   if (t->can_narrow) {   // one buffer for either layout: a run uses one of the two
     t->nsplits = narrow_splits(base, t->V_pad / kTcK, std::max(1, sms));
@@ -3399,22 +3427,24 @@ void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_b
   if (n == 0) return;
   const double* init = add_baseline ? p->d_baseline : p->d_zero_base;
   const uint32_t gx = uint32_t((p->P + 31) / 32);
-  if (t->narrow || t->slots_used || people_as_m(p)) {
-    // over 64 scores, blocks that ran a wide kernel lie in the wide partials
-    const bool wide = !t->can_narrow && t->wide_clear;
-    const WideSums ws{wide ? t->d_part_sum : nullptr, t->d_part_cnt,
-                      wide && t->pass_valid ? t->d_part_pass : nullptr, t->P_pad,
-                      t->K_pad * t->P_pad};
+  // over 64 scores, blocks that ran a wide kernel lie in the wide partials
+  const bool slots = t->narrow || t->slots_used || people_as_m(p);
+  const bool wide = t->wide_clear && !(slots && t->can_narrow);
+  const SlotSums ss{slots ? t->d_slot_sum : nullptr, t->d_slot_cnt, t->P_nar, t->nslot,
+                    t->d_state};
+  const WideSums ws{wide ? t->d_part_sum : nullptr, t->d_part_cnt,
+                    t->pass_valid ? t->d_part_pass : nullptr, t->P_pad, t->K_pad * t->P_pad};
+  // Many slots (few people tiles) are summed by more warps per output: 1,503 people x
+  // 30,011 variants x 12, 30 against 41 us for the whole call; four or fewer leave
+  // the 32 x 32 blocks ahead (100,000 x 4,000 x 16: 69 against 81 us; x 512: 1.49
+  // against 1.88 ms).
+  if (slots && t->nslots8 > 4)
     gnm_tc_finalize_slots<<<dim3(gx, uint32_t((p->K + kSlotScores - 1) / kSlotScores)),
-                            32 * kSlotWarps, 0, s>>>(t->d_slot_sum, t->d_slot_cnt, t->P_nar, init,
-                                                     p->d_out_to_fam, p->P, p->K, t->d_state,
-                                                     t->nslot, ws, d_sums, d_counts);
-  } else {
+                            32 * kSlotWarps, 0, s>>>(ss, ws, init, p->d_out_to_fam, p->P, p->K,
+                                                     d_sums, d_counts);
+  else
     gnm_tc_finalize<<<dim3(gx, uint32_t((p->K + kFinTile - 1) / kFinTile)), 256, 0, s>>>(
-        t->d_part_sum, t->d_part_cnt, t->P_pad, init, p->d_out_to_fam, p->P, p->K,
-        t->pass_valid ? t->d_part_pass : nullptr, t->K_pad * t->P_pad, t->wide_clear ? 0u : 1u,
-        d_sums, d_counts);
-  }
+        ss, ws, init, p->d_out_to_fam, p->P, p->K, d_sums, d_counts);
   check_cuda(cudaGetLastError(), "tensor finalize launch");
   p->launches += 1;
 }

@@ -139,11 +139,11 @@ def test_people_as_m_over_64_scores(cuda, people, variants, scores):
     check(prep, rows, default_run(prep, rows, [(0, variants)]))
 
 
-@pytest.mark.parametrize("scores", [100, 150])
-def test_wide_blocks_in_the_same_run(cuda, scores):
+@pytest.mark.parametrize("people,scores", [(700, 100), (700, 150), (9_500, 150)])
+def test_wide_blocks_in_the_same_run(cuda, people, scores):
     """Blocks off a 128-variant boundary, and shapes changed on the way, add to the
     wide partials; the finalize sums both."""
-    _, prep, rows, _ = synth_case(700, 3_000, scores=scores, config="batched_100k_x_500k_k512")
+    _, prep, rows, _ = synth_case(people, 3_000, scores=scores, config="batched_100k_x_500k_k512")
     pair = 12
     for steps in ([(0, 1_024), (1_024, 960), (1_984, 1_016)], [(0, 64), (64, 2_936)],
                   [(0, 1_024), pair, (1_024, 1_024), 0, (2_048, 952)],
@@ -152,5 +152,5 @@ def test_wide_blocks_in_the_same_run(cuda, scores):
         if steps:
             check(prep, rows, got)
         else:                            # nothing accumulated: the baseline alone
-            sums = got[0].reshape(700, scores)
+            sums = got[0].reshape(people, scores)
             assert not got[1].any() and (sums == sums[0]).all()
