@@ -1884,7 +1884,28 @@ struct WideSums {          // the wide kernels' partials, sum null without any
   const uint32_t* cnt;
   const double* pass;      // passes 1-3 of the SM pairs, or null
   uint64_t P_pad, pass_stride;
+  const uint32_t* opened;  // null, or zero while nothing was added (gnm_tc_open_wide)
 };
+
+// Zeroes the wide partials before the first block that adds to them since the
+// reset, on a plan whose reset does not: state[2] says whether one did, so that
+// captured blocks may replay in any order.
+__global__ void gnm_tc_open_wide(double* sum, uint32_t* cnt, uint64_t n, uint32_t* state) {
+  if (!*reinterpret_cast<volatile uint32_t*>(state + 2))
+    for (uint64_t x = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < n;
+         x += uint64_t(gridDim.x) * blockDim.x) {
+      sum[x] = 0.0;
+      cnt[x] = 0u;
+    }
+  __syncthreads();
+  if (threadIdx.x == 0) {   // every CTA has read the flag once the last one counts
+    __threadfence();
+    if (atomicAdd(state + 1, 1u) + 1 == gridDim.x) {
+      state[1] = 0u;
+      state[2] = 1u;
+    }
+  }
+}
 
 struct SlotSums {          // people as M, sum null without any
   const double* sum;
@@ -1928,7 +1949,7 @@ __global__ void __launch_bounds__(256)
       }
     }
   }
-  if (wide.sum && o < P) {
+  if (wide.sum && o < P && (!wide.opened || *wide.opened)) {
     const uint64_t first = (k0 + w) * wide.P_pad + wide_slot(f);
 #pragma unroll
     for (uint32_t i = 0; i < kPer; ++i) {
@@ -1989,7 +2010,7 @@ __global__ void __launch_bounds__(32 * kSlotWarps)
           cnt += pc[(z + 2 * i) * slots.stride];
         }
     }
-    if (wide.sum && part == 0) {
+    if (wide.sum && part == 0 && (!wide.opened || *wide.opened)) {
       const uint64_t at = k * wide.P_pad + wide_slot(f);
       acc[1] += wide.sum[at];
       cnt += wide.cnt[at];
@@ -3331,7 +3352,16 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
     p->launches += 2;
     return;
   }
-  if (!t->wide_clear) clear_wide(t, s);   // the reset met a plan that runs people as M
+  if (!t->wide_clear) {   // the reset met a plan that runs people as M
+    if (t->can_narrow) {
+      clear_wide(t, s);
+    } else {
+      gnm_tc_open_wide<<<296, 256, 0, s>>>(t->d_part_sum, t->d_part_cnt, t->K_pad * t->P_pad,
+                                           t->d_state);
+      check_cuda(cudaGetLastError(), "wide partials launch");
+      p->launches += 1;
+    }
+  }
   if (t->i8 && v0 % kT8K == 0) {   // a pinned wide shape
     // dosage limbs 0-1 and 2-3, correction limbs 0-1 and 2-3, then the counts
     const CUtensorMap pmap8 = make_row_map(d_rows, p->bpv, nv, pitch, kTcN / 4, kT8K);
@@ -3429,11 +3459,12 @@ void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_b
   const uint32_t gx = uint32_t((p->P + 31) / 32);
   // over 64 scores, blocks that ran a wide kernel lie in the wide partials
   const bool slots = t->narrow || t->slots_used || people_as_m(p);
-  const bool wide = t->wide_clear && !(slots && t->can_narrow);
+  const bool wide = t->can_narrow ? t->wide_clear && !slots : true;
   const SlotSums ss{slots ? t->d_slot_sum : nullptr, t->d_slot_cnt, t->P_nar, t->nslot,
                     t->d_state};
   const WideSums ws{wide ? t->d_part_sum : nullptr, t->d_part_cnt,
-                    t->pass_valid ? t->d_part_pass : nullptr, t->P_pad, t->K_pad * t->P_pad};
+                    t->pass_valid ? t->d_part_pass : nullptr, t->P_pad, t->K_pad * t->P_pad,
+                    t->wide_clear ? nullptr : t->d_state + 2};
   // Many slots (few people tiles) are summed by more warps per output: 1,503 people x
   // 30,011 variants x 12, 30 against 41 us for the whole call; four or fewer leave
   // the 32 x 32 blocks ahead (100,000 x 4,000 x 16: 69 against 81 us; x 512: 1.49

@@ -154,3 +154,32 @@ def test_wide_blocks_in_the_same_run(cuda, people, scores):
         else:                            # nothing accumulated: the baseline alone
             sums = got[0].reshape(people, scores)
             assert not got[1].any() and (sums == sums[0]).all()
+
+
+def test_captured_wide_blocks_replay_in_any_order(cuda):
+    """Over 64 scores: blocks off a 128-variant boundary, each captured by itself,
+    replayed in both orders after a reset outside the graphs."""
+    _, prep, rows, _ = synth_case(700, 1_000, scores=100, config="batched_100k_x_500k_k512")
+    pitch = row_pitch(prep.bytes_per_variant)
+    d = torch.zeros((1_000, pitch), dtype=torch.uint8, device="cuda")
+    d[:, :prep.bytes_per_variant] = torch.from_numpy(rows[:, :prep.bytes_per_variant]).cuda()
+    plan = DevicePlan(prep, engine=_lib.ENGINE_TENSOR)
+    s, c = plan.outputs()
+    graphs = []
+    for v0, n in ((0, 64), (64, 256), (320, 680)):
+        plan.reset()
+        torch.cuda.synchronize()
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            plan.accumulate(d[v0:], pitch, v0, n, torch.cuda.current_stream())
+    for order in ((0, 1, 2), (2, 1, 0)):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            stream = torch.cuda.current_stream()
+            plan.reset(stream)
+            for g in order:
+                graphs[g].replay()
+            plan.finalize(s, c, stream)
+            plan.sync(stream)
+        check(prep, rows, (s.cpu().numpy(), c.cpu().numpy().astype(np.uint32)))
+    del graphs
+    plan.close()
