@@ -474,9 +474,10 @@ def gpu_arm(args, rank, world, local_rank):
         # over 256-person x 128-score tiles (256-score tiles on SM pairs) and
         # 128-variant stages; the integer peak is taken as twice the BF16 one
         # (the nominal dense ratio, 4.5 / 2.25)
-        # (in the shape a plan starts with, 13 or 5, people are the M: 256 people x
-        # 32 scores, 5 + 4 planes)
-        people_m = tshape == (13 if K > 128 else 5) and K > 64
+        # (in the shape a plan starts with, 13 or 5, people are the M, 256 people x
+        # 32 scores, unless over 1 GB of limbs nearly fill tiles of 256 scores)
+        people_m = K > 64 and tshape == (13 if K > 128 else 5) and (
+            9 * K * V <= 1 << 30 or 20 * (-(-K // 256) * 256) > 23 * K)
         mt = 32 if people_m else 256 if tshape & 8 else 128
         ptiles, kpad, vpad = -(-P // 256), -(-K // mt) * mt, -(-V // 128) * 128
         executed = 2.0 * ptiles * 256 * vpad * kpad * 9

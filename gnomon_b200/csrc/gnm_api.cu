@@ -792,7 +792,8 @@ static void autotune_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, ui
     // shape bit 0: raster order of the wide kernel; bit 1: the narrow kernel;
     // bit 2: 8-bit limbs; bit 3: the 8-bit wide kernel over SM pairs.  Over 64
     // scores the plan's first shape (13; 5 up to 128 scores) runs people as M
-    const uint32_t people = tensor_default_shape(p);
+    // unless its limbs are large (prefers_people)
+    const uint32_t people = tensor_people_shape(p);
     std::vector<uint32_t> cand = {0u, 1u, 4u, 5u, 12u, 13u};
     if (tensor_can_narrow(p)) cand.insert(cand.begin(), {2u, 6u});
     uint32_t best = tensor_shape(p);

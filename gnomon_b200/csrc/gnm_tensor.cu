@@ -99,6 +99,7 @@ struct TensorPlan {
   bool pass_valid = false;                // d_part_pass written since the last reset
   bool narrow = false;                    // up to 64 scores: people as M (8-bit or BF16 limbs)
   bool can_narrow = false;                // K <= 64: either kernel can run the plan
+  bool people = false;                    // the default shape runs people as M
   CUtensorMap nmap_dos, nmap_mis;         // narrow boxes: 16 scores x 4 planes
   CUtensorMap nmap8_dos, nmap8_mis;       // 8-bit boxes: 128 variants x 16 nscores x 4 / 5 planes
 };
@@ -3049,6 +3050,18 @@ static uint32_t narrow_scores(const TensorPlan* t, uint64_t K) {
   return 1.15 * cost[0] < cost[1] ? 1 : 2;
 }
 
+// Over 64 scores: people as M against SM pairs, the better wide kernel.  100,000
+// people x 40,000 variants x 512 scores 10.4 against 12.2 ms, x 150,000 37-38
+// against 39.4 ms, 8,000 x 40,000 x 512 0.99 against 1.04; with a last score tile
+// to fill, 20,000 x 40,000 x 256, 1.03 against 1.53, 3,000 x 20,000 x 100, 61 against
+// 882 us.  At 100,000 x 500,000 x 512 the 2.3 GB of limbs stream through L2 once per
+// round of people tiles and the board throttles: 136-145 against 128-130 ms.  So
+// pairs keep plans of over 1 GB of limbs whose scores nearly fill their 256.
+static bool prefers_people(const gnm_plan* p) {
+  const uint64_t limbs = kT8Planes * p->K * p->V;
+  return limbs <= (uint64_t(1) << 30) || 20 * ((p->K + 255) / 256 * 256) > 23 * p->K;
+}
+
 void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trace) {
   auto mark = [&](const char* what) {
     if (trace) trace->mark(what);
@@ -3062,6 +3075,7 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   t->P_pad = uint64_t(t->ptiles) * kTcN;
   t->can_narrow = p->K <= kNarrowMaxScores;
   t->narrow = t->can_narrow;
+  t->people = t->can_narrow || prefers_people(p);
   // 8-bit limbs unless a shape says otherwise: 1.4x the BF16 limbs' speed in the
   // wide kernels on the batched workload, errors below 2.3e-7 at full length on
   // every workload
@@ -3108,7 +3122,11 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   alloc(reinterpret_cast<void**>(&t->d_part_cnt), part_elems * 4, "cudaMalloc(partials)");
   t->d_slot_sum = t->d_part_sum;
   t->d_slot_cnt = t->d_part_cnt;
-  if (!t->can_narrow) {   // blocks that start off a 128-variant boundary add to the wide sums
+  if (!t->people) {   // SM pairs' passes 1-3 (written before being read)
+    if (t->pair)
+      alloc(reinterpret_cast<void**>(&t->d_part_pass), 3 * t->K_pad * t->P_pad * 8,
+            "cudaMalloc(pass partials)");
+  } else if (!t->can_narrow) {   // blocks that start off a 128-variant boundary add to the wide sums
     const uint64_t n = uint64_t(t->nalloc) * t->nslot;
     t->d_slot_sum = nullptr;
     t->d_slot_cnt = nullptr;
@@ -3206,16 +3224,16 @@ void tensor_plan_destroy(gnm_plan* p) {
 uint32_t tensor_default_shape(const gnm_plan* p) {
   return p->tensor->can_narrow ? 7u : (p->tensor->stiles >= 2 ? 13u : 5u);
 }
-// gnm_t8_narrow runs the plan's 8-bit blocks: always up to 64 scores when the
-// shape says narrow; over 64 in the default shape (the wide kernels' bits
-// otherwise, below).  Against SM pairs, the better wide kernel: 100,000 people x
-// 40,000 variants x 512 scores 10.5 against 12.2 ms, 50,000 x 100,000 x 512 12.9
-// against 13.3, 8,000 x 40,000 x 512 0.99 against 1.04; with a last score tile to
-// fill, 20,000 x 40,000 x 256, 1.03 against 1.53, 3,000 x 20,000 x 100, 61 against
-// 882 us.
+uint32_t tensor_people_shape(const gnm_plan* p) {
+  return p->tensor->people ? tensor_default_shape(p) : ~0u;
+}
+// gnm_t8_narrow runs the plan's 8-bit blocks: up to 64 scores when the shape says
+// narrow, over 64 in the default shape (the wide kernels' bits otherwise, below) of
+// a plan that prefers_people.
 static bool people_as_m(const gnm_plan* p) {
   const TensorPlan* t = p->tensor;
-  return t->can_narrow ? t->narrow && t->i8 : tensor_shape(p) == tensor_default_shape(p);
+  return t->can_narrow ? t->narrow && t->i8
+                       : t->people && tensor_shape(p) == tensor_default_shape(p);
 }
 
 bool tensor_can_narrow(const gnm_plan* p) { return p->tensor && p->tensor->can_narrow; }
@@ -3228,7 +3246,7 @@ void tensor_set_shape(gnm_plan* p, uint32_t shape) {
   if ((shape & 2u) && !t->can_narrow)
     fail(GNM_ERR_INVALID, "the narrow tensor kernel serves at most 64 scores");
   const bool pair = (shape & 8u) != 0;
-  if (pair && !t->d_part_pass && (t->can_narrow || shape != tensor_default_shape(p))) {
+  if (pair && !t->d_part_pass && !(t->people && shape == tensor_default_shape(p))) {
     // the pass arrays of the SM-pair kernel, on first use
     const uint64_t bytes = 3 * t->K_pad * t->P_pad * 8;
     t->d_part_pass = static_cast<double*>(pool_alloc(p->device, bytes, "pass partials"));

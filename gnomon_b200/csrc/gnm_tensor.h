@@ -29,6 +29,8 @@ bool tensor_can_narrow(const gnm_plan* p);
 // SM pairs << 3 (gnm_plan_set_shape).
 uint32_t tensor_shape(const gnm_plan* p);
 uint32_t tensor_default_shape(const gnm_plan* p);
+// The shape that runs people as M, or ~0 where none does over 64 scores.
+uint32_t tensor_people_shape(const gnm_plan* p);
 void tensor_set_shape(gnm_plan* p, uint32_t shape);
 void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint64_t v0,
                        uint64_t nv, cudaStream_t s);

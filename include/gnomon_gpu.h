@@ -244,7 +244,9 @@ gnm_status gnm_plan_autotune(gnm_plan* plan, const uint8_t* d_rows, uint64_t pit
  * variants, others fall back to the BF16 limbs) | (8 if the wide kernel's
  * 8-bit MMAs span SM pairs; only with 4 and without 2).  Over 64 scores the
  * shape a plan starts with (13; 5 up to 128 scores) is the 8-bit kernel with
- * people as M; every other shape with 4 is the wide kernel its bits name. */
+ * people as M, or SM pairs for over 1 GB of limbs (9 bytes per variant and
+ * score) that nearly fill tiles of 256 scores; every other shape with 4 is the
+ * wide kernel its bits name. */
 uint32_t gnm_plan_tuned_shape(const gnm_plan* plan);
 
 /* Pin a shape (a value gnm_plan_tuned_shape returned, e.g. saved from an
