@@ -331,7 +331,6 @@ static void plain_shape(gnm_plan* p, uint32_t kernel, double mult) {
   const uint64_t tiles = std::max<uint64_t>(1, (p->bpv + tile_bytes - 1) / tile_bytes);
   const double ctas = double(plain_ctas_per_sm(kernel)) * double(p->num_sms) * mult;
   plain_shape_fixed(p, kernel, uint32_t(std::max(1.0, std::floor(ctas / double(tiles)))));
-  p->split_mult = mult;
 }
 
 // The cost of a launch, in stages of one CTA: its waves of CTAs, 0.13 of one more
@@ -627,6 +626,8 @@ static void accumulate_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, 
   // launch after a reset writes them; a later one adds, after clearing any
   // slots past those written so far.
   const uint32_t covered = uint32_t((stages + sps - 1) / sps);
+  if (covered > p->splits_alloc)
+    fail(GNM_ERR_COMPUTE, "plain engine: more partial slots than allocated");
   const bool store = p->valid_slots == 0;
   if (!store && covered > p->valid_slots) {
     const uint64_t row = uint64_t(p->splits_alloc) * p->part_stride;
@@ -765,29 +766,32 @@ static void autotune_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, ui
   };
   float best_ms = 1e30f;
   if (p->engine == GNM_ENGINE_PLAIN) {
-    uint32_t best_kernel = p->kernel;
-    double best_mult = p->split_mult;
-    p->tuning_log.clear();
+    // The shape the plan has is the first candidate, so there always is one: of a
+    // plan with many scores, whose partials are capped, every other may need more
+    // slots than are allocated.
+    uint32_t best_kernel = p->kernel, best_splits = p->splits;
     const char* tr = std::getenv("GNM_TRACE");
     const bool trace = tr && std::strcmp(tr, "0") != 0;
+    auto candidate = [&] {
+      const float ms = time_best();
+      if (trace)
+        std::fprintf(stderr, "[gnm autotune] tile %u B%s, %u splits: %.4f ms\n",
+                     plain_tile_bytes(p->kernel), (p->kernel & 1u) ? " + producer warp" : "",
+                     p->splits, ms);
+      if (ms < best_ms) {
+        best_ms = ms;
+        best_kernel = p->kernel;
+        best_splits = p->splits;
+      }
+    };
+    candidate();
     for (uint32_t kn : kPlainKernels) {
       for (double m : kPlainSplitMults) {
         plain_shape(p, kn, m);
-        if (p->slots > p->splits_alloc) continue;
-        const float ms = time_best();
-        p->tuning_log.push_back({kn, m, p->splits, p->last_splits, ms});
-        if (trace)
-          std::fprintf(stderr, "[gnm autotune] tile %u B%s, %.1fx slots: %u splits (last tile "
-                               "%u), %.4f ms\n", plain_tile_bytes(kn),
-                       (kn & 1u) ? " + producer warp" : "", m, p->splits, p->last_splits, ms);
-        if (ms < best_ms) {
-          best_ms = ms;
-          best_kernel = kn;
-          best_mult = m;
-        }
+        if (p->slots <= p->splits_alloc) candidate();
       }
     }
-    plain_shape(p, best_kernel, best_mult);
+    plain_shape_fixed(p, best_kernel, best_splits);
   } else {
     // shape bit 0: raster order of the wide kernel; bit 1: the narrow kernel;
     // bit 2: 8-bit limbs; bit 3: the 8-bit wide kernel over SM pairs.  Over 64

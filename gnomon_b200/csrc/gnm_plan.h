@@ -132,7 +132,6 @@ struct gnm_plan {
 
   // plain engine
   uint32_t kernel = 1024;      // plain accumulate kernel (gnm_internal.h kPlain*)
-  double split_mult = 1.0;     // CTA slots per SM multiplier the split counts are sized for
   uint32_t tiles = 0;          // people tiles of the kernel's width
   uint32_t splits = 0;         // variant splits of each full tile
   uint32_t last_splits = 0;    // variant splits of the last (partly populated) tile
@@ -141,13 +140,6 @@ struct gnm_plan {
   uint32_t splits_alloc = 0;   // partial slots allocated per score (autotune range)
   uint32_t raster = 0;         // tensor engine CTA order: 0 people-tile fastest, 1 score-tile
   uint64_t part_stride = 0;    // people per partial slot (bpv rounded up to 2048 bytes, x4)
-  struct Tuning {              // one autotuner candidate and its best accumulate time
-    uint32_t kernel;
-    double mult;
-    uint32_t splits, last_splits;
-    float ms;
-  };
-  std::vector<Tuning> tuning_log;
   uint64_t rec_stride = 0;     // records per score (V + pad)
   float4* d_records = nullptr; // [K][rec_stride]
   uint8_t* d_tables = nullptr;  // stage tables of every score, [K][tab_stages][kPlainTableBytes]

@@ -226,7 +226,8 @@ uint64_t gnm_plan_launch_count(const gnm_plan* plan);
  * the kernel (people tiles of 512 bytes with 4 warps, with or without a
  * producer warp; 1024 bytes with 8 warps, with or without one; 2048 bytes
  * with 16 warps and a producer warp) times the variant-split count (0.5x to
- * 8x the SMs' CTA slots, the same count for every people tile);
+ * 8x the SMs' CTA slots, the same count for every people tile), as far as the
+ * plan's partial slots hold them, and the shape the plan has;
  * tensor engine: the kernel with people as the MMA's M on 8-bit limbs and, up
  * to 64 scores, on BF16 limbs, against the wide kernel (scores as M) on BF16
  * limbs, on 8-bit integer limbs, and on 8-bit limbs over SM pairs (one MMA
