@@ -642,11 +642,12 @@ static void accumulate_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, 
   }
   p->valid_slots = std::max(p->valid_slots, covered);
   // Passes of kPlainPassScores scores, the rest in a last one.  Two scores share a
-  // pass in two launches, each over half of the splits (callers count one
-  // accumulate and one finalize launch per score up to two scores); where half
-  // of the splits do not fill the SMs they go one by one.
+  // pass in two launches, each over half of the splits (so a call of up to two
+  // scores counts one accumulate launch per score whatever its size); where half
+  // of the splits do not fill the SMs, or there is only one, they go one by one.
   const uint64_t half_ctas = uint64_t(p->tiles) * covered / 2;
-  const bool halves = p->K == 2 && half_ctas >= uint64_t(p->num_sms) * plain_ctas_per_sm(p->kernel);
+  const bool halves = p->K == 2 && covered >= 2 &&
+                      half_ctas >= uint64_t(p->num_sms) * plain_ctas_per_sm(p->kernel);
   const uint32_t pass = p->K == 2 && !halves ? 1u : kPlainPassScores;
   for (uint64_t k = 0; k < p->K;) {
     const uint32_t n = uint32_t(std::min<uint64_t>(pass, p->K - k));
@@ -655,7 +656,6 @@ static void accumulate_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, 
     a.num_rows = nv;
     a.bytes_per_row = p->bpv;
     a.tiles = p->tiles;
-    a.splits = uint32_t((stages + sps - 1) / sps);   // non-empty splits of a full tile
     a.stages_per_split = sps;
     a.score_stride = uint64_t(p->splits_alloc) * p->part_stride;
     a.part_sum = p->d_part_sum + k * a.score_stride;
@@ -663,11 +663,10 @@ static void accumulate_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, 
     a.part_stride = p->part_stride;
     a.err = p->d_err;
     a.store = store ? 1u : 0u;
-    const uint32_t all = a.splits;
     const uint32_t parts = halves ? 2 : 1;
     for (uint32_t h = 0; h < parts; ++h) {
-      a.split0 = h * (all / 2);
-      a.splits = h + 1 < parts ? all / 2 : all - a.split0;
+      a.split0 = h * (covered / 2);
+      a.splits = h + 1 < parts ? covered / 2 : covered - a.split0;
       check_cuda(launch_plain_accumulate(map, a, p->kernel, n, s), "plain accumulate launch");
       ++p->launches;
     }
