@@ -2403,27 +2403,116 @@ struct Bw8Args {
   uint32_t vtiles;         // 256-variant tiles
   uint32_t quota;          // (variant tile, stage) units per CTA
   const double* quanta;    // [4][K16]
+  const uint32_t* sparse;  // [K16] scores whose C bw_missing_terms writes
   double* part;            // [score tiles][CTAs][2][G, C][256][16]: a CTA's first / last segment
   float* gw;
   float* gc;               // may be null (CORR false)
   uint32_t* err;
-  const uint8_t* rows;     // packed rows and FP32 dS [people][K]: non-finite scores
+  const uint8_t* rows;     // packed rows and FP32 dS [people][K], for those
   uint64_t pitch;
   const float* ds;
   uint64_t people;
 };
 
-// The missing term of one variant over people [p0, p1) of a score whose largest
-// |dS| is an infinity or NaN, which limbs cannot hold: the sum of the dS values
-// themselves, so that only variants at which such a person is missing get one.
-// (`row`: the variant's packed row, `ds`: the score's column of dS, `K` apart.)
-__device__ __noinline__ double bw_missing_sum(const uint8_t* row, const float* ds, uint64_t K,
-                                              uint64_t p0, uint64_t p1) {
-  double s = 0.0;
-  for (uint64_t p = p0; p < p1; ++p)
-    if (((row[p / 4] >> (2 * (p % 4))) & 3u) == 1u) s += double(ds[p * K]);
-  return s;
+// The missing term of the scores of a tile that the limbs cannot hold (`sparse`):
+// C[v, k] = -(sum of the dS values of the people missing at v), in FP64.  Every warp
+// of the CTA takes variants of its own once the CTA's share of the products is
+// done; these entries of C are written here alone.
+//
+// Latency bounds it (20 warps per SM): a lane reads 64 people's codes two steps
+// ahead, a scan places the missing ones in the warp's list, and when that holds 256
+// or the row ends, lanes take (person, score) pairs, 16 consecutive scores of two
+// people, 16 values each in flight.  20,000 people x 20,000 variants x 16 scores,
+// every dS a NaN: 0.21 ms for the whole step (25.1 with one thread per variant and
+// score walking all people, 0.09 with finite scores); x 200,000: 1.56 ms (0.44).
+constexpr uint32_t kBwList = 256 + 2048;
+__device__ __noinline__ void bw_missing_terms(const uint8_t* rows, uint64_t pitch, uint64_t people,
+                                              uint64_t V, const float* ds, uint32_t K,
+                                              const uint32_t* sparse, uint64_t k0, uint32_t warp,
+                                              uint32_t warps, uint32_t* list, float* gc) {
+  const uint32_t lane = threadIdx.x & 31u, half = lane >> 4;
+  const uint64_t k = k0 + (lane & 15u);
+  const bool on = k < K && sparse[k] != 0u;
+  if (!__any_sync(0xFFFFFFFFu, on)) return;
+  const uint64_t bytes = (people + 3) / 4, step = uint64_t(gridDim.x) * warps;
+  const uint32_t chunks = uint32_t((people + 2047) / 2048);
+  const float* col = ds + k;
+  // (variant, 2,048-person chunk) to load next, two ahead of the one in work
+  uint64_t lv = uint64_t(blockIdx.x) * warps + warp;
+  uint32_t lc = 0;
+  auto load = [&] {   // this lane's 64 people
+    const uint8_t* row = rows + lv * pitch;
+    const uint64_t b0 = 512 * uint64_t(lc) + 16 * lane;
+    uint4 q = make_uint4(0u, 0u, 0u, 0u);
+    // rows start 16-byte aligned, and all but the last one's padding may be read
+    if (lv < V && (b0 + 16 <= bytes || (b0 < bytes && lv + 1 < V))) {
+      q = *reinterpret_cast<const uint4*>(row + b0);
+    } else if (lv < V && b0 < bytes) {
+      uint32_t x[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (uint32_t b = 0; b < 16; ++b)
+        if (b0 + b < bytes) x[b / 4] |= uint32_t(row[b0 + b]) << (8 * (b % 4));
+      q = make_uint4(x[0], x[1], x[2], x[3]);
+    }
+    if (++lc == chunks) {
+      lc = 0;
+      lv += step;
+    }
+    return q;
+  };
+  uint4 q0 = load(), q1 = load();
+  for (uint64_t v = uint64_t(blockIdx.x) * warps + warp; v < V; v += step) {
+    double acc = 0.0;
+    uint32_t held = 0;
+    for (uint32_t c = 0; c < chunks; ++c) {
+      uint32_t m[4] = {q0.x, q0.y, q0.z, q0.w};
+      q0 = q1;
+      q1 = load();
+      const uint64_t p0 = 2048 * uint64_t(c) + 64 * lane;
+      uint32_t mine = 0;
+#pragma unroll
+      for (uint32_t w = 0; w < 4; ++w) {
+        m[w] &= ~(m[w] >> 1) & 0x55555555u;
+        const uint64_t p = p0 + 16 * w;        // padding past the last person may be code 01
+        if (p + 16 > people) m[w] &= p < people ? (1u << (2 * uint32_t(people - p))) - 1u : 0u;
+        mine += __popc(m[w]);
+      }
+      uint32_t at = mine;
+#pragma unroll
+      for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, d);
+        if (lane >= d) at += y;
+      }
+      const uint32_t total = __shfl_sync(0xFFFFFFFFu, at, 31);
+      at += held - mine;
+#pragma unroll
+      for (uint32_t w = 0; w < 4; ++w)
+        for (uint32_t x = m[w]; x; x &= x - 1)
+          list[at++] = uint32_t(p0) + 16 * w + (__ffs(x) - 1) / 2;
+      held += total;
+      if (held < 256 && c + 1 < chunks) continue;
+      __syncwarp();
+      for (uint32_t i = half; i < held; i += 32) {
+        uint32_t p[16];
+        float f[16];
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) p[j] = list[min(i + 2 * j, held - 1)];
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j)
+          f[j] = on && i + 2 * j < held ? col[uint64_t(p[j]) * K] : 0.0f;
+#pragma unroll
+        for (uint32_t j = 0; j < 16; j += 4)
+          acc += (double(f[j]) + double(f[j + 1])) + (double(f[j + 2]) + double(f[j + 3]));
+      }
+      __syncwarp();
+      held = 0;
+    }
+    acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 16);
+    if (on && half == 0) gc[v * K + k] = float(-acc);
+  }
 }
+
+static_assert(kBw8Threads / 32 * kBwList * 4 <= Bw8Smem::kBarOff, "lists in the stage buffers");
 
 // Elements of one segment slot of Bw8Args::part.
 constexpr uint64_t kBw8SlotElems = 2 * uint64_t(kBw8Tile) * kBwScores;
@@ -2688,21 +2777,14 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
           const uint64_t t0 = uint64_t(tile_now) * a.stages;
           const uint64_t v = uint64_t(tile_now) * kBw8Tile + r;
           const uint64_t k0 = uint64_t(stile) * kBwScores;
-          if (CORR && mine == 1 && v < a.V) {
-            const uint64_t s0 = (t0 >= u0 ? t0 : u0) - t0;   // the segment's stages
-#pragma unroll
-            for (uint32_t k = 0; k < kBwScores; ++k)
-              if (k0 + k < a.K && !isfinite(a.quanta[k0 + k]))
-                acc[k] = -bw_missing_sum(a.rows + v * a.pitch, a.ds + k0 + k, a.K, s0 * kBw8K,
-                                         min(a.people, (u + 1 - t0) * kBw8K));
-          }
           if (CORR || mine == 0) {
             if (t0 >= u0 && tile_end) {   // the whole tile is this CTA's
               float* out = mine ? a.gc : a.gw;
               if (v < a.V)
 #pragma unroll
                 for (uint32_t k = 0; k < kBwScores; ++k)
-                  if (k0 + k < a.K) out[v * a.K + k0 + k] = float(acc[k]);
+                  if (k0 + k < a.K && !(CORR && mine && a.sparse[k0 + k]))
+                    out[v * a.K + k0 + k] = float(acc[k]);
             } else {   // slot 0: the tile began in an earlier share, 1: it goes on in the next
               const uint64_t cta = uint64_t(stile) * gridDim.x + blockIdx.x;
               double* ps = a.part + (2 * cta + (t0 >= u0 ? 1 : 0)) * kBw8SlotElems +
@@ -2723,6 +2805,11 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+  // the stage buffers are idle: every load was consumed, every MMA committed
+  if (CORR && !lds_volatile_u32(abort_addr))
+    bw_missing_terms(a.rows, a.pitch, a.people, a.V, a.ds, uint32_t(a.K), a.sparse,
+                     uint64_t(stile) * kBwScores, warp, kBw8Threads / 32,
+                     reinterpret_cast<uint32_t*>(smem) + kBwList * warp, a.gc);
 }
 
 // Adds the segments of every variant tile that spans CTA shares, in share order.
@@ -2740,7 +2827,7 @@ __global__ void __launch_bounds__(256) gnm_bw_join(Bw8Args a, uint32_t ctas) {
     const uint32_t op = x / (kBw8Tile * kBwScores), e = x % (kBw8Tile * kBwScores);
     const uint64_t v = tile * kBw8Tile + e / kBwScores;
     const uint64_t k = uint64_t(stile) * kBwScores + e % kBwScores;
-    if (v >= a.V || k >= a.K) continue;
+    if (v >= a.V || k >= a.K || (op && a.sparse[k])) continue;
     double s = 0.0;
     for (uint64_t c = first; c <= last; ++c) {
       // the first share holds the tile as its last segment, the others as their first
@@ -2753,12 +2840,13 @@ __global__ void __launch_bounds__(256) gnm_bw_join(Bw8Args a, uint32_t ctas) {
 
 // dS [rows][K] -> 8-bit limb rows (tile t = k / 16: rows 64t + 16j + k % 16,
 // limb j) of P_pad people each, and their quanta [4][K16]; zeros past the last
-// person and score.  Person p of each 16 is stored at 4 (p % 4) + p / 4 % 4, the
+// person and score.  sparse[k]: limbs cannot hold the score (an infinity or NaN), its
+// missing term is summed from the dS values themselves.  Person p of each 16 is stored at 4 (p % 4) + p / 4 % 4, the
 // order in which gnm_t8_backward expands a packed word.  A CTA takes 32 people x
 // 16 scores: it reads whole dS rows and writes 32 consecutive bytes of a limb row.
 __global__ void __launch_bounds__(512)
     gnm_bw_build8(const float* g, uint64_t rows, uint64_t K, uint64_t K16, uint64_t P_pad,
-                  const uint32_t* amax_bits, int8_t* planes, double* quanta) {
+                  const uint32_t* amax_bits, int8_t* planes, double* quanta, uint32_t* sparse) {
   __shared__ float s_val[32][kBwScores + 1];
   const uint64_t p0 = uint64_t(blockIdx.x) * 32, k0 = uint64_t(blockIdx.y) * kBwScores;
   {
@@ -2771,6 +2859,7 @@ __global__ void __launch_bounds__(512)
   const uint64_t k = k0 + ks;
   const float am = k < K ? __uint_as_float(amax_bits[k]) : 0.0f;
   double q = am == 0.0f ? 1.0 : double(am) / 127.0;   // a NaN stays one
+  if (blockIdx.x == 0 && at == 0) sparse[k] = isfinite(am) ? 0u : 1u;
   const uint64_t row0 = uint64_t(blockIdx.y) * kBwN + ks;
   double rem = double(s_val[p][ks]);
 #pragma unroll
@@ -3534,7 +3623,7 @@ static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, con
 
   const uint64_t planes_bytes = (limb_rows * P_pad + 255) / 256 * 256;
   const uint64_t q_bytes = 4 * K16 * 8;
-  const uint64_t amax_bytes = (K16 * 4 + 255) / 256 * 256;
+  const uint64_t amax_bytes = (2 * K16 * 4 + 255) / 256 * 256;   // maxima, then `sparse`
   const uint64_t part_bytes = 2 * ctas * stiles * kBw8SlotElems * 8;
   const uint64_t need = planes_bytes + q_bytes + amax_bytes + part_bytes;
   if (p->bw_bytes < need) {
@@ -3551,6 +3640,7 @@ static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, con
   auto* quanta = reinterpret_cast<double*>(p->d_bw + planes_bytes);
   auto* amax = reinterpret_cast<uint32_t*>(p->d_bw + planes_bytes + q_bytes);
   a.quanta = quanta;
+  a.sparse = amax + K16;
   a.part = reinterpret_cast<double*>(p->d_bw + planes_bytes + q_bytes + amax_bytes);
   a.gw = d_grad_w;
   a.gc = d_grad_corr;
@@ -3562,7 +3652,7 @@ static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, con
   check_cuda(cudaMemsetAsync(amax, 0, K16 * 4, s), "memset");
   launch_bw_amax(p, gsf, amax, s);
   gnm_bw_build8<<<dim3(uint32_t(P_pad / 32), uint32_t(stiles)), 512, 0, s>>>(
-      gsf, p->fam, p->K, K16, P_pad, amax, planes, quanta);
+      gsf, p->fam, p->K, K16, P_pad, amax, planes, quanta, amax + K16);
   check_cuda(cudaGetLastError(), "gradient limb launch");
 
   const CUtensorMap rmap = make_row_map(d_rows, p->bpv, p->V, pitch, Bw8Smem::kPkRow, kBw8Tile,
