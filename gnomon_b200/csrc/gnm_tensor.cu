@@ -2433,7 +2433,6 @@ __device__ __noinline__ void bw_missing_terms(const uint8_t* rows, uint64_t pitc
   const uint32_t lane = threadIdx.x & 31u, half = lane >> 4;
   const uint64_t k = k0 + (lane & 15u);
   const bool on = k < K && sparse[k] != 0u;
-  if (!__any_sync(0xFFFFFFFFu, on)) return;
   const uint64_t bytes = (people + 3) / 4, step = uint64_t(gridDim.x) * warps;
   const uint32_t chunks = uint32_t((people + 2047) / 2048);
   const float* col = ds + k;
@@ -2549,6 +2548,7 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
   const uint32_t accempty = accfull + 8, drain0 = accfull + 16;   // one drain per MMA warp
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kHolder + 8);
   const uint32_t abort_addr = sb + L::kHolder + 8;
+  volatile uint32_t* any_sparse = reinterpret_cast<volatile uint32_t*>(smem + L::kHolder + 12);
   auto give_up = [&](uint32_t code) {
     *abort_flag = 1u;
     atomicOr(a.err, code);
@@ -2671,6 +2671,11 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
       __syncwarp();
       mbar_wait_bounded(drain, 0);
     }
+  } else if (warp == 3) {   // for the end, read while the others work
+    const uint64_t k = uint64_t(stile) * kBwScores + lane;
+    const bool on = CORR && lane < kBwScores && k < a.K && a.sparse[k] != 0u;
+    const uint32_t any = __any_sync(0xFFFFFFFFu, on);
+    if (lane == 0) *any_sparse = any;
   } else if (warp >= 4) {
     // ---------------- genotype expansion + epilogue (warps 4-19) ----------------
     const uint32_t quad = warp & 3;
@@ -2806,7 +2811,7 @@ __global__ void __launch_bounds__(kBw8Threads, 1)
     tmem_dealloc(tmem, 512);
   }
   // the stage buffers are idle: every load was consumed, every MMA committed
-  if (CORR && !lds_volatile_u32(abort_addr))
+  if (CORR && *any_sparse && !lds_volatile_u32(abort_addr))
     bw_missing_terms(a.rows, a.pitch, a.people, a.V, a.ds, uint32_t(a.K), a.sparse,
                      uint64_t(stile) * kBwScores, warp, kBw8Threads / 32,
                      reinterpret_cast<uint32_t*>(smem) + kBwList * warp, a.gc);
@@ -2827,39 +2832,120 @@ __global__ void __launch_bounds__(256) gnm_bw_join(Bw8Args a, uint32_t ctas) {
     const uint32_t op = x / (kBw8Tile * kBwScores), e = x % (kBw8Tile * kBwScores);
     const uint64_t v = tile * kBw8Tile + e / kBwScores;
     const uint64_t k = uint64_t(stile) * kBwScores + e % kBwScores;
-    if (v >= a.V || k >= a.K || (op && a.sparse[k])) continue;
+    if (v >= a.V || k >= a.K) continue;
+    const bool sparse = op && a.sparse[k] != 0u;   // (read beside the slots)
     double s = 0.0;
     for (uint64_t c = first; c <= last; ++c) {
       // the first share holds the tile as its last segment, the others as their first
       const uint64_t slot = 2 * (uint64_t(stile) * ctas + c) + (c == first ? 1 : 0);
       s += a.part[slot * kBw8SlotElems + uint64_t(op) * kBw8Tile * kBwScores + e];
     }
-    (op ? a.gc : a.gw)[v * a.K + k] = float(s);
+    if (!sparse) (op ? a.gc : a.gw)[v * a.K + k] = float(s);
   }
+}
+
+// Per-score max |dS| as float bit patterns (non-negative floats order like their
+// bits) and, where `spread` is given, the count of non-zero values and the sum of
+// their biased exponents: integers, so the same whatever the order.  A CTA takes
+// `per` rows of up to 256 scores; a thread's score is fixed, so it keeps its own and
+// adds them once.
+struct BwSpread {
+  unsigned long long* exps;   // [K16]
+  uint32_t* count;            // [K16]
+};
+__global__ void __launch_bounds__(256)
+    gnm_bw_amax(const float* g, uint64_t rows, uint64_t K, uint32_t per, uint32_t* amax_bits,
+                BwSpread spread) {
+  __shared__ uint32_t s_max[256], s_count[256], s_exps[256];
+  const uint32_t k0 = blockIdx.y * 256, K32 = uint32_t(K);
+  const uint32_t cols = min(K32 - k0, 256u);
+  const uint32_t height = cols == 1 ? 256u : 256u / cols;
+  const uint32_t r = cols == 1 ? threadIdx.x : threadIdx.x / cols, c = threadIdx.x - r * cols;
+  const uint64_t r0 = uint64_t(blockIdx.x) * per;
+  const uint32_t n = uint32_t(r0 + per < rows ? per : rows - r0);
+  const float* at = g + r0 * K + k0 + c;
+  uint32_t m = 0, count = 0, exps = 0;
+  for (uint32_t p = r; p < n && r < height; p += 8 * height) {
+    uint32_t v[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i)
+      v[i] = p + i * height < n ? __float_as_uint(fabsf(at[uint64_t(p + i * height) * K32])) : 0u;
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i) {
+      m = max(m, v[i]);
+      count += v[i] != 0u;
+      exps += v[i] >> 23;
+    }
+  }
+  auto add = [&](uint32_t k) {
+    atomicMax(amax_bits + k, m);
+    if (spread.exps) {
+      atomicAdd(spread.exps + k, static_cast<unsigned long long>(exps));
+      atomicAdd(spread.count + k, count);
+    }
+  };
+  if (cols == 1) {   // every thread has the same score
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    count = __reduce_add_sync(0xFFFFFFFFu, count);
+    exps = __reduce_add_sync(0xFFFFFFFFu, exps);
+    if (m && threadIdx.x % 32 == 0) add(k0);
+    return;
+  }
+  s_max[threadIdx.x] = s_count[threadIdx.x] = s_exps[threadIdx.x] = 0u;
+  __syncthreads();
+  if (m) {
+    atomicMax(s_max + c, m);
+    atomicAdd(s_count + c, count);
+    atomicAdd(s_exps + c, exps);
+  }
+  __syncthreads();
+  m = s_max[threadIdx.x];
+  count = s_count[threadIdx.x];
+  exps = s_exps[threadIdx.x];
+  if (threadIdx.x < cols && m) add(k0 + threadIdx.x);
+}
+
+// A score whose missing term needs more than its limbs: an infinity or NaN, or values
+// that lie, in the geometric mean, over 2^8 below the largest one.  The limbs'
+// step is 2^-31.9 of the largest, so values 2^-8 of it keep FP32's 24 bits.  Worst
+// error over 2,000 variants, of the sum of the |dS| added (20,000 people, 0.1 %
+// missing; limbs, an FP32 sum of the values, now): normal dS 3.6e-8, 4.4e-8, 3.6e-8;
+// one of 2^7 4.7e-8, 6.4e-8, 4.7e-8; one of 2^8 8.0e-8, 5.9e-8, 4.0e-8; one of 2^21
+// 3.7e-4, 5.8e-8, 4.0e-8; t with 2 degrees 3.9e-8, 6.2e-8, 3.9e-8; Cauchy 4.5e-6,
+// 9.7e-8, 5.2e-8; half of the people 2^-20 of the others 5.1e-4, 7.3e-8, 4.9e-8.
+__device__ __forceinline__ uint32_t bw_beyond_limbs(float am, unsigned long long exps,
+                                                    uint32_t count) {
+  const unsigned long long top = __float_as_uint(am) >> 23;
+  return !isfinite(am) || top * count > exps + 8ull * count ? 1u : 0u;
 }
 
 // dS [rows][K] -> 8-bit limb rows (tile t = k / 16: rows 64t + 16j + k % 16,
 // limb j) of P_pad people each, and their quanta [4][K16]; zeros past the last
-// person and score.  sparse[k]: limbs cannot hold the score (an infinity or NaN), its
+// person and score.  sparse[k]: limbs cannot hold the score (bw_beyond_limbs), its
 // missing term is summed from the dS values themselves.  Person p of each 16 is stored at 4 (p % 4) + p / 4 % 4, the
 // order in which gnm_t8_backward expands a packed word.  A CTA takes 32 people x
 // 16 scores: it reads whole dS rows and writes 32 consecutive bytes of a limb row.
 __global__ void __launch_bounds__(512)
     gnm_bw_build8(const float* g, uint64_t rows, uint64_t K, uint64_t K16, uint64_t P_pad,
-                  const uint32_t* amax_bits, int8_t* planes, double* quanta, uint32_t* sparse) {
+                  const uint32_t* amax_bits, BwSpread spread, int8_t* planes, double* quanta,
+                  uint32_t* sparse) {
   __shared__ float s_val[32][kBwScores + 1];
   const uint64_t p0 = uint64_t(blockIdx.x) * 32, k0 = uint64_t(blockIdx.y) * kBwScores;
-  {
-    const uint32_t p = threadIdx.x / kBwScores, k = threadIdx.x % kBwScores;
-    s_val[p][k] = (p0 + p < rows && k0 + k < K) ? g[(p0 + p) * K + k0 + k] : 0.0f;
-  }
-  __syncthreads();
   const uint32_t at = threadIdx.x % 32, ks = threadIdx.x / 32;   // stored position, score
   const uint32_t p = (at & 16u) + 4 * (at % 4) + at / 4 % 4;     // its person (an involution)
   const uint64_t k = k0 + ks;
+  // every load ahead of the barrier
   const float am = k < K ? __uint_as_float(amax_bits[k]) : 0.0f;
+  const bool first = blockIdx.x == 0 && at == 0;   // writes the score's quanta and flag
+  const unsigned long long exps = first ? spread.exps[k] : 0ull;
+  const uint32_t count = first ? spread.count[k] : 0u;
+  {
+    const uint32_t q = threadIdx.x / kBwScores, c = threadIdx.x % kBwScores;
+    s_val[q][c] = (p0 + q < rows && k0 + c < K) ? g[(p0 + q) * K + k0 + c] : 0.0f;
+  }
+  __syncthreads();
   double q = am == 0.0f ? 1.0 : double(am) / 127.0;   // a NaN stays one
-  if (blockIdx.x == 0 && at == 0) sparse[k] = isfinite(am) ? 0u : 1u;
+  if (first) sparse[k] = bw_beyond_limbs(am, exps, count);
   const uint64_t row0 = uint64_t(blockIdx.y) * kBwN + ks;
   double rem = double(s_val[p][ks]);
 #pragma unroll
@@ -2867,7 +2953,7 @@ __global__ void __launch_bounds__(512)
     const double li = fmin(fmax(rint(rem / q), -127.0), 127.0);
     rem -= li * q;
     planes[(row0 + kBwScores * j) * P_pad + p0 + at] = int8_t(li);
-    if (blockIdx.x == 0 && at == 0) quanta[j * K16 + k] = q;
+    if (first) quanta[j * K16 + k] = q;
   }
 }
 
@@ -2878,37 +2964,6 @@ __global__ void gnm_scatter_grad(const float* gs, const uint32_t* out_to_fam, ui
   if (x >= P * K) return;
   const uint64_t o = x / K, k = x % K;
   gsf[uint64_t(out_to_fam[o]) * K + k] = gs[x];
-}
-
-// Per-score max |dS| as float bit patterns (non-negative floats order like
-// their bits): a thread reads every 256 K-th element, so its score is fixed and
-// a warp's loads are consecutive; scores meet in shared memory when they fit.
-constexpr uint32_t kAmaxPer = 8;   // elements per thread
-__global__ void __launch_bounds__(256)
-    gnm_bw_amax(const float* g, uint64_t rows, uint64_t K, uint32_t* amax_bits) {
-  extern __shared__ uint32_t s_max[];
-  const bool shared = K <= kAmaxSharedScores;
-  if (shared) {
-    for (uint64_t k = threadIdx.x; k < K; k += 256) s_max[k] = 0u;
-    __syncthreads();
-  }
-  const uint64_t n = rows * K, x0 = uint64_t(blockIdx.x) * (256 * kAmaxPer) + threadIdx.x;
-  uint32_t v[kAmaxPer];
-#pragma unroll
-  for (uint32_t i = 0; i < kAmaxPer; ++i) {
-    const uint64_t x = x0 + 256 * i;
-    v[i] = x < n ? __float_as_uint(fabsf(g[x])) : 0u;
-  }
-#pragma unroll
-  for (uint32_t i = 0; i < kAmaxPer; ++i) {
-    const uint64_t x = x0 + 256 * i;
-    if (x < n && v[i]) atomicMax((shared ? s_max : amax_bits) + x % K, v[i]);
-  }
-  if (shared) {
-    __syncthreads();
-    for (uint64_t k = threadIdx.x; k < K; k += 256)
-      if (s_max[k]) atomicMax(amax_bits + k, s_max[k]);
-  }
 }
 
 // dS [rows][K] -> limb rows (tile t = k / 16: rows 64t + 16j + k % 16, limb j)
@@ -3587,12 +3642,18 @@ void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_b
   p->launches += 1;
 }
 
-static void launch_bw_amax(const gnm_plan* p, const float* gsf, uint32_t* amax, cudaStream_t s) {
+static void launch_bw_amax(const gnm_plan* p, const float* gsf, uint32_t* amax, BwSpread spread,
+                           cudaStream_t s) {
   const uint64_t n = p->fam * p->K;
   if (!n) return;
-  const uint32_t smem = p->K <= kAmaxSharedScores ? uint32_t(p->K * 4) : 0u;
-  const uint64_t blocks = (n + 256 * kAmaxPer - 1) / (256 * kAmaxPer);
-  gnm_bw_amax<<<uint32_t(blocks), 256, smem, s>>>(gsf, p->fam, p->K, amax);
+  // 2,048 values per CTA, more where that would be over 2,048 CTAs (each ends with
+  // up to 256 x 3 atomics); the shared sums of exponents hold 2^23 rows
+  const uint64_t cols = std::min<uint64_t>(256, p->K), height = 256 / cols;
+  const uint64_t tiles = (p->K + 255) / 256, steps = (p->fam + 8 * height - 1) / (8 * height);
+  const uint64_t most = std::max<uint64_t>(1, 2048 / tiles);
+  const uint64_t per = std::min<uint64_t>(uint64_t(1) << 23, (steps + most - 1) / most * 8 * height);
+  const dim3 grid(uint32_t((p->fam + per - 1) / per), uint32_t(tiles));
+  gnm_bw_amax<<<grid, 256, 0, s>>>(gsf, p->fam, p->K, uint32_t(per), amax, spread);
   check_cuda(cudaGetLastError(), "gradient maximum launch");
 }
 
@@ -3623,7 +3684,8 @@ static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, con
 
   const uint64_t planes_bytes = (limb_rows * P_pad + 255) / 256 * 256;
   const uint64_t q_bytes = 4 * K16 * 8;
-  const uint64_t amax_bytes = (2 * K16 * 4 + 255) / 256 * 256;   // maxima, then `sparse`
+  // per score: exponent sum (8 bytes), maximum, count of non-zero values, `sparse`
+  const uint64_t amax_bytes = (K16 * 20 + 255) / 256 * 256;
   const uint64_t part_bytes = 2 * ctas * stiles * kBw8SlotElems * 8;
   const uint64_t need = planes_bytes + q_bytes + amax_bytes + part_bytes;
   if (p->bw_bytes < need) {
@@ -3638,9 +3700,12 @@ static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, con
   }
   auto* planes = reinterpret_cast<int8_t*>(p->d_bw);
   auto* quanta = reinterpret_cast<double*>(p->d_bw + planes_bytes);
-  auto* amax = reinterpret_cast<uint32_t*>(p->d_bw + planes_bytes + q_bytes);
+  auto* exps = reinterpret_cast<unsigned long long*>(p->d_bw + planes_bytes + q_bytes);
+  auto* amax = reinterpret_cast<uint32_t*>(exps + K16);
+  const BwSpread spread{exps, amax + K16};
+  auto* sparse = amax + 2 * K16;
   a.quanta = quanta;
-  a.sparse = amax + K16;
+  a.sparse = sparse;
   a.part = reinterpret_cast<double*>(p->d_bw + planes_bytes + q_bytes + amax_bytes);
   a.gw = d_grad_w;
   a.gc = d_grad_corr;
@@ -3649,10 +3714,10 @@ static void backward_dw8(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, con
   a.pitch = pitch;
   a.ds = gsf;
   a.people = p->fam;
-  check_cuda(cudaMemsetAsync(amax, 0, K16 * 4, s), "memset");
-  launch_bw_amax(p, gsf, amax, s);
+  check_cuda(cudaMemsetAsync(exps, 0, K16 * 16, s), "memset");
+  launch_bw_amax(p, gsf, amax, d_grad_corr ? spread : BwSpread{}, s);
   gnm_bw_build8<<<dim3(uint32_t(P_pad / 32), uint32_t(stiles)), 512, 0, s>>>(
-      gsf, p->fam, p->K, K16, P_pad, amax, planes, quanta, amax + K16);
+      gsf, p->fam, p->K, K16, P_pad, amax, spread, planes, quanta, sparse);
   check_cuda(cudaGetLastError(), "gradient limb launch");
 
   const CUtensorMap rmap = make_row_map(d_rows, p->bpv, p->V, pitch, Bw8Smem::kPkRow, kBw8Tile,
@@ -3729,7 +3794,7 @@ void backward_dw(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, const float
   auto* ds = reinterpret_cast<float*>(p->d_bw + planes_bytes);
   auto* amax = reinterpret_cast<uint32_t*>(p->d_bw + planes_bytes + ds_bytes);
   check_cuda(cudaMemsetAsync(amax, 0, K16 * 4, s), "memset");
-  launch_bw_amax(p, gsf, amax, s);
+  launch_bw_amax(p, gsf, amax, BwSpread{}, s);
   p->launches += 1;
   const uint64_t nb = K16 * P_pad;
   gnm_bw_build<<<uint32_t((nb + 255) / 256), 256, 0, s>>>(gsf, p->fam, p->K, K16, P_pad, amax,

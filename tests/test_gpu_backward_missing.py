@@ -100,3 +100,44 @@ def test_time_with_nan_everywhere(cuda):
         took.append(min(ms[1:]))
     plan.close()
     assert took[1] < 8 * took[0], took
+
+
+@pytest.mark.parametrize("power", [9, 12, 16, 19])
+@pytest.mark.parametrize("missing", [0.001, 0.01])
+def test_one_dominant_gradient(cuda, power, missing):
+    """One person's dS 2^power times the others': where that person is called, the sum
+    over the missing is as accurate as its FP32 terms."""
+    plan, d, pitch, codes = make(20_000, 400, 4, missing, power)
+    gs = np.random.default_rng(power).standard_normal((20_000, 4)).astype(np.float32)
+    gs[4_711, 1], gs[4_711, 3] = 2.0 ** power, -2.0 ** power
+    gs[5::7, 3] = 0                    # people outside a keep set
+    _, gc = plan.backward(d, pitch, torch.from_numpy(gs).cuda(), grad_corr=True)
+    plan.sync()
+    plan.close()
+    gc = gc.cpu().numpy().astype(np.float64)
+    check_corrections(gc[:, [1, 3]], codes, gs[:, [1, 3]])
+
+
+@pytest.mark.parametrize("people,variants,scores", [
+    (700, 300, 300), (33, 40, 600), (600_001, 20, 16), (2_100_003, 3, 3)])
+def test_scores_of_different_scales(cuda, people, variants, scores):
+    """Largest values and spreads are found per score: every third score dominated by
+    one person, magnitudes from 2^-60 to 2^60, a score of zeros."""
+    plan, d, pitch, codes = make(people, variants, scores, 0.02, scores)
+    rng = np.random.default_rng(people)
+    gs = rng.standard_normal((people, scores)).astype(np.float32)
+    gs *= np.ldexp(np.float32(1), rng.integers(-60, 60, scores)).astype(np.float32)
+    gs[rng.integers(people), ::3] *= 2.0 ** 15
+    gs[:, 1] = 0
+    gw, gc = plan.backward(d, pitch, torch.from_numpy(gs).cuda(), grad_corr=True)
+    plan.sync()
+    plan.close()
+    gw, gc = gw.cpu().numpy().astype(np.float64), gc.cpu().numpy().astype(np.float64)
+    check_corrections(gc[:, ::3], codes, gs[:, ::3])
+    g = gs.astype(np.float64)
+    top = np.abs(g).max(axis=0)
+    for got, x in ((gw, np.array([0.0, 0.0, 1.0, 2.0])[codes]), (gc, (codes == 1) * -1.0)):
+        want = x @ g
+        # limbs leave a value within 2^-31.9 of its score's largest; one rounding to FP32
+        err = 2.0 ** -31.9 * (np.abs(x).sum(axis=1)[:, None] * top) + 2.0 ** -24 * np.abs(want)
+        assert (np.abs(got - want) <= err).all()
