@@ -339,7 +339,7 @@ def gpu_arm(args, rank, world, local_rank):
         shape = plan.autotune(rows, pitch, stream=stream)
         tuned = ({"kernel": shape >> 16, "splits_per_full_tile": shape & 0xFFFF}
                  if not tensor else tensor_shape(shape))
-    tshape = plan.shape if tensor else 0
+    tshape = plan.exact_shape if tensor else 0
     sums, counts = plan.outputs()
     grad_s = None
     if args.backward:
@@ -444,7 +444,7 @@ def gpu_arm(args, rank, world, local_rank):
     pairs = P * nnz
     value = world * pairs / (ms / 1e3)
     peak_hbm, peak_kind = peaks()
-    if tensor and tshape & 2:
+    if tensor and tshape & 2 and K <= 64:
         # narrow engine: M = 128 people, N = limb planes x 16 scores, two MMAs
         # (dosage, missing) per slice; one launch per block.  BF16: 4 + 4
         # planes (the missing operand's padded to four); 8-bit: 4 + 5 planes
@@ -474,10 +474,8 @@ def gpu_arm(args, rank, world, local_rank):
         # over 256-person x 128-score tiles (256-score tiles on SM pairs) and
         # 128-variant stages; the integer peak is taken as twice the BF16 one
         # (the nominal dense ratio, 4.5 / 2.25)
-        # (in the shape a plan starts with, 13 or 5, people are the M, 256 people x
-        # 32 scores, unless over 1 GB of limbs nearly fill tiles of 256 scores)
-        people_m = K > 64 and tshape == (13 if K > 128 else 5) and (
-            9 * K * V <= 1 << 30 or 20 * (-(-K // 256) * 256) > 23 * K)
+        # (with people as M, 256 people x 32 scores)
+        people_m = bool(tshape & 2)
         mt = 32 if people_m else 256 if tshape & 8 else 128
         ptiles, kpad, vpad = -(-P // 256), -(-K // mt) * mt, -(-V // 128) * 128
         executed = 2.0 * ptiles * 256 * vpad * kpad * 9

@@ -87,6 +87,7 @@ SIGNATURES = {
     "gnm_plan_autotune": (C.c_int, [C.c_void_p, C.c_void_p, C.c_uint64, C.c_uint64, C.c_void_p,
                                     C.POINTER(gnm_error)]),
     "gnm_plan_tuned_shape": (C.c_uint32, [C.c_void_p]),
+    "gnm_plan_exact_shape": (C.c_uint32, [C.c_void_p]),
     "gnm_plan_set_shape": (C.c_int, [C.c_void_p, C.c_uint32, C.POINTER(gnm_error)]),
     "gnm_plan_set_backward_limbs": (C.c_int, [C.c_void_p, C.c_uint32, C.POINTER(gnm_error)]),
     "gnm_decode_device": (C.c_int, [C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint64, C.c_void_p,

@@ -792,27 +792,36 @@ static void autotune_impl(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, ui
     }
     plain_shape_fixed(p, best_kernel, best_splits);
   } else {
-    // shape bit 0: raster order of the wide kernel; bit 1: the narrow kernel;
-    // bit 2: 8-bit limbs; bit 3: the 8-bit wide kernel over SM pairs.  Over 64
-    // scores the plan's first shape (13; 5 up to 128 scores) runs people as M
-    // unless its limbs are large (prefers_people)
+    // every kernel that can run the plan, the wide ones in both raster orders; a code
+    // that the plan's first shape has taken (13, or 5 up to 128 scores, over 64)
+    // gives way to the exact one
     const uint32_t people = tensor_people_shape(p);
     std::vector<uint32_t> cand = {0u, 1u, 4u, 5u, 12u, 13u};
-    if (tensor_can_narrow(p)) cand.insert(cand.begin(), {2u, 6u});
+    for (uint32_t& c : cand)
+      if (c == people) c |= kShapeExact;
+    if (tensor_can_narrow(p))
+      cand.insert(cand.begin(), {2u, 6u});
+    else
+      cand.push_back(people);
     uint32_t best = tensor_shape(p);
     const char* tr = std::getenv("GNM_TRACE");
     const bool trace = tr && std::strcmp(tr, "0") != 0;
     for (uint32_t c : cand) {
-      tensor_set_shape(p, c);
+      try {
+        tensor_set_shape(p, c);
+      } catch (const Failure&) {
+        continue;   // no memory for the partials that only this shape needs
+      }
       const float ms = time_best();
+      const uint32_t run = tensor_exact(p, c);
       if (trace)
-        std::fprintf(stderr, "[gnm autotune] tensor %s kernel%s: %.4f ms\n",
-                     c == people ? "8-bit (people as M)"
-                     : (c & 2u)  ? ((c & 4u) ? "narrow 8-bit (people as M)" : "narrow (people as M)")
-                              : ((c & 8u) ? "wide 8-bit on SM pairs (scores as M)"
-                                          : ((c & 4u) ? "wide 8-bit (scores as M)"
-                                                      : "wide (scores as M)")),
-                     (c & 2u) || c == people ? "" : ((c & 1u) ? ", score tiles fastest" : ", people tiles fastest"),
+        std::fprintf(stderr, "[gnm autotune] tensor shape %u: %s%s%s: %.4f ms\n", c,
+                     (run & 4u) ? "8-bit limbs" : "BF16 limbs",
+                     (run & 2u)   ? ", people as M"
+                     : (run & 8u) ? ", scores as M on SM pairs"
+                                  : ", scores as M",
+                     (run & 2u) ? "" : ((run & 1u) ? ", score tiles fastest"
+                                                   : ", people tiles fastest"),
                      ms);
       if (ms < best_ms) {
         best_ms = ms;
@@ -1732,10 +1741,11 @@ gnm_status gnm_plan_set_shape(gnm_plan* p, uint32_t shape, gnm_error* err) {
   if (!p) return GNM_ERR_INVALID;
   return guarded(err, [&] {
     if (p->engine != GNM_ENGINE_PLAIN) {
-      if (shape > 15 || ((shape & 8u) && (shape & 6u) != 4u))
+      if (shape > 31 || ((shape & 8u) && (shape & 6u) != 4u) ||
+          ((shape & kShapeExact) && !(shape & 4u)))
         fail(GNM_ERR_INVALID,
              "tensor engine shape is raster | (narrow << 1) | (8-bit limbs << 2) | "
-             "(8-bit wide kernel on SM pairs << 3)");
+             "(8-bit wide kernel on SM pairs << 3) | (exactly this 8-bit kernel << 4)");
       tensor_set_shape(p, shape);
       return;
     }
@@ -1763,6 +1773,11 @@ uint32_t gnm_plan_tuned_shape(const gnm_plan* p) {
   if (!p) return 0;
   return p->engine == GNM_ENGINE_PLAIN ? (p->kernel << 16) | std::min<uint32_t>(p->splits, 0xFFFFu)
                                        : tensor_shape(p);
+}
+
+uint32_t gnm_plan_exact_shape(const gnm_plan* p) {
+  if (!p || p->engine == GNM_ENGINE_PLAIN) return gnm_plan_tuned_shape(p);
+  return tensor_exact(p, tensor_shape(p));
 }
 
 gnm_status gnm_decode_device(const uint8_t* d_rows, uint64_t pitch, uint64_t nv, uint64_t np,

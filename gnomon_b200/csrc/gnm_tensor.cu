@@ -100,6 +100,8 @@ struct TensorPlan {
   bool narrow = false;                    // up to 64 scores: people as M (8-bit or BF16 limbs)
   bool can_narrow = false;                // K <= 64: either kernel can run the plan
   bool people = false;                    // the default shape runs people as M
+  bool pinned_people = false;             // over 64 scores: a shape that names people as M
+  uint32_t exact = 0;                     // kShapeExact of the shape
   CUtensorMap nmap_dos, nmap_mis;         // narrow boxes: 16 scores x 4 planes
   CUtensorMap nmap8_dos, nmap8_mis;       // 8-bit boxes: 128 variants x 16 nscores x 4 / 5 planes
 };
@@ -3206,6 +3208,23 @@ static bool prefers_people(const gnm_plan* p) {
   return limbs <= (uint64_t(1) << 30) || 20 * ((p->K + 255) / 256 * 256) > 23 * p->K;
 }
 
+// Over 64 scores, the slots of people as M beside the wide partials.
+static void alloc_slots(gnm_plan* p) {
+  TensorPlan* t = p->tensor;
+  const uint64_t n = uint64_t(t->nalloc) * t->nslot;
+  void* sum = pool_alloc(p->device, n * 8, "cudaMalloc(slots)");
+  void* cnt = nullptr;
+  try {
+    cnt = pool_alloc(p->device, n * 4, "cudaMalloc(slots)");
+  } catch (...) {
+    pool_free(sum);
+    throw;
+  }
+  t->d_slot_sum = static_cast<double*>(sum);
+  t->d_slot_cnt = static_cast<uint32_t*>(cnt);
+  p->device_bytes += n * 12;
+}
+
 void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trace) {
   auto mark = [&](const char* what) {
     if (trace) trace->mark(what);
@@ -3271,11 +3290,7 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
       alloc(reinterpret_cast<void**>(&t->d_part_pass), 3 * t->K_pad * t->P_pad * 8,
             "cudaMalloc(pass partials)");
   } else if (!t->can_narrow) {   // blocks that start off a 128-variant boundary add to the wide sums
-    const uint64_t n = uint64_t(t->nalloc) * t->nslot;
-    t->d_slot_sum = nullptr;
-    t->d_slot_cnt = nullptr;
-    alloc(reinterpret_cast<void**>(&t->d_slot_sum), n * 8, "cudaMalloc(slots)");
-    alloc(reinterpret_cast<void**>(&t->d_slot_cnt), n * 4, "cudaMalloc(slots)");
+    alloc_slots(p);
   }
   check_cuda(cudaMemset(t->d_planes_dos, 0, 4 * plane * 2), "memset planes");
   check_cuda(cudaMemset(t->d_planes_mis, 0, 4 * plane * 2), "memset planes");
@@ -3363,43 +3378,53 @@ void tensor_plan_destroy(gnm_plan* p) {
   p->tensor = nullptr;
 }
 
-// The plan's shape is its default one: 8-bit limbs with people as M (score tiles
-// fastest, and over 64 scores the bit of SM pairs where the plan fills them).
+// The shape a plan starts with: 8-bit limbs with people as M (score tiles fastest,
+// and over 64 scores the bit of SM pairs where the plan fills them).
 uint32_t tensor_default_shape(const gnm_plan* p) {
   return p->tensor->can_narrow ? 7u : (p->tensor->stiles >= 2 ? 13u : 5u);
 }
-uint32_t tensor_people_shape(const gnm_plan* p) {
-  return p->tensor->people ? tensor_default_shape(p) : ~0u;
+// The kernel that runs 8-bit blocks in a shape is gnm_t8_narrow: with the narrow bit
+// (over 64 scores only beside kShapeExact), and over 64 scores in the default shape
+// of a plan that prefers_people.  Every other shape with 8-bit limbs is the wide
+// kernel its bits name.
+static bool runs_people(const gnm_plan* p, uint32_t shape) {
+  if (!(shape & 4u)) return false;
+  return (shape & 2u) || (!p->tensor->can_narrow && p->tensor->people &&
+                          shape == tensor_default_shape(p));
 }
-// gnm_t8_narrow runs the plan's 8-bit blocks: up to 64 scores when the shape says
-// narrow, over 64 in the default shape (the wide kernels' bits otherwise, below) of
-// a plan that prefers_people.
-static bool people_as_m(const gnm_plan* p) {
-  const TensorPlan* t = p->tensor;
-  return t->can_narrow ? t->narrow && t->i8
-                       : t->people && tensor_shape(p) == tensor_default_shape(p);
+static bool people_as_m(const gnm_plan* p) { return runs_people(p, tensor_shape(p)); }
+uint32_t tensor_people_shape(const gnm_plan* p) {
+  return p->tensor->people ? tensor_default_shape(p) : kShapeExact | 7u;
+}
+uint32_t tensor_exact(const gnm_plan* p, uint32_t shape) {
+  if (!(shape & 4u)) return shape;   // BF16 limbs have one code per kernel
+  return kShapeExact | (runs_people(p, shape) ? 6u | (shape & 1u) : shape);
 }
 
 bool tensor_can_narrow(const gnm_plan* p) { return p->tensor && p->tensor->can_narrow; }
 uint32_t tensor_shape(const gnm_plan* p) {
   const TensorPlan* t = p->tensor;
-  return p->raster | (t->narrow ? 2u : 0u) | (t->i8 ? 4u : 0u) | (t->pair ? 8u : 0u);
+  return p->raster | (t->narrow || t->pinned_people ? 2u : 0u) | (t->i8 ? 4u : 0u) |
+         (t->pair ? 8u : 0u) | t->exact;
 }
 void tensor_set_shape(gnm_plan* p, uint32_t shape) {
   TensorPlan* t = p->tensor;
-  if ((shape & 2u) && !t->can_narrow)
+  if ((shape & 2u) && !t->can_narrow && !(shape & kShapeExact))
     fail(GNM_ERR_INVALID, "the narrow tensor kernel serves at most 64 scores");
-  const bool pair = (shape & 8u) != 0;
-  if (pair && !t->d_part_pass && !(t->people && shape == tensor_default_shape(p))) {
-    // the pass arrays of the SM-pair kernel, on first use
+  const bool people = runs_people(p, shape);
+  // what only some shapes need is allocated on first use
+  if ((shape & 8u) && !people && !t->d_part_pass) {   // the SM-pair kernel's passes 1-3
     const uint64_t bytes = 3 * t->K_pad * t->P_pad * 8;
     t->d_part_pass = static_cast<double*>(pool_alloc(p->device, bytes, "pass partials"));
     p->device_bytes += bytes;
     t->pass_valid = false;
   }
-  t->narrow = (shape & 2u) != 0;
+  if (people && !t->can_narrow && t->d_slot_sum == t->d_part_sum) alloc_slots(p);
+  t->narrow = (shape & 2u) != 0 && t->can_narrow;
+  t->pinned_people = (shape & 2u) != 0 && !t->can_narrow;
   t->i8 = (shape & 4u) != 0;
-  t->pair = pair;
+  t->pair = (shape & 8u) != 0;
+  t->exact = shape & kShapeExact;
   p->raster = shape & 1u;
 }
 

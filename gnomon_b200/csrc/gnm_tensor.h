@@ -26,11 +26,16 @@ void tensor_reset(gnm_plan* p, cudaStream_t s);
 // and the wide kernels (scores as M); over 64 see tensor_default_shape.
 bool tensor_can_narrow(const gnm_plan* p);
 // Shape codes: raster order of the wide kernels | narrow << 1 | 8-bit limbs << 2 |
-// SM pairs << 3 (gnm_plan_set_shape).
+// SM pairs << 3 | kShapeExact (gnm_plan_set_shape).  A code with kShapeExact always
+// means the kernel that its other bits name; without it, over 64 scores, the
+// default shape stands for whichever kernel the plan prefers.
+constexpr uint32_t kShapeExact = 16;
 uint32_t tensor_shape(const gnm_plan* p);
 uint32_t tensor_default_shape(const gnm_plan* p);
-// The shape that runs people as M, or ~0 where none does over 64 scores.
+// A shape that runs people as M.
 uint32_t tensor_people_shape(const gnm_plan* p);
+// The code that names the kernel which runs the plan's blocks in a shape.
+uint32_t tensor_exact(const gnm_plan* p, uint32_t shape);
 void tensor_set_shape(gnm_plan* p, uint32_t shape);
 void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint64_t v0,
                        uint64_t nv, cudaStream_t s);

@@ -124,6 +124,11 @@ class DevicePlan:
     def shape(self) -> int:
         return int(self.lib.gnm_plan_tuned_shape(self.handle))
 
+    @property
+    def exact_shape(self) -> int:
+        """``shape`` with the bits of the kernel that runs (16 set on 8-bit limbs)."""
+        return int(self.lib.gnm_plan_exact_shape(self.handle))
+
     def set_backward_limbs(self, bits: int) -> None:
         """dS limb width of ``backward``: 8 (default) or 16 (BF16)."""
         e = self._err()

@@ -240,20 +240,27 @@ gnm_status gnm_plan_autotune(gnm_plan* plan, const uint8_t* d_rows, uint64_t pit
 
 /* The tuned shape.  Plain engine: (kernel << 16) | splits per full people
  * tile, kernel = tile bytes (512, 1024, 2048) + 1 with a producer warp;
- * tensor engine: raster order | (2 if the narrow kernel runs the plan) |
- * (4 if it runs on 8-bit limbs; its blocks then start at multiples of 128
- * variants, others fall back to the BF16 limbs) | (8 if the wide kernel's
- * 8-bit MMAs span SM pairs; only with 4 and without 2).  Over 64 scores the
- * shape a plan starts with (13; 5 up to 128 scores) is the 8-bit kernel with
- * people as M, or SM pairs for over 1 GB of limbs (9 bytes per variant and
- * score) that nearly fill tiles of 256 scores; every other shape with 4 is the
- * wide kernel its bits name. */
+ * tensor engine: raster order | (2 if the narrow kernel, people as M, runs the
+ * plan) | (4 if it runs on 8-bit limbs; its blocks then start at multiples of
+ * 128 variants, others fall back to the BF16 limbs) | (8 if the wide kernel's
+ * 8-bit MMAs span SM pairs; only with 4 and without 2) | (16: exactly this
+ * 8-bit kernel; only with 4).  Over 64 scores the shape a plan starts with (13;
+ * 5 up to 128 scores) stands for the kernel that suits the plan, people as M
+ * or SM pairs; with 16 beside it, it is SM pairs (or one SM) with score
+ * tiles fastest, and 22 is people as M.  2 without 16 is for up to 64
+ * scores. */
 uint32_t gnm_plan_tuned_shape(const gnm_plan* plan);
 
-/* Pin a shape (a value gnm_plan_tuned_shape returned, e.g. saved from an
- * earlier autotune of the same workload).  GNM_ERR_INVALID for an unknown
- * kernel, more splits than the plan's partial slots hold, or a tensor shape
- * with unknown bits or SM pairs on anything but the 8-bit wide kernel. */
+/* The shape with the bits of the kernel that runs: on the tensor engine's 8-bit
+ * limbs always a code with 16, otherwise gnm_plan_tuned_shape. */
+uint32_t gnm_plan_exact_shape(const gnm_plan* plan);
+
+/* Pin a shape (a value gnm_plan_tuned_shape or gnm_plan_exact_shape returned,
+ * e.g. saved from an earlier autotune of the same workload).  GNM_ERR_INVALID for
+ * an unknown kernel, more splits than the plan's partial slots hold, or a tensor
+ * shape with unknown bits, SM pairs on anything but the 8-bit wide kernel, or 16
+ * without 8-bit limbs.  A shape's partials are allocated when it is first
+ * pinned. */
 gnm_status gnm_plan_set_shape(gnm_plan* plan, uint32_t shape, gnm_error* err);
 
 /* ---- Packed-row utilities ------------------------------------------------ */
