@@ -3181,19 +3181,25 @@ static uint32_t narrow_ctas(const TensorPlan* t, uint64_t K, uint32_t ns) {
   return std::max<uint32_t>(1, uint32_t(t->sms / stiles));
 }
 
+// The longest a CTA works, in units of 16 scores x all people tiles: its scores over
+// the CTAs that share them, times the waves of CTAs (more than one past one score
+// tile per SM).
+static double narrow_cost(const TensorPlan* t, uint64_t K, uint32_t ns) {
+  const uint64_t tiles = (K + kNrScores * ns - 1) / (kNrScores * ns);
+  const uint64_t ctas = narrow_ctas(t, K, ns);
+  const uint64_t waves = (tiles * ctas + t->sms - 1) / t->sms;   // over one only past `sms` tiles
+  return double(ns * waves) / double(ctas);
+}
 // 16-score groups per CTA.  32 scores halve the CTAs that expand the same rows
 // (20,000 people x 100,000 variants x 32: 337 us on 16, 324 on 32; 20,000 x 40,000
 // x 256: 1123 and 1034), unless 16 pad enough fewer scores per CTA in use: 15 %,
 // the expansion's share (40 scores, 48 against 64 padded: 71 and 77 us at 3,000 x
-// 60,000; 100 scores, 112 against 128: 493 and 484 us at 20,000 x 40,000).
+// 60,000; 100 scores, 112 against 128: 493 and 484 us at 20,000 x 40,000; 4,000
+// scores, 250 tiles of 16 in two waves against 125 in one: 24.2 and 25.2 ms at
+// 50,000 x 20,000, 3,000 scores 23.7 and 21.6).
 static uint32_t narrow_scores(const TensorPlan* t, uint64_t K) {
   if (K <= kNrScores) return 1;
-  double cost[2];
-  for (uint32_t ns : {1u, 2u}) {
-    const uint64_t tiles = (K + kNrScores * ns - 1) / (kNrScores * ns);
-    cost[ns - 1] = double(tiles * ns) / double(tiles * narrow_ctas(t, K, ns));
-  }
-  return 1.15 * cost[0] < cost[1] ? 1 : 2;
+  return 1.15 * narrow_cost(t, K, 1) < narrow_cost(t, K, 2) ? 1 : 2;
 }
 
 // Over 64 scores: people as M against SM pairs, the better wide kernel.  100,000
@@ -3203,9 +3209,21 @@ static uint32_t narrow_scores(const TensorPlan* t, uint64_t K) {
 // 882 us.  At 100,000 x 500,000 x 512 the 2.3 GB of limbs stream through L2 once per
 // round of people tiles and the board throttles: 136-145 against 128-130 ms.  So
 // pairs keep plans of over 1 GB of limbs whose scores nearly fill their 256.
-static bool prefers_people(const gnm_plan* p) {
-  const uint64_t limbs = kT8Planes * p->K * p->V;
-  return limbs <= (uint64_t(1) << 30) || 20 * ((p->K + 255) / 256 * 256) > 23 * p->K;
+//
+// Pairs also keep the plans whose score tiles leave SMs without work: a CTA belongs
+// to one score tile, so 75 to 95 tiles of 32 scores occupy little more than half of
+// 148 SMs.  What a kernel pays for, in scores of a full GPU: people as M 16 x SMs per
+// unit of narrow_cost, pairs 256 each.  Where people as M pay 1.5 times as much or
+// more, pairs are as fast or faster (people against pairs, 50,000 x 20,000 and 100,000
+// x 39,000): 2,400 scores, 1.85, 21.2 and 18.7, 77.8 and 60.5 ms; 3,000 scores, 1.54,
+// 21.6 and 23.0, 84.8 and 73.0 ms; below, 4,800 scores, 1.46, 36.0 and 36.1 ms; 1,600
+// scores, 1.32, 10.6 and 13.2, 39.1 and 42.9 ms; 1,000 scores, 1.16, 5.4 and 7.4,
+// 20.0 and 24.3 ms.
+static bool prefers_people(const gnm_plan* p, const TensorPlan* t) {
+  const uint64_t K256 = (p->K + 255) / 256 * 256, limbs = kT8Planes * p->K * p->V;
+  if (limbs > (uint64_t(1) << 30) && 20 * K256 <= 23 * p->K) return false;
+  const double paid = 16.0 * t->sms * narrow_cost(t, p->K, narrow_scores(t, p->K));
+  return t->stiles < 2 || paid < 1.5 * double(K256);
 }
 
 // Over 64 scores, the slots of people as M beside the wide partials.
@@ -3238,7 +3256,11 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   t->P_pad = uint64_t(t->ptiles) * kTcN;
   t->can_narrow = p->K <= kNarrowMaxScores;
   t->narrow = t->can_narrow;
-  t->people = t->can_narrow || prefers_people(p);
+  int sms = 0;
+  check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device),
+             "cudaDeviceGetAttribute");
+  t->sms = uint32_t(std::max(1, sms));
+  t->people = t->can_narrow || prefers_people(p, t);
   // 8-bit limbs unless a shape says otherwise: 1.4x the BF16 limbs' speed in the
   // wide kernels on the batched workload, errors below 2.3e-7 at full length on
   // every workload
@@ -3261,12 +3283,8 @@ void tensor_plan_create(gnm_plan* p, const gnm_prep_view* prep, PhaseTrace* trac
   alloc(reinterpret_cast<void**>(&t->d_planes_mis), 4 * plane * 2, "cudaMalloc(limb planes)");
   const uint64_t k16 = (p->K + kNrScores - 1) / kNrScores * kNrScores;
   const uint64_t base = ((p->fam + kNrM - 1) / kNrM) * (k16 / kNrScores);
-  int sms = 0;
-  check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device),
-             "cudaDeviceGetAttribute");
   t->P_nar = std::max<uint64_t>(1, (p->fam + 4 * kNrM - 1) / (4 * kNrM)) * (4 * kNrM);
   t->nslot = k16 * t->P_nar;
-  t->sms = uint32_t(std::max(1, sms));
   t->d_state = p->d_err + 1;   // cleared with the error word by every reset
   // a tile of S stages meets at most S / quota + 2 CTAs' shares, and quota >=
   // ptiles * S / (CTAs per score tile); after whole tiles, quota >= S

@@ -137,3 +137,39 @@ def test_rejected_codes(cuda, bad, scores):
         plan.set_shape(bad)
     assert ei.value.status == _lib.GNM_ERR_INVALID and plan.shape == before
     plan.close()
+
+
+@pytest.mark.parametrize("scores", [1_000, 1_600, 2_400, 3_000, 4_800])
+def test_default_is_not_the_slower_kernel(cuda, scores):
+    """Many scores, one cell per variant: the shape a plan starts with takes no more than
+    1.15 times the faster of people as M and SM pairs, and all agree."""
+    people, variants = 20_000, 20_000
+    rng = np.random.default_rng(scores)
+    prep = PreparationResult(rng.standard_normal(variants).astype(np.float32), np.zeros(variants),
+                             rng.integers(0, scores, variants), np.arange(variants + 1),
+                             ["S%d" % k for k in range(scores)], people)
+    gen = torch.Generator(device="cuda").manual_seed(scores)
+    pitch = row_pitch(prep.bytes_per_variant)
+    d = torch.randint(0, 256, (variants, pitch), dtype=torch.uint8, device="cuda", generator=gen)
+    plan = DevicePlan(prep, engine=_lib.ENGINE_TENSOR)
+    s, c = plan.outputs()
+    ms, sums, counts = {}, {}, {}
+    for code in (plan.shape, PEOPLE, PAIRS_SCORES_FIRST):
+        plan.set_shape(code)
+        took = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            plan.score(d, pitch, s, c)
+            b.record()
+            plan.sync()
+            took.append(a.elapsed_time(b))
+        ms[code] = min(took[1:])
+        sums[code], counts[code] = s.clone(), c.clone()
+    plan.close()
+    first = next(iter(ms))
+    assert ms[first] <= 1.15 * min(ms[PEOPLE], ms[PAIRS_SCORES_FIRST]), ms
+    for code in ms:
+        assert torch.equal(counts[code], counts[first])
+        top = sums[first].abs().max()
+        assert (sums[code] - sums[first]).abs().max() <= 1e-7 * top
