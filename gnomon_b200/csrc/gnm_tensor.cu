@@ -1924,12 +1924,13 @@ __device__ __forceinline__ uint64_t wide_slot(uint64_t f) {
 
 __global__ void __launch_bounds__(256)
     gnm_tc_finalize(SlotSums slots, WideSums wide, const double* init,
-                    const uint32_t* out_to_fam, uint64_t P, uint64_t K, double* sums,
-                    uint32_t* counts) {
+                    const uint32_t* out_to_fam, uint64_t P, uint64_t K, uint32_t ktile0,
+                    double* sums, uint32_t* counts) {
   __shared__ double s_sum[kFinTile][kFinTile + 1];
   __shared__ uint32_t s_cnt[kFinTile][kFinTile + 1];
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint64_t o0 = uint64_t(blockIdx.x) * kFinTile, k0 = uint64_t(blockIdx.y) * kFinTile;
+  const uint64_t o0 = uint64_t(blockIdx.x) * kFinTile;
+  const uint64_t k0 = uint64_t(ktile0 + blockIdx.y) * kFinTile;
   constexpr uint32_t kPer = kFinTile / 8;   // scores per warp
   const uint64_t o = o0 + lane;
   const uint64_t f = o >= P ? 0 : (out_to_fam ? out_to_fam[o] : o);
@@ -1991,12 +1992,13 @@ __global__ void __launch_bounds__(256)
 constexpr uint32_t kSlotScores = 8, kSlotWarps = 2 * kSlotScores;
 __global__ void __launch_bounds__(32 * kSlotWarps)
     gnm_tc_finalize_slots(SlotSums slots, WideSums wide, const double* init,
-                          const uint32_t* out_to_fam, uint64_t P, uint64_t K, double* sums,
-                          uint32_t* counts) {
+                          const uint32_t* out_to_fam, uint64_t P, uint64_t K, uint32_t ktile0,
+                          double* sums, uint32_t* counts) {
   __shared__ double s_sum[kSlotWarps][33];
   __shared__ uint32_t s_cnt[kSlotWarps][33];
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const uint64_t o0 = uint64_t(blockIdx.x) * 32, k0 = uint64_t(blockIdx.y) * kSlotScores;
+  const uint64_t o0 = uint64_t(blockIdx.x) * 32;
+  const uint64_t k0 = uint64_t(ktile0 + blockIdx.y) * kSlotScores;
   const uint64_t o = o0 + lane, k = k0 + w % kSlotScores;
   const uint32_t nslots = *slots.state, part = w / kSlotScores;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
@@ -3219,10 +3221,13 @@ static uint32_t narrow_scores(const TensorPlan* t, uint64_t K) {
 // 21.6 and 23.0, 84.8 and 73.0 ms; below, 4,800 scores, 1.46, 36.0 and 36.1 ms; 1,600
 // scores, 1.32, 10.6 and 13.2, 39.1 and 42.9 ms; 1,000 scores, 1.16, 5.4 and 7.4,
 // 20.0 and 24.3 ms.
+constexpr uint32_t kGridY = 65535;   // rows of a grid
 static bool prefers_people(const gnm_plan* p, const TensorPlan* t) {
   const uint64_t K256 = (p->K + 255) / 256 * 256, limbs = kT8Planes * p->K * p->V;
   if (limbs > (uint64_t(1) << 30) && 20 * K256 <= 23 * p->K) return false;
-  const double paid = 16.0 * t->sms * narrow_cost(t, p->K, narrow_scores(t, p->K));
+  const uint32_t ns = narrow_scores(t, p->K);
+  if ((p->K + kNrScores * ns - 1) / (kNrScores * ns) > kGridY) return false;
+  const double paid = 16.0 * t->sms * narrow_cost(t, p->K, ns);
   return t->stiles < 2 || paid < 1.5 * double(K256);
 }
 
@@ -3674,15 +3679,20 @@ void tensor_finalize(gnm_plan* p, double* d_sums, uint32_t* d_counts, bool add_b
   // 30,011 variants x 12, 30 against 41 us for the whole call; four or fewer leave
   // the 32 x 32 blocks ahead (100,000 x 4,000 x 16: 69 against 81 us; x 512: 1.49
   // against 1.88 ms).
-  if (slots && t->nslots8 > 4)
-    gnm_tc_finalize_slots<<<dim3(gx, uint32_t((p->K + kSlotScores - 1) / kSlotScores)),
-                            32 * kSlotWarps, 0, s>>>(ss, ws, init, p->d_out_to_fam, p->P, p->K,
-                                                     d_sums, d_counts);
-  else
-    gnm_tc_finalize<<<dim3(gx, uint32_t((p->K + kFinTile - 1) / kFinTile)), 256, 0, s>>>(
-        ss, ws, init, p->d_out_to_fam, p->P, p->K, d_sums, d_counts);
-  check_cuda(cudaGetLastError(), "tensor finalize launch");
-  p->launches += 1;
+  const bool many = slots && t->nslots8 > 4;
+  const uint32_t per = many ? kSlotScores : kFinTile;
+  const uint32_t ktiles = uint32_t((p->K + per - 1) / per);
+  for (uint32_t y = 0; y < ktiles; y += kGridY) {   // a grid has at most 65,535 rows
+    const dim3 grid(gx, std::min(kGridY, ktiles - y));
+    if (many)
+      gnm_tc_finalize_slots<<<grid, 32 * kSlotWarps, 0, s>>>(ss, ws, init, p->d_out_to_fam, p->P,
+                                                             p->K, y, d_sums, d_counts);
+    else
+      gnm_tc_finalize<<<grid, 256, 0, s>>>(ss, ws, init, p->d_out_to_fam, p->P, p->K, y, d_sums,
+                                           d_counts);
+    check_cuda(cudaGetLastError(), "tensor finalize launch");
+    p->launches += 1;
+  }
 }
 
 static void launch_bw_amax(const gnm_plan* p, const float* gsf, uint32_t* amax, BwSpread spread,
