@@ -912,7 +912,10 @@ template <class W>
 static void staged_pieces(uint64_t pieces, uint64_t piece, cudaStream_t s, W work) {
   if (pieces == 0) return;
   const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  const uint64_t nt = std::min<uint64_t>(hw, pieces);
+  // as many threads as a kept buffer serves: pieces of over 1 MB (rows of over 4.2
+  // million people) would take a buffer that is pinned and freed per call
+  const uint64_t fit = std::max<uint64_t>(1, kPinnedChunk / (2 * std::max<uint64_t>(1, piece)));
+  const uint64_t nt = std::min({uint64_t(hw), pieces, fit});
   PinnedBuffer pinned(2 * nt * piece);
   int device = 0;
   check_cuda(cudaGetDevice(&device), "cudaGetDevice");
