@@ -34,6 +34,7 @@ struct gnm_projector {
   int device = 0;
   uint64_t n = 0, K = 0;
   std::vector<double> acc;   // [n][K] row-major, every block so far
+  bool partial = false;      // a block's sums were not all added: the projector is unusable
 };
 
 namespace gnm {
@@ -1431,6 +1432,7 @@ static gnm_plan* plan_create_projection(int device, uint64_t n, uint64_t K, uint
 static void project_block_impl(gnm_projector* pj, const uint8_t* packed, uint64_t filled,
                                const float* coeffs, const float* loadings_cm) {
   if (!pj) fail(GNM_ERR_INVALID, "projector is NULL");
+  if (pj->partial) fail(GNM_ERR_COMPUTE, "an earlier block of this projector failed half added");
   if (filled == 0) return;
   if (!packed || !coeffs || !loadings_cm) fail(GNM_ERR_INVALID, "block buffers are NULL");
   PhaseTrace trace;
@@ -1492,16 +1494,24 @@ static void project_block_impl(gnm_projector* pj, const uint8_t* packed, uint64_
   finalize_impl(plan.get(), d_sums, d_counts, true, b.s);
   sync_impl(plan.get(), b.s);
   trace.mark("project: accumulate");
-  // the sums come back piece by piece and are added as they land
+  // the sums come back piece by piece and are added as they land; if a copy fails
+  // between two of them, neither this block nor a retry of it can be right
   const uint64_t n = pj->n * pj->K, per = kStagedPiece / sizeof(double);
   double* acc = pj->acc.data();
-  staged_pieces((n + per - 1) / per, kStagedPiece, b.s, [&](uint64_t i, uint8_t* buf, auto done) {
-    const uint64_t c0 = i * per, nc = std::min(per, n - c0);
-    check_cuda(cudaMemcpyAsync(buf, d_sums + c0, nc * 8, cudaMemcpyDeviceToHost, b.s), "sums");
-    done();
-    const double* from = reinterpret_cast<const double*>(buf);
-    for (uint64_t x = 0; x < nc; ++x) acc[c0 + x] += from[x];
-  });
+  std::atomic<bool> adding{false};
+  try {
+    staged_pieces((n + per - 1) / per, kStagedPiece, b.s, [&](uint64_t i, uint8_t* buf, auto done) {
+      const uint64_t c0 = i * per, nc = std::min(per, n - c0);
+      check_cuda(cudaMemcpyAsync(buf, d_sums + c0, nc * 8, cudaMemcpyDeviceToHost, b.s), "sums");
+      done();
+      const double* from = reinterpret_cast<const double*>(buf);
+      adding.store(true, std::memory_order_relaxed);
+      for (uint64_t x = 0; x < nc; ++x) acc[c0 + x] += from[x];
+    });
+  } catch (...) {
+    pj->partial = adding;
+    throw;
+  }
   trace.mark("project: add");
 }
 
@@ -1653,6 +1663,7 @@ gnm_status gnm_project_block(gnm_projector* pj, const uint8_t* packed, uint64_t 
 gnm_status gnm_project_scores(const gnm_projector* pj, double* scores_row_major, gnm_error* err) {
   return guarded(err, [&] {
     if (!pj || !scores_row_major) fail(GNM_ERR_INVALID, "NULL argument");
+    if (pj->partial) fail(GNM_ERR_COMPUTE, "a block of this projector failed half added");
     for (uint64_t i = 0; i < pj->acc.size(); ++i) scores_row_major[i] += pj->acc[i];
   });
 }

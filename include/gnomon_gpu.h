@@ -438,7 +438,10 @@ void gnm_project_destroy(gnm_projector* pj);
 
 /* One block of `filled` variants: packed .bed rows (host, ceil(n_samples/4)
  * bytes each, back to back), coeffs [filled][3] and column-major loadings
- * [components][filled] (f32, as the reference stages them).  Synchronous. */
+ * [components][filled] (f32, as the reference stages them).  Synchronous.  A
+ * failed call leaves the sums of earlier blocks as they were; should a copy back
+ * fail with the block half added, every later call on the projector but
+ * gnm_project_destroy fails. */
 gnm_status gnm_project_block(gnm_projector* pj, const uint8_t* packed, uint64_t filled,
                              const float* coeffs, const float* loadings_col_major,
                              gnm_error* err);
