@@ -319,7 +319,6 @@ static void plain_shape_fixed(gnm_plan* p, uint32_t kernel, uint32_t splits) {
   p->kernel = kernel;
   p->tiles = uint32_t(tiles);
   p->splits = uint32_t(sp);
-  p->last_splits = uint32_t(sp);
   p->slots = uint32_t(sp);
 }
 
@@ -476,7 +475,7 @@ static void upload_plain_records(gnm_plan* p, const std::vector<float4>& rec, Ph
   // Stage tables (the 3-variant lookup tables) of every score, built once on
   // the device while they fit the cache budget; blocks that start on a
   // kPlainRows-variant boundary read them directly.  Otherwise each accumulate call
-  // builds the tables of its block into a one-score scratch.
+  // builds the tables of its block into a scratch, a pass of scores at a time.
   const uint64_t stages = (p->V + kPlainRows - 1) / kPlainRows;
   if (p->K * stages * kPlainTableBytes <= kTableCacheBytes) {
     p->tab_stages = stages;
@@ -1767,15 +1766,13 @@ gnm_status gnm_plan_set_shape(gnm_plan* p, uint32_t shape, gnm_error* err) {
     bool known = false;
     for (uint32_t kn : kPlainKernels) known |= kn == kernel;
     if (!known) fail(GNM_ERR_INVALID, "unknown plain kernel in shape " + std::to_string(shape));
-    const uint32_t k0 = p->kernel, t0 = p->tiles, s0 = p->splits, l0 = p->last_splits,
-                   n0 = p->slots;
+    const uint32_t k0 = p->kernel, t0 = p->tiles, s0 = p->splits, n0 = p->slots;
     plain_shape_fixed(p, kernel, shape & 0xFFFFu);
     if (p->slots > p->splits_alloc) {
       const uint32_t need = p->slots;
       p->kernel = k0;
       p->tiles = t0;
       p->splits = s0;
-      p->last_splits = l0;
       p->slots = n0;
       fail(GNM_ERR_INVALID, "shape needs " + std::to_string(need) + " partial slots; the plan has " +
                                 std::to_string(p->splits_alloc));

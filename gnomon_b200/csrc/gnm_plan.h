@@ -133,9 +133,8 @@ struct gnm_plan {
   // plain engine
   uint32_t kernel = 1024;      // plain accumulate kernel (gnm_internal.h kPlain*)
   uint32_t tiles = 0;          // people tiles of the kernel's width
-  uint32_t splits = 0;         // variant splits of each full tile
-  uint32_t last_splits = 0;    // variant splits of the last (partly populated) tile
-  uint32_t slots = 0;          // partial slots in use: max(splits, last_splits)
+  uint32_t splits = 0;         // variant splits of every tile
+  uint32_t slots = 0;          // partial slots in use: one per split
   uint32_t valid_slots = 0;    // slots written since the last reset (finalize sums these)
   uint32_t splits_alloc = 0;   // partial slots allocated per score (autotune range)
   uint32_t raster = 0;         // tensor engine CTA order: 0 people-tile fastest, 1 score-tile
@@ -144,7 +143,7 @@ struct gnm_plan {
   float4* d_records = nullptr; // [K][rec_stride]
   uint8_t* d_tables = nullptr;  // stage tables of every score, [K][tab_stages][kPlainTableBytes]
   uint64_t tab_stages = 0;      // ceil(V / kPlainRows) when d_tables is cached, else 0
-  uint8_t* d_tab_scratch = nullptr;  // one score's tables for blocks the cache cannot serve
+  uint8_t* d_tab_scratch = nullptr;  // tables of a pass's scores for blocks the cache cannot serve
   uint64_t tab_scratch_stages = 0;
   double* d_part_sum = nullptr;
   uint32_t* d_part_cnt = nullptr;
@@ -155,7 +154,7 @@ struct gnm_plan {
   uint32_t* d_out_to_fam = nullptr;
   uint32_t* d_err = nullptr;
   float* d_grad_fam = nullptr;     // backward: dS in .bed person order (keep subsets)
-  uint8_t* d_bw = nullptr;         // backward: dS limb rows, FP32 dS, per-score maxima
+  uint8_t* d_bw = nullptr;         // backward: dS limb rows, quanta, per-score maxima, segments
   uint64_t bw_bytes = 0;
   uint32_t bw_limb_bits = 8;       // backward dS limbs: 8 (gnm_t8_backward) or 16 (BF16)
   std::vector<double> h_baseline;

@@ -4,8 +4,9 @@
 //   gnm_tc_accumulate / gnm_t8_accumulate  wide: scores as M, one SM per tile
 //   gnm_t8_pairs                           wide, 8-bit, SM pairs (cta_group::2),
 //                                          one persistent launch per call
-//   gnm_t8_narrow                          8-bit, people as M: the default for
-//                                          every score count
+//   gnm_t8_narrow                          8-bit, people as M: the default but for
+//                                          large limbs and some score counts
+//                                          (prefers_people)
 //   gnm_tc_narrow                          the same on BF16 limbs (<= 64 scores)
 //   gnm_tc_backward                        dW = G^T dS, dC on CUDA cores
 //   gnm_t8_backward                        dW and dC on the tensor cores (default)
@@ -1347,7 +1348,8 @@ __global__ void __launch_bounds__(kNrThreads, 1)
 // rows in step and share them in L2; whole tiles let the people tiles share the
 // limbs too, which even shares alone, each at its own variants, read from HBM
 // once they overflow L2 (200,000 people x 60,000 variants x 64 scores: 3.84 ms
-// on 16 scores per CTA, 3.76 on 32, 3.39 on 32 with whole tiles).
+// on 16 scores per CTA, 3.76 on 32, 3.39 on 32 with whole tiles, each a first pass;
+// back to back the board's power limits it to 3.87).
 //
 // S32 sums are exact for 2^17 variants: |limb x 4^q x dosage| <= 127 x 128.
 constexpr uint32_t kT8NrFlush = 1024;                // stages per exact S32 block (2^17 variants)
@@ -1409,7 +1411,6 @@ __global__ void gnm_tc_open_slots(double* sum, uint32_t* cnt, uint64_t slot_stri
 }
 
 struct T8NrArgs {
-  uint64_t num_rows;       // rows of this block
   int32_t a_x0;            // absolute variant index of block row 0 (multiple of 128)
   double* part_sum;        // [slots][K rounded to 16][P_pad]
   uint32_t* part_cnt;
@@ -1421,7 +1422,7 @@ struct T8NrArgs {
   uint32_t rounds;         // whole people tiles per CTA, before its share of the rest
   uint32_t quota;          // (people tile, stage) units per share
   uint32_t slots;          // slots of every tile; those without a segment are zeroed
-  uint32_t* state;         // {slots written since the reset, CTAs done}: see SlotState
+  uint32_t* state;         // {slots written since the reset, CTAs done}: see slots_written
   const double* quanta;    // [kT8Planes][K_pad]
   uint64_t K_pad;
   uint64_t K16;            // scores the partials hold
@@ -2367,10 +2368,13 @@ __global__ void __launch_bounds__(kBwThreads, 1)
 //     transposed; tcgen05.st.32x32b writes 64 people of both operands.
 //
 // Both operands meet the same limbs (two MMAs of N = 64 per 32 people, at least
-// 32 clocks each: 0.22 of the 0.44 ms at 20,000 x 200,000 x 16; the operand ring's
-// latency takes the rest); the dense missing product costs less than the sparse
-// FP32 sums did and is exact to the limbs.  256 variants per CTA share each limb tile (2 x 128 accumulator
-// columns + 256 of operand ring).  CTAs take equal shares of (variant tile,
+// 32 clocks each: 0.22 ms at 20,000 x 200,000 x 16, where the whole call takes 0.44
+// in a short run and 0.49 in a long one; the operand ring's latency takes the
+// rest).  The dense missing product costs less than the sparse FP32 sums did (0.44
+// against 1.55 ms); it is right to the limbs' step, and a score whose values are
+// spread wider than that allows takes sparse sums in FP64 (bw_beyond_limbs).  256
+// variants per CTA share each limb tile (2 x 128 accumulator columns + 256 of
+// operand ring).  CTAs take equal shares of (variant tile,
 // 512-person stage) units; a tile inside one share is written by its CTA, the
 // segments of a tile that spans shares go through FP64 slots that gnm_bw_join
 // adds in order.  S32 sums are exact for 2^17 people (127 x 2 x 64 each).
@@ -3205,7 +3209,7 @@ static uint32_t narrow_scores(const TensorPlan* t, uint64_t K) {
 }
 
 // Over 64 scores: people as M against SM pairs, the better wide kernel.  100,000
-// people x 40,000 variants x 512 scores 10.4 against 12.2 ms, x 150,000 37-38
+// people x 40,000 variants x 512 scores 10.0 against 12.2 ms, x 150,000 37-38
 // against 39.4 ms, 8,000 x 40,000 x 512 0.99 against 1.04; with a last score tile
 // to fill, 20,000 x 40,000 x 256, 1.03 against 1.53, 3,000 x 20,000 x 100, 61 against
 // 882 us.  At 100,000 x 500,000 x 512 the 2.3 GB of limbs stream through L2 once per
@@ -3516,7 +3520,6 @@ void tensor_accumulate(gnm_plan* p, const uint8_t* d_rows, uint64_t pitch, uint6
     fail(GNM_ERR_INVALID, "tensor engine blocks must start at a multiple of 64 variants");
   if (people_as_m(p) && v0 % kT8K == 0) {
     T8NrArgs a{};
-    a.num_rows = nv;
     a.a_x0 = int32_t(v0);
     a.part_sum = t->d_slot_sum;
     a.part_cnt = t->d_slot_cnt;

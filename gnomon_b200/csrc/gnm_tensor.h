@@ -9,8 +9,8 @@ struct gnm_prep_view;
 namespace gnm {
 
 // AUTO picks the tensor engine from this many score columns on.  Its cost alone
-// would put the line lower (20,000 x 200,000: 16 scores take 0.37 ms, one score
-// on the plain engine 0.33); it stays where the plain engine's sums, on another
+// would put the line lower (20,000 x 200,000: 16 scores take 0.41 ms, one score
+// on the plain engine 0.31); it stays where the plain engine's sums, on another
 // grid, have always ended, so that a call's result does not move.
 constexpr uint64_t kTensorMinScores = 8;
 
